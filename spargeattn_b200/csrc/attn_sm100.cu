@@ -3,8 +3,7 @@
 //                   s32 accumulator in tensor memory (TMEM). Two live 64-key blocks are paired into one
 //                   N = 128 step: their K tiles sit next to each other in shared memory, so one
 //                   instruction covers both (an odd last block runs as N = 64).
-//   online softmax in registers, two threads per query row (one per block of the pair; they exchange their
-//                   row maxima through shared memory): one running-maximum update, one output rescale and
+//   online softmax in registers, one thread per query row: one running-maximum update, one output rescale and
 //                   one round of hand-offs per 128 keys; P rounded to e4m3 and stored to a 128B-swizzled
 //                   shared-memory tile
 //   O += P8 V8    : tcgen05.mma kind::f8f6f4, A = P tile (K-major), B = V tiles (token-major,
@@ -12,15 +11,17 @@
 // Replaces qk_int_sv_f8_block_sparse_attn_kernel (csrc/qattn/qk_int_sv_f8_cuda_sm89.cuh:42-755)
 // and its host wrapper (csrc/qattn/qk_int_sv_f8_cuda_sm89.cu:392-585).
 //
-// One CTA per (q-block of 128 rows, head, batch); 10 warps:
-//   warps 0-7  softmax / correction / epilogue (warps w and w + 4 own query rows 32 (w & 3) ... = TMEM lanes)
-//   warp  8    TMA producer: walks the delta-encoded LUT and fetches only live K/V blocks
-//   warp  9    MMA issuer (one elected lane) and TMEM owner
-// Sixteen softmax warps per SM (two CTAs): four per scheduler, enough to keep the exponential unit fed while
-// other warps wait on a hand-off.
+// One CTA per (q-block of 128 rows, head, batch); 6 warps:
+//   warps 0-3  softmax / correction / epilogue (warp w owns query rows 32 w ... = TMEM lanes)
+//   warp  4    TMA producer: walks the delta-encoded LUT and fetches only live K/V blocks
+//   warp  5    MMA issuer (one elected lane) and TMEM owner
 // TMEM columns: [0,128) S of the current step, [128,128+D) O  -> 256 columns, two CTAs per SM.
-// S is single-buffered: the softmax warps release it as soon as their last tcgen05.ld of the step has
-// landed (half way through the step), and QK^T of the next step runs under the second half's exponentials.
+//
+// What bounds it: the instruction stream of the softmax warps, two per scheduler (one of each CTA). Per score it takes
+// the exponential unit 8 cycles of a warp and about four issue slots; everything else a step needs (hand-offs, TMEM
+// reads, row maxima, stores) is latency that only the other CTA's warp can fill, so the step is arranged to have as few
+// serial stages as possible: a thread reads its 128 scores at once and releases S (QK^T of the next step runs under this
+// step's exponentials), and P has two buffers, so that nothing waits for P.V of the previous step except a rescale.
 //
 // Every wait is bounded; on expiry the kernel records a code in *dev_status and unwinds.
 #include <cuda.h>
@@ -33,32 +34,28 @@ namespace sparge {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kFp8Offset = 8.807f;     // csrc/qattn/attn_utils.cuh:28-30: 2^8.807 = 448 = e4m3 max
 constexpr float kMaskValue = -5000000.0f;  // csrc/qattn/attn_utils.cuh:348-352
-constexpr uint32_t kMagicBits = 0x4B400000u;   // bit pattern of 12582912.0f = 1.5 * 2^23
-constexpr float kMagic = 12582912.0f;
-constexpr float kFastScaleLimit = 0.0078125f;  // 2^-7: bounds the fast path's per-block weight error by 0.41 %
-
 
 // PVF16: P and V in fp16 (tcgen05.mma kind::f16) instead of e4m3 -- the arithmetic of the reference's fp16-PV kernel
 // (csrc/qattn/qk_int_sv_f16_cuda_sm80.cuh), which its Sage1-signature entry points run. V then is the caller's fp16
 // tensor itself (no quantiser); a 64-key V tile is D/64 sub-tiles of [64 keys x 128 bytes] (64 channels each, 128B
 // swizzle), P is two sub-tiles of [128 rows x 128 bytes], one per block of a pair. The tiles are twice as large,
-// so the rings are shorter (see kKTiles) to keep two CTAs per SM.
+// so P has one buffer and the rings are shorter (see kKTiles) to keep two CTAs per SM.
 template <int D, bool PVF16 = false>
 struct AttnShape {
-  // K ring of single tiles (fp16 variant at D = 128): three 64-key tile slots instead of two pair slots, and one V
-  // pair slot, bring the CTA down to 105 KB of shared memory so that two fit per SM; a step's two K tiles are then not
+  // K ring of single tiles (fp16 variant at D = 128): three 64-key tile slots instead of two pair slots bring the CTA
+  // down to 105 KB of shared memory so that two fit per SM; a step's two K tiles are then not
   // adjacent and QK^T is issued as two N = 64 instruction groups.
   static constexpr bool kKTiles = PVF16 && D == 128;
   static constexpr int kStagesK = kKTiles ? 3 : (D == 128 || PVF16) ? 2 : 4;   // ring slots: PAIRS of 64-key tiles (tiles if kKTiles)
-  static constexpr int kStagesV = kKTiles ? 1 : (D == 128 || PVF16) ? 2 : 4;
+  static constexpr int kSlotsV = PVF16 ? (D == 128 ? 2 : 4) : (D == 128 ? 3 : 8);   // single 64-key tiles
   static constexpr int kTileQ = 128 * D;
   static constexpr int kTileKV = 64 * D;
   static constexpr int kPairKV = 2 * kTileKV;
   static constexpr int kTileV = PVF16 ? 2 * kTileKV : kTileKV;
-  static constexpr int kPairV = 2 * kTileV;
   static constexpr int kTileP = PVF16 ? 2 * 128 * 128 : 128 * 128;   // 128 rows x 128 keys of e4m3 / fp16
+  static constexpr int kBuffersP = PVF16 ? 1 : 2;
   static constexpr int kRingK = kStagesK * (kKTiles ? kTileKV : kPairKV);
-  static constexpr int kSmemBytes = 1024 + kTileQ + kTileP + kRingK + kStagesV * kPairV;
+  static constexpr int kSmemBytes = 1024 + kTileQ + kBuffersP * kTileP + kRingK + kSlotsV * kTileV;
   static constexpr int kTmemCols = 256;
   static constexpr int kCtasPerSm = 2;
   static constexpr uint32_t kSwizzle = (D == 128) ? kSwizzle128B : kSwizzle64B;
@@ -85,170 +82,100 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t* w) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
 
-// Row maximum of 32 scores, in log2 units. klim: keys with local index >= klim are masked.
+// Row maximum of a block's 64 scores, in log2 units. klim: keys with block-local index >= klim are masked.
 template <bool MASKED>
-__device__ __forceinline__ float chunk_rowmax(const uint32_t* sr, float c, int klim) {
+__device__ __forceinline__ float block_rowmax(const uint32_t* sr, float c, int klim) {
   if (!MASKED) {
-    int m0 = (int)sr[0], m1 = (int)sr[8], m2 = (int)sr[16], m3 = (int)sr[24];   // four chains: short latency
+    int m[4];   // four chains of 3-input maxima: short latency
 #pragma unroll
-    for (int k = 1; k < 7; k += 2) {
-      m0 = __vimax3_s32(m0, (int)sr[k], (int)sr[k + 1]);
-      m1 = __vimax3_s32(m1, (int)sr[8 + k], (int)sr[8 + k + 1]);
-      m2 = __vimax3_s32(m2, (int)sr[16 + k], (int)sr[16 + k + 1]);
-      m3 = __vimax3_s32(m3, (int)sr[24 + k], (int)sr[24 + k + 1]);
+    for (int g = 0; g < 4; g++) {
+      m[g] = __vimax3_s32((int)sr[16 * g], (int)sr[16 * g + 1], (int)sr[16 * g + 2]);
+#pragma unroll
+      for (int k = 3; k < 15; k += 2) m[g] = __vimax3_s32(m[g], (int)sr[16 * g + k], (int)sr[16 * g + k + 1]);
     }
-    m0 = __vimax3_s32(m0, m1, (int)sr[7]);
-    m2 = __vimax3_s32(m2, m3, (int)sr[15]);
-    const int mx = max(__vimax3_s32(m0, m2, (int)sr[23]), (int)sr[31]);
-    return (__int_as_float(mx + (int)kMagicBits) - kMagic) * c;   // c > 0: max commutes with the scaling
+    m[0] = __vimax3_s32(m[0], m[1], (int)sr[15]);
+    m[2] = __vimax3_s32(m[2], m[3], (int)sr[31]);
+    m[0] = __vimax3_s32(m[0], m[2], (int)sr[47]);
+    return __int2float_rn(max(m[0], (int)sr[63])) * c;   // c > 0: max commutes with the scaling
   } else {
     int mx = INT_MIN;
 #pragma unroll
-    for (int k = 0; k < 32; k++) mx = (k < klim) ? max(mx, (int)sr[k]) : mx;
+    for (int k = 0; k < 64; k++) mx = (k < klim) ? max(mx, (int)sr[k]) : mx;
     return (klim > 0) ? __int2float_rn(mx) * c : kMaskValue;
   }
 }
 
 // Per-thread granularity (QuantGranularity::kPerThread, qk_int_sv_f8_cuda_sm89.cuh:116-136): key column n of a
-// block is scaled by entry (n % 8) / 2 of the block's four K scales, so a thread's 32 scores carry four different
+// block is scaled by entry (n % 8) / 2 of the block's four K scales, so a thread's 64 scores carry four different
 // factors c4[0..3] and the integer maximum no longer commutes with the scaling: one maximum per factor.
-__device__ __forceinline__ float chunk_rowmax_g(const uint32_t* sr, const float* c4, int klim) {
+__device__ __forceinline__ float block_rowmax_g(const uint32_t* sr, const float* c4, int klim) {
   int mx[4] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN};
 #pragma unroll
-  for (int k = 0; k < 32; k++) mx[(k & 7) >> 1] = (k < klim) ? max(mx[(k & 7) >> 1], (int)sr[k]) : mx[(k & 7) >> 1];
+  for (int k = 0; k < 64; k++) mx[(k & 7) >> 1] = (k < klim) ? max(mx[(k & 7) >> 1], (int)sr[k]) : mx[(k & 7) >> 1];
   float r = kMaskValue;
 #pragma unroll
   for (int g = 0; g < 4; g++) r = (mx[g] != INT_MIN) ? fmaxf(r, __int2float_rn(mx[g]) * c4[g]) : r;
   return r;
 }
 
-__device__ __forceinline__ float chunk_exp_g(const uint32_t* sr, const float* c4, float m, int klim, uint32_t prow,
-                                             int chunk0, int rsw) {
-  uint32_t pr[4];
-  const float off = kFp8Offset - m;
-  float sum = 0.f;
-#pragma unroll
-  for (int k = 0; k < 32; k += 4) {
-    float p0 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 0]), c4[((k + 0) & 7) >> 1], off));
-    float p1 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 1]), c4[((k + 1) & 7) >> 1], off));
-    float p2 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 2]), c4[((k + 2) & 7) >> 1], off));
-    float p3 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 3]), c4[((k + 3) & 7) >> 1], off));
-    p0 = (k + 0 < klim) ? p0 : 0.f;
-    p1 = (k + 1 < klim) ? p1 : 0.f;
-    p2 = (k + 2 < klim) ? p2 : 0.f;
-    p3 = (k + 3 < klim) ? p3 : 0.f;
-    sum += (p0 + p1) + (p2 + p3);
-    pr[(k >> 2) & 3] = cvt_e4m3x4(p0, p1, p2, p3);
-    if ((k & 12) == 12) st_shared_v4(prow + (uint32_t)(((chunk0 + (k >> 4)) ^ rsw) << 4), pr);
-  }
-  return sum;
-}
-
-// P = 2^(S*c - m + 8.807) for 32 scores: row sum in fp32 before the e4m3 rounding
-// (ComputeUnit::kCudaCore, qk_int_sv_f8_cuda_sm89.cuh:773), bytes stored to the row's two 16-byte chunks
-// chunk0, chunk0+1 of the 128B-swizzled P tile. `prow` = shared address of the row, rsw = row & 7.
-template <bool EXACT>
-__device__ __forceinline__ float chunk_exp(const uint32_t* sr, float c, float m, int klim, int one, uint32_t prow,
-                                           int chunk0, int rsw) {
-  uint32_t pr[4];
-  if (!EXACT) {
-    // int32 -> fp32 by adding the bit pattern of 1.5 * 2^23 (exact for |S| < 2^22; here |S| <= 127^2 * 128);
-    // the 2^23 bias is taken out again inside the FMA constant. Packed f32x2 FMA / ADD halve the issue slots.
-    // That constant is rounded at the magnitude of 1.5 * 2^23 * c, so the exponents of this block are off
-    // by a common amount of at most 0.75 * c: blocks whose scale is not small take the exact path.
-    // `one` is a kernel argument equal to 1 that the compiler cannot fold: multiplying by it turns the
-    // int->float bias add into an IMAD, which issues on the FMA pipe instead of the half-rate integer pipe.
-    // (Pre-loading the accumulator with the bias through tcgen05.cp, so that no add is needed at all, was
-    // measured 14 % slower: the sixteen 4 KB copies per step delay QK^T more than 64 IMADs cost. Evaluating
-    // a quarter or half of the exponentials as a polynomial on the FMA pipe was 1.5 - 12 % slower: the loop
-    // is bound by issue slots, and each such element costs four more of them than a MUFU does.)
-    const float off = fmaf(-kMagic, c, kFp8Offset - m);
-    const float2 c2 = make_float2(c, c), o2 = make_float2(off, off);
-    float2 s0 = make_float2(0.f, 0.f), s1 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < 32; k += 4) {
-      float2 a = make_float2(__int_as_float((int)sr[k + 0] * one + (int)kMagicBits),
-                             __int_as_float((int)sr[k + 1] * one + (int)kMagicBits));
-      float2 bb = make_float2(__int_as_float((int)sr[k + 2] * one + (int)kMagicBits),
-                              __int_as_float((int)sr[k + 3] * one + (int)kMagicBits));
-      a = __ffma2_rn(a, c2, o2);
-      bb = __ffma2_rn(bb, c2, o2);
-      a.x = ex2_approx(a.x);
-      a.y = ex2_approx(a.y);
-      bb.x = ex2_approx(bb.x);
-      bb.y = ex2_approx(bb.y);
-      s0 = __fadd2_rn(s0, a);
-      s1 = __fadd2_rn(s1, bb);
-      pr[(k >> 2) & 3] = cvt_e4m3x4(a.x, a.y, bb.x, bb.y);
-      if ((k & 12) == 12) st_shared_v4(prow + (uint32_t)(((chunk0 + (k >> 4)) ^ rsw) << 4), pr);
-    }
-    s0 = __fadd2_rn(s0, s1);
-    return s0.x + s0.y;
+// Probabilities of four neighbouring keys, packed for the P tile: four e4m3 bytes or four fp16.
+template <bool PVF16>
+__device__ __forceinline__ void pack_p(uint32_t* w, float a, float b, float c, float d) {
+  if (PVF16) {
+    w[0] = pack2<__half>(a, b);
+    w[1] = pack2<__half>(c, d);
   } else {
-    const float off = kFp8Offset - m;
-    float sum = 0.f;
-#pragma unroll
-    for (int k = 0; k < 32; k += 4) {
-      float p0 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 0]), c, off));
-      float p1 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 1]), c, off));
-      float p2 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 2]), c, off));
-      float p3 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 3]), c, off));
-      p0 = (k + 0 < klim) ? p0 : 0.f;
-      p1 = (k + 1 < klim) ? p1 : 0.f;
-      p2 = (k + 2 < klim) ? p2 : 0.f;
-      p3 = (k + 3 < klim) ? p3 : 0.f;
-      sum += (p0 + p1) + (p2 + p3);
-      pr[(k >> 2) & 3] = cvt_e4m3x4(p0, p1, p2, p3);
-      if ((k & 12) == 12) st_shared_v4(prow + (uint32_t)(((chunk0 + (k >> 4)) ^ rsw) << 4), pr);
-    }
-    return sum;
+    w[0] = cvt_e4m3x4(a, b, c, d);
   }
 }
 
-// PVF16: P = 2^(S*c - m) for 32 scores as fp16 (no offset: the values are at most 1), row sum in fp32 before the
-// rounding; written to the four 16-byte chunks chunk0 .. chunk0+3 of the row in a [128 x 128 B] swizzled sub-tile.
-template <bool EXACT>
-__device__ __forceinline__ float chunk_exp_f16(const uint32_t* sr, float c, float m, int klim, int one, uint32_t prow,
-                                               int chunk0, int rsw) {
-  uint32_t pr[4];
-  if (!EXACT) {   // same int->float bias trick and packed arithmetic as the e4m3 path (see chunk_exp)
-    const float off = fmaf(-kMagic, c, -m);
-    const float2 c2 = make_float2(c, c), o2 = make_float2(off, off);
-    float2 s0 = make_float2(0.f, 0.f);
+// P = 2^(S*c - m + offset) for a block's 64 scores (offset 8.807 for e4m3, 0 for fp16 whose values are at most 1): row
+// sum in fp32 before the rounding (ComputeUnit::kCudaCore, qk_int_sv_f8_cuda_sm89.cuh:773); the packed values go to the
+// row's 16-byte chunks chunk0 ... of the 128B-swizzled tile. `prow` = shared address of the row, rsw = row & 7.
+// The scores are converted with the integer-to-float instruction: it is exact and runs at half rate beside the FMA
+// pipe's packed f32x2 work (adding a float bias as an integer multiply-add instead cost 3 % of the kernel).
+// EXACT: one factor per pair of key columns (c4, see block_rowmax_g; all equal for the coarser granularities) and a key
+// limit: keys >= klim get probability zero.
+template <bool EXACT, bool PVF16>
+__device__ __forceinline__ float block_exp(const uint32_t* sr, const float* c4, float m, int klim, uint32_t prow, int chunk0,
+                                           int rsw) {
+  constexpr int kKeysPerChunk = PVF16 ? 8 : 16;
+  const float off = (PVF16 ? 0.f : kFp8Offset) - m;
+  const float2 c2 = make_float2(c4[0], c4[0]), o2 = make_float2(off, off);
+  float2 s0 = make_float2(0.f, 0.f), s1 = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int k = 0; k < 32; k += 2) {
-      float2 a = make_float2(__int_as_float((int)sr[k + 0] * one + (int)kMagicBits),
-                             __int_as_float((int)sr[k + 1] * one + (int)kMagicBits));
-      a = __ffma2_rn(a, c2, o2);
-      a.x = ex2_approx(a.x);
-      a.y = ex2_approx(a.y);
+  for (int ch = 0; ch < 64 / kKeysPerChunk; ch++) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < kKeysPerChunk; i += 4) {
+      const int k = ch * kKeysPerChunk + i;
+      float2 a = make_float2(__int2float_rn((int)sr[k]), __int2float_rn((int)sr[k + 1]));
+      float2 b = make_float2(__int2float_rn((int)sr[k + 2]), __int2float_rn((int)sr[k + 3]));
+      if (EXACT) {
+        a = make_float2(fmaf(a.x, c4[(k & 7) >> 1], off), fmaf(a.y, c4[(k & 7) >> 1], off));
+        b = make_float2(fmaf(b.x, c4[((k + 2) & 7) >> 1], off), fmaf(b.y, c4[((k + 2) & 7) >> 1], off));
+      } else {
+        a = __ffma2_rn(a, c2, o2);
+        b = __ffma2_rn(b, c2, o2);
+      }
+      a = make_float2(ex2_approx(a.x), ex2_approx(a.y));
+      b = make_float2(ex2_approx(b.x), ex2_approx(b.y));
+      if (EXACT) {
+        a = make_float2(k < klim ? a.x : 0.f, k + 1 < klim ? a.y : 0.f);
+        b = make_float2(k + 2 < klim ? b.x : 0.f, k + 3 < klim ? b.y : 0.f);
+      }
       s0 = __fadd2_rn(s0, a);
-      const __half2 h = __floats2half2_rn(a.x, a.y);
-      pr[(k >> 1) & 3] = *reinterpret_cast<const uint32_t*>(&h);
-      if ((k & 6) == 6) st_shared_v4(prow + (uint32_t)(((chunk0 + (k >> 3)) ^ rsw) << 4), pr);
+      s1 = __fadd2_rn(s1, b);
+      pack_p<PVF16>(w + (PVF16 ? i / 2 : i / 4), a.x, a.y, b.x, b.y);
     }
-    return s0.x + s0.y;
+    st_shared_v4(prow + (uint32_t)(((chunk0 + ch) ^ rsw) << 4), w);
   }
-  float sum = 0.f;
-#pragma unroll
-  for (int k = 0; k < 32; k += 2) {
-    float p0 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 0]), c, -m));
-    float p1 = ex2_approx(fmaf(__int2float_rn((int)sr[k + 1]), c, -m));
-    p0 = (k + 0 < klim) ? p0 : 0.f;
-    p1 = (k + 1 < klim) ? p1 : 0.f;
-    sum += p0 + p1;
-    const __half2 h = __floats2half2_rn(p0, p1);
-    pr[(k >> 1) & 3] = *reinterpret_cast<const uint32_t*>(&h);
-    if ((k & 6) == 6) st_shared_v4(prow + (uint32_t)(((chunk0 + (k >> 3)) ^ rsw) << 4), pr);
-  }
-  return sum;
+  s0 = __fadd2_rn(s0, s1);
+  return s0.x + s0.y;
 }
 
-__device__ __forceinline__ void pair_sync(int id) {   // the two warps that share 32 query rows
-  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
-}
-
-constexpr int kAttnThreads = 320;
+constexpr int kSoftmaxWarps = 4, kProducerWarp = 4, kMmaWarp = 5;
+constexpr int kAttnThreads = 192;
 
 // GRAN = qk_quant_gran: 1 one Q scale per 128-row block, 2 one per 32-row group (the K scale is per 64-key block in
 // both), 3 per-thread Q/K scales. PV_MODE = PVThresholdMode: 0 no skip test, 1 the test decides per block, 2 per
@@ -259,28 +186,30 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
             const __grid_constant__ CUtensorMap tmap_v, OutT* __restrict__ o, const int32_t* __restrict__ lut,
             const int32_t* __restrict__ valid, const float* __restrict__ pvthr, const float* __restrict__ q_scale,
             const float* __restrict__ k_scale, const float* __restrict__ v_scale, int32_t* dev_status, int N, int H,
-            int nq, int nk, float sm_scale_log2, int one, long long osb, long long osh, long long osn,
+            int nq, int nk, float sm_scale_log2, long long osb, long long osh, long long osn,
             int32_t* __restrict__ pv_count, const int32_t* __restrict__ q_ranges) {
   using Shape = AttnShape<D, PVF16>;
   constexpr bool PV_SKIP = PV_MODE != 0, pv_per_warp = PV_MODE == 2, GRAN3 = GRAN == 3;
-  constexpr int SK = Shape::kStagesK, SV = Shape::kStagesV;
+  constexpr int SK = Shape::kStagesK, NV = Shape::kSlotsV;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sP = smem + Shape::kTileQ;
-  uint8_t* sK = sP + Shape::kTileP;                  // slot s: sK + s * kPairKV
-  uint8_t* sV = sK + Shape::kRingK;                    // slot s: sV + s * kPairV
+  uint8_t* sP = smem + Shape::kTileQ;                                // buffer b: sP + b * kTileP
+  uint8_t* sK = sP + Shape::kBuffersP * Shape::kTileP;               // slot s: sK + s * kPairKV
+  uint8_t* sV = sK + Shape::kRingK;                                  // slot n: sV + n * kTileV
   constexpr bool KT = Shape::kKTiles;
 
-  __shared__ uint64_t bar_q, bar_k_full[SK], bar_k_empty[SK], bar_v_full[SV], bar_v_empty[SV], bar_s_full, bar_s_free,
-      bar_p_ready, bar_o_done, bar_delta[2];
+  __shared__ uint64_t bar_q, bar_k_full[SK], bar_k_empty[SK], bar_v_full[NV], bar_v_empty[NV], bar_s_full, bar_s_free,
+      bar_p_ready[2], bar_o_done[2], bar_vote[2];   // the pairs alternate by step
   __shared__ uint32_t s_tmem_base;
-  __shared__ int s_skip[2];
-  __shared__ float s_delta[2][2][4];   // [step parity][block of the pair][row quarter]
-  __shared__ float s_rmax[2][2][128];  // [step parity][thread of the row pair][row]
+  __shared__ int s_skip[2][2], s_fail;   // [step parity][block of the pair]
+  // PV-skip votes, one byte per softmax warp: [step parity][block of the pair]
+  __shared__ uint32_t s_vote[2][2];
   __shared__ int4 s_meta[8];           // per step (ring of 8): block indices of the pair and their K scales (as bits)
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the shuffles let the compiler see that these are the same for the whole warp: branches on them need no convergence
+  // bookkeeping and the operands of the MMA instructions can be kept in uniform registers
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // Query blocks are issued last-first: under a causal mask the late rows hold the most live blocks,
   // and starting the longest rows first keeps the final wave short.
   // With q_ranges, (batch, head) bh computes only its query blocks [begin, begin + count): the unit of the
@@ -291,8 +220,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   if ((int)blockIdx.x >= q_count) return;
   const int qi = q_begin + q_count - 1 - (int)blockIdx.x;
   const size_t row_id = (size_t)bh * nq + qi;
-  int cnt = valid[row_id];
-  cnt = min(cnt, nk);
+  const int cnt = __shfl_sync(0xffffffffu, min(valid[row_id], nk), 0);
 
   if (cnt <= 0) {   // no live block: defined output (zeros)
     const int rows = min(128, N - qi * 128);
@@ -305,11 +233,11 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   }
   const int nsteps = (cnt + 1) >> 1;
 
-  if (warp == 9) {
+  if (warp == kMmaWarp) {
     tmem_alloc(&s_tmem_base, Shape::kTmemCols);
     tmem_relinquish();
   }
-  if (tid == 256) {
+  if (tid == kProducerWarp * 32) {
     mbar_init(&bar_q, 1);
 #pragma unroll
     for (int s = 0; s < SK; s++) {
@@ -317,19 +245,20 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       mbar_init(&bar_k_empty[s], 1);
     }
 #pragma unroll
-    for (int s = 0; s < SV; s++) {
+    for (int s = 0; s < NV; s++) {
       mbar_init(&bar_v_full[s], 1);
       mbar_init(&bar_v_empty[s], 1);
     }
     mbar_init(&bar_s_full, 1);
-    mbar_init(&bar_s_free, 8);     // one arrival per softmax warp
-    mbar_init(&bar_p_ready, 8);
-    mbar_init(&bar_o_done, 1);
-    mbar_init(&bar_delta[0], 8);
-    mbar_init(&bar_delta[1], 8);
+    mbar_init(&bar_s_free, kSoftmaxWarps);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      mbar_init(&bar_p_ready[i], kSoftmaxWarps);
+      mbar_init(&bar_o_done[i], 1);
+      mbar_init(&bar_vote[i], kSoftmaxWarps);
+    }
     mbar_fence_init();
-    s_skip[0] = 0;
-    s_skip[1] = 0;
+    s_fail = 0;
   }
   tc_fence_before();
   __syncthreads();
@@ -338,7 +267,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   const uint32_t tO = tbase + 128;
   const int32_t* lrow = lut + row_id * nk;
 
-  if (warp == 8) {
+  if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tmap_q);
@@ -369,78 +298,65 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       ks_out = __shfl_sync(0xffffffffu, ks_lane, n - win);
       return __shfl_sync(0xffffffffu, jabs, n - win);
     };
-    int ok = 1, issued_k = 0, issued_v = 0, issued_tiles = 0;   // issued_tiles: K tiles requested in tile-ring mode
-    auto load_pair = [&](const CUtensorMap* map, uint8_t* ring, uint64_t* full, uint64_t* empty, int stages, int s, int ja,
-                         int jb, const int4* meta) {   // lane 0 only
-      if (KT && meta) {   // K ring of single tiles: block n of the row's live list goes to slot n % 3
+    int ok = 1, issued_k = 0, issued_v = 0;   // K slots (pairs, or tiles if KT) and V tiles requested
+    // The step's block indices and K scales are published before its K tiles are requested: the softmax
+    // warps read them once S of that step is complete, which is ordered after the tiles' arrival. The ring
+    // slot was last used eight steps ago; the wait for a free K slot has just shown that step s - stages has retired.
+    auto load_k = [&](int s, int ja, int jb, const int4& meta) {   // lane 0 only
+      if (KT) {   // ring of single tiles: block n of the row's live list goes to slot n % SK
 #pragma unroll
         for (int blk = 0; blk < 2; blk++) {
           if (blk == 1 && jb < 0) break;
-          const int n = 2 * s + blk, ts = n % 3;
-          if (n >= 3) ok = mbar_wait(&empty[ts], ((n / 3) - 1) & 1) ? 1 : 0;
+          const int n = 2 * s + blk, ts = n % SK;
+          if (n >= SK) ok = mbar_wait(&bar_k_empty[ts], ((n / SK) - 1) & 1) ? 1 : 0;
           if (!ok) return;
-          if (blk == 0) s_meta[s & 7] = *meta;   // see below: before the step's first K tile is requested
-          mbar_arrive_expect_tx(&full[ts], Shape::kTileKV);
-          tma_load_3d(ring + ts * Shape::kTileKV, map, &full[ts], 0, (blk ? jb : ja) * 64, bh);
-          issued_tiles = n + 1;
+          if (blk == 0) s_meta[s & 7] = meta;
+          mbar_arrive_expect_tx(&bar_k_full[ts], Shape::kTileKV);
+          tma_load_3d(sK + ts * Shape::kTileKV, &tmap_k, &bar_k_full[ts], 0, (blk ? jb : ja) * 64, bh);
+          issued_k = n + 1;
         }
-        return;
+      } else {
+        const int slot = s % SK;
+        if (s >= SK) ok = mbar_wait(&bar_k_empty[slot], ((s / SK) - 1) & 1) ? 1 : 0;
+        if (!ok) return;
+        s_meta[s & 7] = meta;
+        uint8_t* dst = sK + slot * Shape::kPairKV;
+        mbar_arrive_expect_tx(&bar_k_full[slot], (jb >= 0 ? 2 : 1) * Shape::kTileKV);
+        tma_load_3d(dst, &tmap_k, &bar_k_full[slot], 0, ja * 64, bh);
+        if (jb >= 0) tma_load_3d(dst + Shape::kTileKV, &tmap_k, &bar_k_full[slot], 0, jb * 64, bh);
+        issued_k = s + 1;
       }
-      const int slot = s % stages;
-      if (s >= stages) ok = mbar_wait(&empty[slot], ((s / stages) - 1) & 1) ? 1 : 0;
-      if (!ok) return;
-      // The step's block indices and K scales are published before its K tiles are requested: the softmax
-      // warps read them once S of that step is complete, which is ordered after the tiles' arrival. The ring
-      // slot was last used eight steps ago; the wait above has just shown that step s - stages has retired.
-      if (meta) s_meta[s & 7] = *meta;
-      if (PVF16 && !meta) {   // fp16 V: D/64 sub-tiles of 64 channels (128 bytes) per block
-        uint8_t* dst = ring + slot * Shape::kPairV;
-        mbar_arrive_expect_tx(&full[slot], (jb >= 0 ? 2 : 1) * Shape::kTileV);
-#pragma unroll
-        for (int nh = 0; nh < D / 64; nh++) {
-          tma_load_3d(dst + nh * 8192, map, &full[slot], nh * 128, ja * 64, bh);
-          if (jb >= 0) tma_load_3d(dst + Shape::kTileV + nh * 8192, map, &full[slot], nh * 128, jb * 64, bh);
-        }
-        return;
-      }
-      uint8_t* dst = ring + slot * Shape::kPairKV;
-      mbar_arrive_expect_tx(&full[slot], (jb >= 0 ? 2 : 1) * Shape::kTileKV);
-      tma_load_3d(dst, map, &full[slot], 0, ja * 64, bh);
-      if (jb >= 0) tma_load_3d(dst + Shape::kTileKV, map, &full[slot], 0, jb * 64, bh);
     };
-    int ja = block_of(0);
-    float ka = ks_out, kb = 0.f;
-    int jb = -1;
-    if (cnt > 1) {
-      jb = block_of(1);
-      kb = ks_out;
-    }
-    if (lane == 0) {
-      const int4 mt = make_int4(ja, max(jb, 0), __float_as_int(ka), __float_as_int(kb));
-      load_pair(&tmap_k, sK, bar_k_full, bar_k_empty, SK, 0, ja, jb, &mt);
-      issued_k = 1;
-    }
-    for (int s = 0; s < nsteps && ok; s++) {
+    auto load_v = [&](int n, int j) {   // tile n of the row's live list; lane 0 only
+      const int slot = n % NV;
+      if (n >= NV) ok = mbar_wait(&bar_v_empty[slot], ((n / NV) - 1) & 1) ? 1 : 0;
+      if (!ok) return;
+      uint8_t* dst = sV + slot * Shape::kTileV;
+      mbar_arrive_expect_tx(&bar_v_full[slot], Shape::kTileV);
+      if (PVF16) {   // D/64 sub-tiles of 64 channels (128 bytes)
+#pragma unroll
+        for (int nh = 0; nh < D / 64; nh++) tma_load_3d(dst + nh * 8192, &tmap_v, &bar_v_full[slot], nh * 128, j * 64, bh);
+      } else {
+        tma_load_3d(dst, &tmap_v, &bar_v_full[slot], 0, j * 64, bh);
+      }
+      issued_v = n + 1;
+    };
+    int ja = 0, jb = -1;
+    for (int s = -1; s < nsteps && ok; s++) {   // K of step s + 1, then V of step s
       int na = -1, nb = -1;
+      float ka = 0.f, kb = 0.f;
       if (s + 1 < nsteps) {
         na = block_of(2 * s + 2);
         ka = ks_out;
-        kb = 0.f;
         if (2 * s + 3 < cnt) {
           nb = block_of(2 * s + 3);
           kb = ks_out;
         }
       }
       if (lane == 0) {
-        if (s + 1 < nsteps) {
-          const int4 mt = make_int4(na, max(nb, 0), __float_as_int(ka), __float_as_int(kb));
-          load_pair(&tmap_k, sK, bar_k_full, bar_k_empty, SK, s + 1, na, nb, &mt);
-          if (ok) issued_k = s + 2;
-        }
-        if (ok) {
-          load_pair(&tmap_v, sV, bar_v_full, bar_v_empty, SV, s, ja, jb, nullptr);
-          if (ok) issued_v = s + 1;
-        }
+        if (s + 1 < nsteps) load_k(s + 1, na, nb, make_int4(na, max(nb, 0), __float_as_int(ka), __float_as_int(kb)));
+        if (ok && s >= 0) load_v(2 * s, ja);
+        if (ok && s >= 0 && jb >= 0) load_v(2 * s + 1, jb);
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       ja = na;
@@ -449,311 +365,278 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     if (!ok && lane == 0) {
       report(dev_status, SPARGE_DEV_TIMEOUT_PRODUCER);
       // drain our own copies before the CTA's shared memory goes away
-      if (KT) {
-        for (int n = max(0, issued_tiles - 3); n < issued_tiles; n++) mbar_wait(&bar_k_full[n % 3], (n / 3) & 1);
-      } else {
-        for (int s = max(0, issued_k - SK); s < issued_k; s++) mbar_wait(&bar_k_full[s % SK], (s / SK) & 1);
-      }
-      for (int s = max(0, issued_v - SV); s < issued_v; s++) mbar_wait(&bar_v_full[s % SV], (s / SV) & 1);
+      for (int n = max(0, issued_k - SK); n < issued_k; n++) mbar_wait(&bar_k_full[n % SK], (n / SK) & 1);
+      for (int n = max(0, issued_v - NV); n < issued_v; n++) mbar_wait(&bar_v_full[n % NV], (n / NV) & 1);
     }
-  } else if (warp == 9) {
+  } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk2 = make_idesc(2, 1, 1, 0, 0, 128, 128);  // s32 += s8 * s8, both K-major, two blocks
-      constexpr uint32_t idesc_qk1 = make_idesc(2, 1, 1, 0, 0, 128, 64);   // odd last block
-      constexpr uint32_t idesc_pv = make_idesc(1, 0, 0, 0, 1, 128, D);     // f32 += e4m3 * e4m3, B MN-major
-      constexpr uint32_t idesc_pv16 = make_idesc(1, 0, 0, 0, 1, 128, 64);  // f32 += f16 * f16, B MN-major, 64 channels
-      constexpr uint32_t sbo = 8 * D;
-      bool ok = mbar_wait(&bar_q, 0);
-      // Every operand descriptor is built once: this thread shares its scheduler with four softmax warps,
-      // and each instruction it spends between a hand-off and the MMAs it releases delays the other side.
-      // A descriptor's low field is the address in 16-byte units, so moving to another ring slot is one add.
-      uint64_t qd[D / 32], kd[D / 32], pd[4], vd[4];
-#pragma unroll
-      for (int ks = 0; ks < D / 32; ks++) {
-        qd[ks] = make_smem_desc(smem_u32(sQ) + ks * 32, 16, sbo, Shape::kSwizzle);
-        kd[ks] = make_smem_desc(smem_u32(sK) + ks * 32, 16, sbo, Shape::kSwizzle);
+    // The whole warp walks the loop and one elected lane issues: with warp-uniform control flow the operands of the
+    // MMA instructions live in uniform registers. A single-lane loop has to move every descriptor word there by itself
+    // first; issuing a step's four P.V instructions that way took about 580 cycles.
+    constexpr uint32_t idesc_qk2 = make_idesc(2, 1, 1, 0, 0, 128, 128);  // s32 += s8 * s8, both K-major, two blocks
+    constexpr uint32_t idesc_qk1 = make_idesc(2, 1, 1, 0, 0, 128, 64);   // odd last block
+    constexpr uint32_t idesc_pv = make_idesc(1, 0, 0, 0, 1, 128, D);     // f32 += e4m3 * e4m3, B MN-major
+    constexpr uint32_t idesc_pv16 = make_idesc(1, 0, 0, 0, 1, 128, 64);  // f32 += f16 * f16, B MN-major, 64 channels
+    constexpr uint32_t sbo = 8 * D;
+    // a descriptor's low field is the address in 16-byte units: moving inside a tile or to another slot is one add
+    const uint64_t qd = make_smem_desc(smem_u32(sQ), 16, sbo, Shape::kSwizzle);
+    const uint64_t kd = make_smem_desc(smem_u32(sK), 16, sbo, Shape::kSwizzle);
+    const uint64_t pd = make_smem_desc(smem_u32(sP), 16, 1024, kSwizzle128B);
+    const uint64_t vd = PVF16 ? make_smem_desc(smem_u32(sV), 8192, 1024, kSwizzle128B)
+                              : make_smem_desc(smem_u32(sV), 64 * D, sbo, Shape::kSwizzle);
+    const bool leader = elect_one();
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, uint32_t parity) { ok = ok && __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
+    // waits for the K tiles of step s (one pair slot, or one or two tile slots of the tile ring)
+    auto wait_k = [&](int s) {
+      if (KT) {
+        wait(&bar_k_full[(2 * s) % SK], ((2 * s) / SK) & 1);
+        if (cnt - 2 * s >= 2) wait(&bar_k_full[(2 * s + 1) % SK], ((2 * s + 1) / SK) & 1);
+      } else {
+        wait(&bar_k_full[s % SK], (s / SK) & 1);
       }
-#pragma unroll
-      for (int ks = 0; ks < 4; ks++) {
-        pd[ks] = make_smem_desc(smem_u32(sP) + ks * 32, 16, 1024, kSwizzle128B);
-        vd[ks] = make_smem_desc(smem_u32(sV) + ks * 32 * D, 64 * D, sbo, Shape::kSwizzle);
-      }
-      constexpr uint64_t kSlotStep = (uint64_t)(Shape::kPairKV >> 4);
-      // fp16 P.V of one block: per 64-channel sub-tile of V four instructions of 16 keys each
-      auto issue_pv16 = [&](int blk, uint32_t slot_ofs_bytes, uint32_t& started) {
-        const uint32_t pbase = smem_u32(sP) + blk * 16384, vbase = smem_u32(sV) + slot_ofs_bytes + blk * Shape::kTileV;
-#pragma unroll
-        for (int nh = 0; nh < D / 64; nh++) {
-#pragma unroll
-          for (int ks = 0; ks < 4; ks++)
-            mma_f16_ss(tO + nh * 64, make_smem_desc(pbase + ks * 32, 16, 1024, kSwizzle128B),
-                       make_smem_desc(vbase + nh * 8192 + ks * 2048, 8192, 1024, kSwizzle128B), idesc_pv16,
-                       (ks > 0) ? 1u : started);
-        }
-        started = 1;
-      };
-      // waits for the K tiles of step s (one pair slot, or one or two tile slots of the tile ring)
-      auto wait_k = [&](int s) -> bool {
-        if (KT) {
-          const int nblk = min(2, cnt - 2 * s);
-          for (int blk = 0; blk < nblk; blk++) {
-            const int n = 2 * s + blk;
-            if (!mbar_wait(&bar_k_full[n % 3], (n / 3) & 1)) return false;
-          }
-          return true;
-        }
-        return mbar_wait(&bar_k_full[s % SK], (s / SK) & 1);
-      };
-      auto issue_qk = [&](int s) {   // the caller has waited for the K tiles of step s
-        if (KT) {   // the step's tiles are not adjacent in the ring: one N = 64 instruction group per block
-          tc_fence_after();
-          const int nblk = min(2, cnt - 2 * s);
-          for (int blk = 0; blk < nblk; blk++) {
-            const int ts = (2 * s + blk) % 3;
-            const uint64_t kofs = (uint64_t)ts * (uint64_t)(Shape::kTileKV >> 4);
+    };
+    auto issue_qk = [&](int s) {   // the K tiles of step s have arrived, S is free
+      tc_fence_after();
+      const bool two = cnt - 2 * s >= 2;
+      if (KT) {   // the step's tiles are not adjacent in the ring: one N = 64 instruction group per block
+        for (int blk = 0; blk < (two ? 2 : 1); blk++) {
+          const int ts = (2 * s + blk) % SK;
+          if (leader) {
 #pragma unroll
             for (int ks = 0; ks < D / 32; ks++)
-              mma_i8_ss(tbase + blk * 64, qd[ks], kd[ks] + kofs, idesc_qk1, ks > 0 ? 1u : 0u);
+              mma_i8_ss(tbase + blk * 64, qd + 2 * ks, kd + ts * (Shape::kTileKV >> 4) + 2 * ks, idesc_qk1, ks > 0);
             tc_commit(&bar_k_empty[ts]);
           }
-          tc_commit(&bar_s_full);
-          return;
         }
+        if (leader) tc_commit(&bar_s_full);
+      } else {
         const int slot = s % SK;
-        tc_fence_after();
-        const uint64_t kofs = (uint64_t)slot * kSlotStep;
-        const uint32_t idesc = (cnt - 2 * s >= 2) ? idesc_qk2 : idesc_qk1;
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < D / 32; ks++) mma_i8_ss(tbase, qd[ks], kd[ks] + kofs, idesc, ks > 0 ? 1u : 0u);
-        tc_commit(&bar_k_empty[slot]);
-        tc_commit(&bar_s_full);
-      };
-      if (ok) ok = wait_k(0);
-      if (ok) issue_qk(0);
-      uint32_t o_started = 0;
-      for (int s = 0; s < nsteps && ok; s++) {
-        // Tiles arrive long before the softmax warps' hand-offs: their barriers are checked first, so that
-        // only one wait stands between a hand-off and the MMAs it releases.
-        if (s + 1 < nsteps) {
-          ok = wait_k(s + 1);
-          if (!ok) break;
-          ok = mbar_wait(&bar_s_free, s & 1);      // every softmax warp has read S(s) into registers
-          if (!ok) break;
-          issue_qk(s + 1);
+          for (int ks = 0; ks < D / 32; ks++)
+            mma_i8_ss(tbase, qd + 2 * ks, kd + slot * (Shape::kPairKV >> 4) + 2 * ks, two ? idesc_qk2 : idesc_qk1, ks > 0);
+          tc_commit(&bar_k_empty[slot]);
+          tc_commit(&bar_s_full);
         }
-        const int slot = s % SV;
-        ok = mbar_wait(&bar_v_full[slot], (s / SV) & 1);
-        if (!ok) break;
-        const uint64_t vofs = (uint64_t)slot * kSlotStep;
-        const int nb = min(2, cnt - 2 * s);
-        ok = mbar_wait(&bar_p_ready, s & 1);
-        if (!ok) break;
-        tc_fence_after();
-        if (PVF16) {
-          if (!(PV_SKIP && s_skip[0])) issue_pv16(0, slot * Shape::kPairV, o_started);
-          if (nb == 2 && !(PV_SKIP && s_skip[1])) issue_pv16(1, slot * Shape::kPairV, o_started);
-        } else if (!(PV_SKIP && s_skip[0])) {
-          mma_f8_ss(tO, pd[0], vd[0] + vofs, idesc_pv, o_started);
-          mma_f8_ss(tO, pd[1], vd[1] + vofs, idesc_pv, 1u);
-          o_started = 1;
-        }
-        if (!PVF16 && nb == 2 && !(PV_SKIP && s_skip[1])) {
-          mma_f8_ss(tO, pd[2], vd[2] + vofs, idesc_pv, o_started);
-          mma_f8_ss(tO, pd[3], vd[3] + vofs, idesc_pv, 1u);
-          o_started = 1;
-        }
-        tc_commit(&bar_v_empty[slot]);
-        tc_commit(&bar_o_done);
       }
-      if (!ok) report(dev_status, SPARGE_DEV_TIMEOUT_MMA);
+    };
+    wait(&bar_q, 0);
+    wait_k(0);
+    if (ok) issue_qk(0);
+    bool started = false;          // the skip test may leave out the first products
+    for (int s = 0; s < nsteps && ok; s++) {
+      // Tiles arrive long before the softmax warps' hand-offs: their barriers are checked first, so that
+      // only one wait stands between a hand-off and the MMAs it releases.
+      if (s + 1 < nsteps) {
+        wait_k(s + 1);
+        wait(&bar_s_free, s & 1);      // every softmax warp has read S(s) into registers
+        if (!ok) break;
+        issue_qk(s + 1);
+      }
+      const bool two = cnt - 2 * s >= 2;
+      wait(&bar_v_full[(2 * s) % NV], ((2 * s) / NV) & 1);
+      if (two) wait(&bar_v_full[(2 * s + 1) % NV], ((2 * s + 1) / NV) & 1);
+      wait(&bar_p_ready[s & 1], (s >> 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t pbuf = pd + (s % Shape::kBuffersP) * (Shape::kTileP >> 4);
+#pragma unroll
+      for (int blk = 0; blk < 2; blk++) {
+        if (blk == 1 && !two) break;
+        const int slot = (2 * s + blk) % NV;
+        const uint64_t vtile = vd + slot * (Shape::kTileV >> 4);
+        if (!(PV_SKIP && __any_sync(0xffffffffu, s_skip[s & 1][blk]))) {
+          const uint32_t acc0 = PV_SKIP ? started : (s > 0 || blk > 0);
+          if (leader) {
+            if (PVF16) {   // per 64-channel sub-tile of V four instructions of 16 keys each
+#pragma unroll
+              for (int nh = 0; nh < D / 64; nh++)
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++)
+                  mma_f16_ss(tO + nh * 64, pbuf + blk * (16384 >> 4) + 2 * ks, vtile + nh * (8192 >> 4) + ks * (2048 >> 4),
+                             idesc_pv16, ks > 0 ? 1u : acc0);
+            } else {
+#pragma unroll
+              for (int ks = 0; ks < 2; ks++)
+                mma_f8_ss(tO, pbuf + 2 * (2 * blk + ks), vtile + ks * (32 * D >> 4), idesc_pv, ks > 0 ? 1u : acc0);
+            }
+          }
+          started = true;
+        }
+        if (leader) tc_commit(&bar_v_empty[slot]);
+      }
+      if (leader) tc_commit(&bar_o_done[s & 1]);
     }
+    if (!ok && lane == 0) report(dev_status, SPARGE_DEV_TIMEOUT_MMA);
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ softmax / correction / epilogue
-    // Two threads per query row (warps w and w + 4 share TMEM lanes 32 * (w & 3) ...): in a two-block step
-    // thread `half` = 0 takes block A (S columns 0..63) and thread 1 block B (64..127); in an odd last step
-    // they split the single block's 64 columns. Each thread works on its columns 32 at a time.
-    const int half = warp >> 2, wq = warp & 3;
-    const int row = wq * 32 + lane;
-    const uint32_t tlane = (uint32_t)(wq * 32) << 16;
+    // One thread per query row (TMEM lane). Waits record a failure in s_fail and run on; it is looked at once, in the
+    // epilogue.
+    const int row = warp * 32 + lane;
+    const uint32_t tlane = (uint32_t)(warp * 32) << 16;
     const uint32_t tS = tbase + tlane;
     const int qrow = qi * 128 + row;
-    const float qs = (GRAN3 ? q_scale[row_id * 32 + wq * 8 + (lane & 7)]
-                            : q_scale[GRAN == 1 ? row_id : row_id * 4 + wq]) * sm_scale_log2;
+    const float qs = (GRAN3 ? q_scale[row_id * 32 + warp * 8 + (lane & 7)]
+                            : q_scale[GRAN == 1 ? row_id : row_id * 4 + warp]) * sm_scale_log2;
     const float* ks_row = k_scale + (size_t)bh * nk * 4;   // GRAN3 only: four K scales per block
     const float thr = PV_SKIP ? pvthr[h] : 0.f;
     const uint32_t prow = smem_u32(sP) + (uint32_t)row * 128u;
     const int rsw = row & 7;
     float m = kMaskValue, d = 0.f;
-    bool ok = true;
     int npv = 0;   // PV products issued for this query block (all of them unless the skip test fires)
     for (int s = 0; s < nsteps; s++) {
-      const int nb = min(2, cnt - 2 * s);
-      const int col0 = (nb == 2) ? half * 64 : half * 32;      // first S column of this thread
-      const int nch = nb;                                       // 32-column chunks this thread handles
-      ok = __all_sync(0xffffffffu, mbar_wait(&bar_s_full, s & 1));
-      if (!ok) break;
+      const bool two = cnt - 2 * s >= 2;                          // the last step of an odd count has one block
+      mbar_wait_or_flag(&bar_s_full, s & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
       tc_fence_after();
-      // this thread's block and scale (published by the producer warp before the step's K tiles were requested)
+      uint32_t sr[128];
+      tmem_ld32(tS, sr);
+      tmem_ld32(tS + 32, sr + 32);
+      if (two) {
+        tmem_ld32(tS + 64, sr + 64);
+        tmem_ld32(tS + 96, sr + 96);
+      }
+      // the blocks and their scales (published by the producer warp before the step's K tiles were requested)
       const int4 mt = s_meta[s & 7];
-      const bool second = (nb == 2) && half;
-      const int j = second ? mt.y : mt.x;
-      const float c = qs * __int_as_float(second ? mt.w : mt.z);
-      float c4[4];
-      if (GRAN3) {
-        const float4 k4 = *reinterpret_cast<const float4*>(ks_row + (size_t)j * 4);
-        c4[0] = qs * k4.x; c4[1] = qs * k4.y; c4[2] = qs * k4.z; c4[3] = qs * k4.w;
-      }
-      // per-key mask limit of this row inside the block: keys with block-local index >= klim are masked
-      const int key0 = j * 64;
-      const bool masked = (key0 + 64 > N) || (CAUSAL && (key0 + 63 > qi * 128));
-      int klim = 64;
-      if (masked) {
-        klim = min(64, N - key0);
-        if (CAUSAL) klim = min(klim, qrow - key0 + 1);
-        klim = max(klim, 0);
-      }
-      const int kofs = col0 & 63;                                // block-local index of this thread's first column
-      uint32_t sr[32];
-      tmem_ld32(tS + col0, sr);
       tmem_wait_ld();
-      float rmax = GRAN3 ? chunk_rowmax_g(sr, c4, klim - kofs)
-                         : masked ? chunk_rowmax<true>(sr, c, klim - kofs) : chunk_rowmax<false>(sr, c, 32);
-      if (nch == 2) {
-        tmem_ld32(tS + col0 + 32, sr);
-        tmem_wait_ld();
-        rmax = fmaxf(rmax, GRAN3 ? chunk_rowmax_g(sr, c4, klim - kofs - 32)
-                                 : masked ? chunk_rowmax<true>(sr, c, klim - kofs - 32) : chunk_rowmax<false>(sr, c, 32));
-      }
-      // exchange the partial row maxima of the two threads of a row
-      s_rmax[s & 1][half][row] = rmax;
-      pair_sync(1 + wq);
-      const float r0 = s_rmax[s & 1][0][row], r1 = s_rmax[s & 1][1][row];
-      const float m1 = fmaxf(m, r0);                              // two-block step: maximum after block A
-      const float m2 = fmaxf(m1, r1);
-      // PV-skip test (qk_int_sv_f8_cuda_sm89.cuh:317-353), per 64-key block as in the reference: block A is
-      // tested against the running maximum before it, block B against the maximum after A. The warps
-      // publish their partial maxima now and read the result only after the exponentials, so the reduction
-      // latency is hidden; the last two live blocks are never skipped.
-      const bool candA = PV_SKIP && (2 * s < cnt - 2), candB = PV_SKIP && (nb == 2) && (2 * s + 1 < cnt - 2);
-      bool own_skip = false;   // per-warp mode: this warp's 32 rows drop their block (known before the exponentials)
-      if (PV_SKIP && (candA || candB)) {
-        // half 0 publishes block A's delta, half 1 block B's (a single-block step cannot be a candidate)
-        const float w = warp_max(half ? (r1 - m1) : (r0 - m));
-        if (lane == 0) {
-          s_delta[s & 1][half][wq] = w;
-          mbar_arrive(&bar_delta[s & 1]);
-        }
-        own_skip = pv_per_warp && (half ? candB : candA) && (w + thr <= 0.f);
-      }
-      const float alpha = (s > 0) ? ex2_approx(m - m2) : 0.f;
-      const bool need_rescale = (s > 0) && __any_sync(0xffffffffu, m2 > m);
-      // PV(s-1) must have retired before P is overwritten and before O is rescaled. (A second P buffer, which
-      // takes this wait off all steps that do not rescale, was measured slower: the kernel is bound by issue
-      // slots and the exponential unit together, not by this hand-off.)
-      if (s > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&bar_o_done, (s - 1) & 1));
-        if (!ok) break;
-        if (need_rescale) {   // some row of this warp raised its maximum: this thread rescales its half of O
-          tc_fence_after();
-#pragma unroll
-          for (int c0 = 0; c0 < D / 2; c0 += 16) {   // 16 columns at a time: 32 scores are still held in registers
-            uint32_t ov[16];
-            tmem_ld16(tO + tlane + half * (D / 2) + c0, ov);
-            tmem_wait_ld();
-            const float2 al2 = make_float2(alpha, alpha);
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-              const float2 r2 = __fmul2_rn(make_float2(__uint_as_float(ov[i]), __uint_as_float(ov[i + 1])), al2);
-              ov[i] = __float_as_uint(r2.x);
-              ov[i + 1] = __float_as_uint(r2.y);
-            }
-            tmem_st16(tO + tlane + half * (D / 2) + c0, ov);
-          }
-          tmem_wait_st();
-        }
-      }
-      d *= alpha;
-      m = m2;
-      // A 32-row group that drops its block in per-warp mode still writes its rows of P (as zeros, through the
-      // masked path with no visible key): the other groups' rows of the same block may be multiplied.
-      if (PV_SKIP && own_skip) klim = 0;
-      const bool exact = masked || own_skip || !(c < kFastScaleLimit);
-      // fp16 variant: this thread's block is sub-tile 0 or 1 of P, 8 keys per 16-byte chunk
-      const uint32_t prow16 = smem_u32(sP) + (second ? 16384u : 0u) + (uint32_t)row * 128u;
-      float sum = 0.f;
-      if (nch == 2) {   // the second 32 columns are still in registers
-        sum = PVF16 ? (exact ? chunk_exp_f16<true>(sr, c, m, klim - kofs - 32, one, prow16, (kofs >> 3) + 4, rsw)
-                             : chunk_exp_f16<false>(sr, c, m, 32, one, prow16, (kofs >> 3) + 4, rsw))
-              : GRAN3 ? chunk_exp_g(sr, c4, m, klim - kofs - 32, prow, (col0 >> 4) + 2, rsw)
-              : exact ? chunk_exp<true>(sr, c, m, klim - kofs - 32, one, prow, (col0 >> 4) + 2, rsw)
-                      : chunk_exp<false>(sr, c, m, 32, one, prow, (col0 >> 4) + 2, rsw);
-        tmem_ld32(tS + col0, sr);            // the first 32 again: they did not stay in registers
-        tmem_wait_ld();
-      }
-      // S has been read for the last time: the MMA warp may overwrite it with the next step's scores
+      // S is in registers: the MMA warp may overwrite it with the next step's scores
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_s_free);
-      sum += PVF16 ? (exact ? chunk_exp_f16<true>(sr, c, m, klim - kofs, one, prow16, kofs >> 3, rsw)
-                            : chunk_exp_f16<false>(sr, c, m, 32, one, prow16, kofs >> 3, rsw))
-             : GRAN3 ? chunk_exp_g(sr, c4, m, klim - kofs, prow, col0 >> 4, rsw)
-             : exact ? chunk_exp<true>(sr, c, m, klim - kofs, one, prow, col0 >> 4, rsw)
-                     : chunk_exp<false>(sr, c, m, 32, one, prow, col0 >> 4, rsw);
-      bool skip = false;
-      if (PV_SKIP && (candA || candB)) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&bar_delta[s & 1], (s >> 1) & 1));
-        if (!ok) break;
-        const float* da = s_delta[s & 1][0];
-        const float* db = s_delta[s & 1][1];
-        const bool skipA = candA && (fmaxf(fmaxf(da[0], da[1]), fmaxf(da[2], da[3])) + thr <= 0.f);
-        const bool skipB = candB && (fmaxf(fmaxf(db[0], db[1]), fmaxf(db[2], db[3])) + thr <= 0.f);
-        // candidates only occur in two-block steps: one block per thread. The product itself is left out only
-        // when all four groups drop the block, which is the per-block decision in either mode.
-        skip = pv_per_warp ? own_skip : (half ? skipB : skipA);
-        if (tid == 0) {
-          s_skip[0] = skipA ? 1 : 0;
-          s_skip[1] = skipB ? 1 : 0;
+
+      float cc[2][4];   // scale of each block's scores (per-thread granularity: of each pair of key columns)
+      int klim[2];      // keys with block-local index >= klim are masked
+      bool exact[2];
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        const int key0 = (b ? mt.y : mt.x) * 64;
+        if (GRAN3) {
+          const float4 k4 = *reinterpret_cast<const float4*>(ks_row + (size_t)(b ? mt.y : mt.x) * 4);
+          cc[b][0] = qs * k4.x; cc[b][1] = qs * k4.y; cc[b][2] = qs * k4.z; cc[b][3] = qs * k4.w;
+        } else {
+          cc[b][0] = cc[b][1] = cc[b][2] = cc[b][3] = qs * __int_as_float(b ? mt.w : mt.z);
         }
-        // per-warp mode counts this warp's own block; the two warps of a group are added up at the end
-        npv += pv_per_warp ? (own_skip ? 0 : 1) : (skipA ? 0 : 1) + (skipB ? 0 : 1);
+        klim[b] = 64;
+        exact[b] = __any_sync(0xffffffffu, (key0 + 64 > N) || (CAUSAL && (key0 + 63 > qi * 128)));
+        if (exact[b]) {
+          klim[b] = min(64, N - key0);
+          if (CAUSAL) klim[b] = min(klim[b], qrow - key0 + 1);
+          klim[b] = max(klim[b], 0);
+        }
+      }
+      float r[2];
+#pragma unroll
+      for (int b = 0; b < 2; b++)
+        r[b] = (b == 1 && !two) ? m
+               : GRAN3 ? block_rowmax_g(sr + 64 * b, cc[b], klim[b])
+               : exact[b] ? block_rowmax<true>(sr + 64 * b, cc[b][0], klim[b]) : block_rowmax<false>(sr + 64 * b, cc[b][0], 64);
+      const float m1 = fmaxf(m, r[0]);                            // maximum after block A
+      const float m2 = fmaxf(m1, r[1]);
+      // PV-skip test (qk_int_sv_f8_cuda_sm89.cuh:317-353), per 64-key block as in the reference: a block is dropped
+      // when no row's maximum comes within `thr` of the running one -- block A against the maximum before it, block B
+      // against the maximum after A. The warps publish their votes now and read the result only after the
+      // exponentials, so the reduction latency is hidden; the last two live blocks are never skipped (so a candidate
+      // step has two blocks).
+      const bool candA = PV_SKIP && (2 * s < cnt - 2), candB = PV_SKIP && (2 * s + 1 < cnt - 2);
+      bool own_skip[2] = {false, false};   // this warp's 32 rows vote to drop the block
+      if (PV_SKIP && candA) {
+        own_skip[0] = __all_sync(0xffffffffu, (r[0] - m) + thr <= 0.f);
+        own_skip[1] = __all_sync(0xffffffffu, (r[1] - m1) + thr <= 0.f) && candB;
+        if (lane == 0) {
+          reinterpret_cast<volatile uint8_t*>(&s_vote[s & 1][0])[warp] = own_skip[0];
+          reinterpret_cast<volatile uint8_t*>(&s_vote[s & 1][1])[warp] = own_skip[1];
+          mbar_arrive(&bar_vote[s & 1]);
+        }
+      }
+      const float alpha = (s > 0) ? ex2_approx(m - m2) : 0.f;
+      const bool need_rescale = (s > 0) && __any_sync(0xffffffffu, m2 > m);
+      m = m2;
+      // PV of the step that used this P buffer must have retired before the buffer is overwritten. With two buffers that
+      // is step s - 2, whose products were issued before QK^T of this step, so S being complete shows it.
+      if (Shape::kBuffersP == 1 && s > 0) mbar_wait_or_flag(&bar_o_done[(s - 1) & 1], ((s - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+      const uint32_t pb = prow + (s % Shape::kBuffersP) * Shape::kTileP;
+      float sum[2] = {0.f, 0.f};
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        if (b == 1 && !two) break;
+        // A 32-row group that drops its block in per-warp mode still writes its rows of P (as zeros, through the
+        // exact path with no visible key): the other groups' rows of the same block may be multiplied.
+        if (pv_per_warp && own_skip[b]) klim[b] = 0;
+        const uint32_t dst = pb + (PVF16 ? b * 16384u : 0u);
+        const int chunk0 = PVF16 ? 0 : 4 * b;
+        if (GRAN3 || exact[b] || (pv_per_warp && own_skip[b]))
+          sum[b] = block_exp<true, PVF16>(sr + 64 * b, cc[b], m, klim[b], dst, chunk0, rsw);
+        else
+          sum[b] = block_exp<false, PVF16>(sr + 64 * b, cc[b], m, 64, dst, chunk0, rsw);
+      }
+      // A wait names a phase by its parity, so the waiter must know that the phase before it is complete: PV(s-3), the
+      // previous user of this barrier, is (see above). With one barrier for all steps that would not hold.
+      if (need_rescale) {   // some row of this warp raised its maximum: O must hold everything up to PV(s-1)
+        if (Shape::kBuffersP > 1) mbar_wait_or_flag(&bar_o_done[(s - 1) & 1], ((s - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+        tc_fence_after();
+        const float2 al2 = make_float2(alpha, alpha);
+#pragma unroll
+        for (int c0 = 0; c0 < D; c0 += 16) {   // (32 columns at a time made the compiler spill)
+          uint32_t ov[16];
+          tmem_ld16(tO + tlane + c0, ov);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            const float2 r2 = __fmul2_rn(make_float2(__uint_as_float(ov[i]), __uint_as_float(ov[i + 1])), al2);
+            ov[i] = __float_as_uint(r2.x);
+            ov[i + 1] = __float_as_uint(r2.y);
+          }
+          tmem_st16(tO + tlane + c0, ov);
+        }
+        tmem_wait_st();
+      }
+      d *= alpha;
+      bool skip[2] = {false, false};
+      if (PV_SKIP && candA) {
+        mbar_wait_or_flag(&bar_vote[s & 1], (s >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+        // The product itself is left out only when all four groups drop the block, which is the per-block decision
+        // in either mode.
+        const bool skipA = s_vote[s & 1][0] == 0x01010101u, skipB = s_vote[s & 1][1] == 0x01010101u;
+        skip[0] = pv_per_warp ? own_skip[0] : skipA;
+        skip[1] = pv_per_warp ? own_skip[1] : skipB;
+        if (tid == 0) {
+          s_skip[s & 1][0] = skipA ? 1 : 0;
+          s_skip[s & 1][1] = skipB ? 1 : 0;
+        }
+        npv += (skip[0] ? 0 : 1) + (skip[1] ? 0 : 1);
       } else {
         if (PV_SKIP && tid == 0) {
-          s_skip[0] = 0;
-          s_skip[1] = 0;
+          s_skip[s & 1][0] = 0;
+          s_skip[s & 1][1] = 0;
         }
-        npv += pv_per_warp ? (nb == 2 ? 1 : 1 - half) : nb;
+        npv += two ? 2 : 1;
       }
-      if (!skip) d += sum;
+      if (!skip[0]) d += sum[0];
+      if (!skip[1]) d += sum[1];
       fence_proxy_async_smem();      // P bytes visible to the tensor core's operand fetch
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_p_ready);
+      if (lane == 0) mbar_arrive(&bar_p_ready[s & 1]);   // (two barriers: a warp may be a step ahead of another)
     }
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bar_o_done, (nsteps - 1) & 1));
-    if (ok) {
-      tc_fence_after();
-      // total row sum = the two threads' partial sums
-      s_rmax[0][half][row] = d;
-      if (PV_SKIP && pv_per_warp) s_rmax[1][half][row] = __int_as_float(npv);
-      pair_sync(1 + wq);
+    mbar_wait_or_flag(&bar_o_done[(nsteps - 1) & 1], ((nsteps - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+    tc_fence_after();
+    const int fail = *(volatile int*)&s_fail;
+    if (__all_sync(0xffffffffu, fail == 0)) {
       // One count per 32-row group, the layout of the reference's PV_Count (qk_int_sv_f8_cuda_sm89.cuh:650-656).
       // With the per-block decision the four entries of a block are equal; with the per-warp decision each group
-      // has its own, the sum of what its two warps (one per block of a pair) kept.
-      if (PV_SKIP && pv_per_warp) npv = __float_as_int(s_rmax[1][0][row]) + __float_as_int(s_rmax[1][1][row]);
-      if (pv_count && lane == 0 && half == 0) pv_count[row_id * 4 + wq] = npv;
+      // has its own.
+      if (pv_count && lane == 0) pv_count[row_id * 4 + warp] = npv;
       // A row that saw no key at all (token-level causal mask over every live block of its row of blocks) has an
       // empty sum: it is written as zeros. (The reference gives such a row the plain average of V over the masked
       // keys, because its mask value is a large finite number and exp2(mask - mask) = 1.)
-      const float dsum = s_rmax[0][0][row] + s_rmax[0][1][row];
-      const float inv = dsum > 0.f ? rcp_approx(dsum) : 0.f;
-      const float* vs = PVF16 ? nullptr : v_scale + (size_t)bh * D + half * (D / 2);   // fp16 V carries no scale
-      OutT* orow = o + (size_t)(bh / H) * osb + (size_t)(bh % H) * osh + (size_t)qrow * osn + half * (D / 2);
+      const float inv = d > 0.f ? rcp_approx(d) : 0.f;
+      const float* vs = PVF16 ? nullptr : v_scale + (size_t)bh * D;   // fp16 V carries no scale
+      OutT* orow = o + (size_t)(bh / H) * osb + (size_t)(bh % H) * osh + (size_t)qrow * osn;
 #pragma unroll
-      for (int c0 = 0; c0 < D / 2; c0 += 32) {
+      for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t ov[32];
-        tmem_ld32(tO + tlane + half * (D / 2) + c0, ov);
+        tmem_ld32(tO + tlane + c0, ov);
         tmem_wait_ld();
         uint32_t w[16];
 #pragma unroll
@@ -769,13 +652,13 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
         }
       }
     } else if (lane == 0) {
-      report(dev_status, SPARGE_DEV_TIMEOUT_SOFTMAX);
+      report(dev_status, fail ? fail : SPARGE_DEV_TIMEOUT_SOFTMAX);
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tbase, Shape::kTmemCols);
+  if (warp == kMmaWarp) tmem_dealloc(tbase, Shape::kTmemCols);
 }
 
 // ---------------------------------------------------------------------------- host side
@@ -823,7 +706,7 @@ static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
   const int nq = (N + 127) / 128, nk = (N + 63) / 64;
   const int gx = q_ranges ? min(q_blocks_max, nq) : nq;
   kern<<<dim3(gx, BH), kAttnThreads, smem, st>>>(tq, tk, tv, (OutT*)o, lut, valid, pvthr, qs, ks, vs, status, N, H, nq, nk,
-                                                 sm_scale_log2, 1, osb, osh, osn, pv_count, q_ranges);
+                                                 sm_scale_log2, osb, osh, osn, pv_count, q_ranges);
   return launch_status();
 }
 

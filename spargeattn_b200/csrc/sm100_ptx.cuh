@@ -82,6 +82,33 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
       : "memory");
   return ok != 0;
 }
+// The same wait for a loop that must not spend instructions on its outcome: when the time is up, `code` is written to
+// the shared word `fail`, and a wait that finds the word set gives up at once. The caller runs on (on whatever data is
+// there) and looks at the word once, at its end. Called by whole warps.
+__device__ __forceinline__ void mbar_wait_or_flag(uint64_t* bar, uint32_t parity, int* fail, int code) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P1, P2;\n\t"
+      ".reg .u32 cnt, f;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%0], %1;\n\t"
+      "@P1 bra SPARGE_DONE;\n\t"
+      "mov.u32 cnt, 0;\n\t"
+      "SPARGE_WAIT:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%0], %1, %4;\n\t"
+      "@P1 bra SPARGE_DONE;\n\t"
+      "ld.volatile.shared.u32 f, [%2];\n\t"
+      "setp.ne.u32 P2, f, 0;\n\t"
+      "@P2 bra SPARGE_DONE;\n\t"
+      "add.u32 cnt, cnt, 1;\n\t"
+      "setp.lt.u32 P2, cnt, %5;\n\t"
+      "@P2 bra SPARGE_WAIT;\n\t"
+      "st.volatile.shared.u32 [%2], %3;\n\t"
+      "SPARGE_DONE:\n\t"
+      "}\n" ::"r"(smem_u32(bar)),
+      "r"(parity), "r"(smem_u32(fail)), "r"(code), "n"(kWaitSliceNs), "n"(kWaitSlices)
+      : "memory");
+  __syncwarp();   // lanes may leave the loop at different tries; warp-collective instructions follow
+}
 
 // ---------------------------------------------------------------- TMA (tiled, no multicast)
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
@@ -103,6 +130,12 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, ui
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+
+// ---------------------------------------------------------------- register split between warpgroups
+template <int N>
+__device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ---------------------------------------------------------------- TMEM
 // One full warp executes alloc / dealloc. ncols: power of two in [32, 512].
@@ -160,6 +193,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
+}
+// The same 32-bit value into 8 consecutive columns of the warp's 32 lanes.
+__device__ __forceinline__ void tmem_fill8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
@@ -257,8 +296,17 @@ __device__ __forceinline__ uint16_t cvt_e4m3x2(float lo, float hi) {
   asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
   return r;
 }
+// Four floats -> four e4m3 bytes, a in bits [7:0]. Joining the halves with mov.b32 lets the second conversion merge into
+// the first one's register: 2 issue slots for four values instead of 3 (measured 2.0 against 4.0 cycles per conversion).
 __device__ __forceinline__ uint32_t cvt_e4m3x4(float a, float b, float c, float d) {
-  return static_cast<uint32_t>(cvt_e4m3x2(a, b)) | (static_cast<uint32_t>(cvt_e4m3x2(c, d)) << 16);
+  uint32_t r;
+  asm("{\n\t.reg .b16 lo, hi;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\t"
+      "mov.b32 %0, {lo, hi};\n\t}\n"
+      : "=r"(r)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
 }
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
