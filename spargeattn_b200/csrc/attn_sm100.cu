@@ -26,7 +26,10 @@
 // Every wait is bounded; on expiry the kernel records a code in *dev_status and unwinds.
 #include <cuda.h>
 
-#include "common.cuh"
+#include <atomic>
+
+#include "attn.cuh"
+#include "launch.cuh"
 #include "sm100_ptx.cuh"
 
 namespace sparge {
@@ -220,24 +223,15 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   if ((int)blockIdx.x >= q_count) return;
   const int qi = q_begin + q_count - 1 - (int)blockIdx.x;
   const size_t row_id = (size_t)bh * nq + qi;
-  const int cnt = __shfl_sync(0xffffffffu, min(valid[row_id], nk), 0);
-
-  if (cnt <= 0) {   // no live block: defined output (zeros)
-    const int rows = min(128, N - qi * 128);
-    constexpr int kChunks = D * (int)sizeof(OutT) / 16;
-    OutT* obase = o + (size_t)(bh / H) * osb + (size_t)(bh % H) * osh + (size_t)qi * 128 * osn;
-    for (int i = tid; i < rows * kChunks; i += kAttnThreads)
-      reinterpret_cast<uint4*>(obase + (size_t)(i / kChunks) * osn)[i % kChunks] = make_uint4(0, 0, 0, 0);
-    if (pv_count && tid < 4) pv_count[row_id * 4 + tid] = 0;
-    return;
-  }
-  const int nsteps = (cnt + 1) >> 1;
 
   if (warp == kMmaWarp) {
     tmem_alloc(&s_tmem_base, Shape::kTmemCols);
     tmem_relinquish();
   }
   if (tid == kProducerWarp * 32) {
+    tma_prefetch_desc(&tmap_q);
+    tma_prefetch_desc(&tmap_k);
+    tma_prefetch_desc(&tmap_v);
     mbar_init(&bar_q, 1);
 #pragma unroll
     for (int s = 0; s < SK; s++) {
@@ -260,6 +254,9 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     mbar_fence_init();
     s_fail = 0;
   }
+  pdl_wait();   // everything below reads what the kernels before this one wrote
+  const int cnt = __shfl_sync(0xffffffffu, min(valid[row_id], nk), 0);
+  const int nsteps = (cnt + 1) >> 1;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -267,12 +264,16 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   const uint32_t tO = tbase + 128;
   const int32_t* lrow = lut + row_id * nk;
 
-  if (warp == kProducerWarp) {
+  if (cnt <= 0) {   // no live block: defined output (zeros)
+    const int rows = min(128, N - qi * 128);
+    constexpr int kChunks = D * (int)sizeof(OutT) / 16;
+    OutT* obase = o + (size_t)(bh / H) * osb + (size_t)(bh % H) * osh + (size_t)qi * 128 * osn;
+    for (int i = tid; i < rows * kChunks; i += kAttnThreads)
+      reinterpret_cast<uint4*>(obase + (size_t)(i / kChunks) * osn)[i % kChunks] = make_uint4(0, 0, 0, 0);
+    if (pv_count && tid < 4) pv_count[row_id * 4 + tid] = 0;
+  } else if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      tma_prefetch_desc(&tmap_q);
-      tma_prefetch_desc(&tmap_k);
-      tma_prefetch_desc(&tmap_v);
       mbar_arrive_expect_tx(&bar_q, Shape::kTileQ);
       tma_load_3d(sQ, &tmap_q, &bar_q, 0, qi * 128, bh);
     }
@@ -335,7 +336,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       mbar_arrive_expect_tx(&bar_v_full[slot], Shape::kTileV);
       if (PVF16) {   // D/64 sub-tiles of 64 channels (128 bytes)
 #pragma unroll
-        for (int nh = 0; nh < D / 64; nh++) tma_load_3d(dst + nh * 8192, &tmap_v, &bar_v_full[slot], nh * 128, j * 64, bh);
+        for (int nh = 0; nh < D / 64; nh++)
+          tma_load_4d(dst + nh * 8192, &tmap_v, &bar_v_full[slot], nh * 128, j * 64, bh % H, bh / H);
       } else {
         tma_load_3d(dst, &tmap_v, &bar_v_full[slot], 0, j * 64, bh);
       }
@@ -677,37 +679,84 @@ static EncodeTiledFn encode_fn() {
 }
 
 // Byte tensor [planes, rows, inner] with a [1, box_rows, inner] box, swizzle span = inner bytes.
-// box_inner: bytes of a row that one copy takes (default: the whole row); x coordinates are multiples of it.
-static bool make_map(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows, uint64_t planes, uint32_t box_rows,
-                     uint32_t box_inner = 0) {
+static bool make_map(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows, uint64_t planes, uint32_t box_rows) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return false;
-  if (box_inner == 0) box_inner = (uint32_t)inner;
   cuuint64_t dims[3] = {inner, rows, planes};
   cuuint64_t strides[2] = {inner, inner * rows};
-  cuuint32_t box[3] = {box_inner, box_rows, 1};
+  cuuint32_t box[3] = {(cuuint32_t)inner, box_rows, 1};
   cuuint32_t es[3] = {1, 1, 1};
-  const CUtensorMapSwizzle sw = box_inner == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  const CUtensorMapSwizzle sw = inner == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16 = false>
-static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o, const int32_t* lut,
-                       const int32_t* valid, const float* pvthr, const float* qs, const float* ks, const float* vs,
-                       int32_t* status, int BH, int H, int N, float sm_scale_log2, long long osb, long long osh,
-                       long long osn, int32_t* pv_count, const int32_t* q_ranges, int q_blocks_max, cudaStream_t st) {
+// fp16 V as bytes, any strides: [B, H, N, 2 D], copied as 64 rows of 128 bytes (64 channels; x is 0 or 128); rows past N
+// read as zeros.
+static bool make_map_v16(CUtensorMap* m, const AttnArgs& a) {
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return false;
+  cuuint64_t dims[4] = {2 * (cuuint64_t)a.D, (cuuint64_t)a.N, (cuuint64_t)a.H, (cuuint64_t)a.B};
+  cuuint64_t strides[3] = {2 * (cuuint64_t)a.v_st[2], 2 * (cuuint64_t)a.v_st[1], 2 * (cuuint64_t)a.v_st[0]};
+  cuuint32_t box[4] = {128, 64, 1, 1};
+  cuuint32_t es[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(a.v), dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Function attributes are per device and outlive the call: set once for each (kernel, device).
+static bool attn_attributes(const void* kern, int smem, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return true;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+    return false;
+  if (dev < 64) done.fetch_or(bit, std::memory_order_release);
+  return true;
+}
+
+template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16>
+static int launch_attn(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, cudaStream_t st) {
   auto kern = attn_kernel<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16>;
   constexpr int smem = AttnShape<D, PVF16>::kSmemBytes;
-  // function attributes are per device: set on every call (cheap) rather than caching
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return SPARGE_ERR_CUDA;
-  cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  const int nq = (N + 127) / 128, nk = (N + 63) / 64;
-  const int gx = q_ranges ? min(q_blocks_max, nq) : nq;
-  kern<<<dim3(gx, BH), kAttnThreads, smem, st>>>(tq, tk, tv, (OutT*)o, lut, valid, pvthr, qs, ks, vs, status, N, H, nq, nk,
-                                                 sm_scale_log2, osb, osh, osn, pv_count, q_ranges);
-  return launch_status();
+  static std::atomic<uint64_t> done{0};
+  if (!attn_attributes((const void*)kern, smem, done)) return SPARGE_ERR_CUDA;
+  const int nq = (a.N + 127) / 128, nk = (a.N + 63) / 64;
+  const int gx = a.q_ranges ? min(a.q_blocks_max, nq) : nq;
+  const cudaError_t e = launch(kern, dim3(gx, a.B * a.H), kAttnThreads, smem, st, a.dependent, tq, tk, tv, (OutT*)a.o, a.lut,
+                               a.valid, a.pvthr, a.q_scale, a.k_scale, a.v_scale, a.dev_status, a.N, a.H, nq, nk,
+                               a.sm_scale * kLog2e, a.o_st[0], a.o_st[1], a.o_st[2], a.pv_count, a.q_ranges);
+  return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
+}
+
+// The checks are the callers'; fp16 V has per-block scales and the per-block skip test only.
+int attn_launch(const AttnArgs& a, cudaStream_t st) {
+  const int BH = a.B * a.H, n_pad = (a.N + 127) / 128 * 128;
+  CUtensorMap tq, tk, tv;
+  if (!make_map(&tq, a.q8, a.D, a.N, BH, 128) || !make_map(&tk, a.k8, a.D, a.N, BH, 64) ||
+      !(a.v_f16 ? make_map_v16(&tv, a) : make_map(&tv, a.v, a.D, n_pad, BH, 64)))
+    return SPARGE_ERR_CUDA;
+  const bool bf = a.out_dtype == SPARGE_BF16;
+#define SPARGE_ATTN_G(DD, C, S, G, F) \
+  (bf ? launch_attn<DD, C, S, __nv_bfloat16, G, F>(a, tq, tk, tv, st) : launch_attn<DD, C, S, __half, G, F>(a, tq, tk, tv, st))
+#define SPARGE_ATTN(DD, C, S) \
+  (a.gran == 3 ? SPARGE_ATTN_G(DD, C, S, 3, false) : a.gran == 2 ? SPARGE_ATTN_G(DD, C, S, 2, false) : SPARGE_ATTN_G(DD, C, S, 1, false))
+#define SPARGE_ATTN_S(DD, C) (a.pv_mode == 2 ? SPARGE_ATTN(DD, C, 2) : a.pv_mode == 1 ? SPARGE_ATTN(DD, C, 1) : SPARGE_ATTN(DD, C, 0))
+#define SPARGE_F16PV_S(DD, C) (a.pv_mode != 0 ? SPARGE_ATTN_G(DD, C, 1, 1, true) : SPARGE_ATTN_G(DD, C, 0, 1, true))
+  if (a.v_f16) {
+    if (a.D == 64) return a.causal ? SPARGE_F16PV_S(64, true) : SPARGE_F16PV_S(64, false);
+    return a.causal ? SPARGE_F16PV_S(128, true) : SPARGE_F16PV_S(128, false);
+  }
+  if (a.D == 64) return a.causal ? SPARGE_ATTN_S(64, true) : SPARGE_ATTN_S(64, false);
+  return a.causal ? SPARGE_ATTN_S(128, true) : SPARGE_ATTN_S(128, false);
+#undef SPARGE_F16PV_S
+#undef SPARGE_ATTN_S
+#undef SPARGE_ATTN
+#undef SPARGE_ATTN_G
 }
 
 // One warp waits on an mbarrier that nobody arrives at, with a caller-chosen short limit, and reports
@@ -756,28 +805,14 @@ extern "C" int sparge_attn_fwd_gran(const int8_t* q_int8, const int8_t* k_int8, 
   if (!(sm_scale > 0.f)) return SPARGE_ERR_INVALID_ARG;
   if ((long long)B * H > 65535) return SPARGE_ERR_TOO_LARGE;
   if (!strides_ok(o, o_stride_b, o_stride_h, o_stride_n)) return SPARGE_ERR_INVALID_ARG;
-  const int BH = B * H;
-  const int N_pad = (N + 127) / 128 * 128;
-  CUtensorMap tq, tk, tv;
-  if (!make_map(&tq, q_int8, D, N, BH, 128) || !make_map(&tk, k_int8, D, N, BH, 64) || !make_map(&tv, v8, D, N_pad, BH, 64))
-    return SPARGE_ERR_CUDA;
-  cudaStream_t st = (cudaStream_t)stream;
-  const float sl2 = sm_scale * kLog2e;
-  const bool causal = is_causal != 0, bf = out_dtype == SPARGE_BF16;
-#define SPARGE_ATTN_G(DD, C, S, T, G) \
-  launch_attn<DD, C, S, T, G>(tq, tk, tv, o, lut, valid, pvthreshd, q_scale, k_scale, v_scale, dev_status, BH, H, N, sl2, o_stride_b, o_stride_h, o_stride_n, pv_count, q_block_ranges, q_blocks_max, st)
-#define SPARGE_ATTN(DD, C, S, T) \
-  (qk_quant_gran == 3 ? SPARGE_ATTN_G(DD, C, S, T, 3) : qk_quant_gran == 2 ? SPARGE_ATTN_G(DD, C, S, T, 2) : SPARGE_ATTN_G(DD, C, S, T, 1))
-#define SPARGE_ATTN_T(DD, C, S) (bf ? SPARGE_ATTN(DD, C, S, __nv_bfloat16) : SPARGE_ATTN(DD, C, S, __half))
-#define SPARGE_ATTN_S(DD, C) \
-  (pv_threshold_mode == 2 ? SPARGE_ATTN_T(DD, C, 2) : pv_threshold_mode == 1 ? SPARGE_ATTN_T(DD, C, 1) : SPARGE_ATTN_T(DD, C, 0))
-#define SPARGE_ATTN_C(DD) (causal ? SPARGE_ATTN_S(DD, true) : SPARGE_ATTN_S(DD, false))
-  return D == 64 ? SPARGE_ATTN_C(64) : SPARGE_ATTN_C(128);
-#undef SPARGE_ATTN_C
-#undef SPARGE_ATTN_S
-#undef SPARGE_ATTN_T
-#undef SPARGE_ATTN
-#undef SPARGE_ATTN_G
+  AttnArgs a = {};
+  a.q8 = q_int8, a.k8 = k_int8, a.v = v8, a.o = o;
+  a.o_st[0] = o_stride_b, a.o_st[1] = o_stride_h, a.o_st[2] = o_stride_n;
+  a.lut = lut, a.valid = valid, a.pvthr = pvthreshd, a.q_scale = q_scale, a.k_scale = k_scale, a.v_scale = v_scale;
+  a.dev_status = dev_status, a.pv_count = pv_count, a.q_ranges = q_block_ranges, a.q_blocks_max = q_blocks_max;
+  a.B = B, a.H = H, a.N = N, a.D = D, a.out_dtype = out_dtype, a.causal = is_causal, a.gran = qk_quant_gran;
+  a.pv_mode = pv_threshold_mode, a.sm_scale = sm_scale;
+  return attn_launch(a, (cudaStream_t)stream);
 }
 
 extern "C" int sparge_attn_fwd_f16pv(const int8_t* q_int8, const int8_t* k_int8, const void* v_f16, void* o,
@@ -794,25 +829,15 @@ extern "C" int sparge_attn_fwd_f16pv(const int8_t* q_int8, const int8_t* k_int8,
   if (!(sm_scale > 0.f) || (reinterpret_cast<uintptr_t>(v_f16) & 15)) return SPARGE_ERR_INVALID_ARG;
   if ((long long)B * H > 65535) return SPARGE_ERR_TOO_LARGE;
   if (!strides_ok(o, o_stride_b, o_stride_h, o_stride_n)) return SPARGE_ERR_INVALID_ARG;
-  const int BH = B * H;
-  CUtensorMap tq, tk, tv;
-  // V as bytes: rows of 2 D bytes, copied 128 bytes (64 channels) at a time; rows past N read as zeros
-  if (!make_map(&tq, q_int8, D, N, BH, 128) || !make_map(&tk, k_int8, D, N, BH, 64) ||
-      !make_map(&tv, v_f16, 2 * (uint64_t)D, N, BH, 64, 128))
-    return SPARGE_ERR_CUDA;
-  cudaStream_t st = (cudaStream_t)stream;
-  const float sl2 = sm_scale * kLog2e;
-  const bool causal = is_causal != 0, bf = out_dtype == SPARGE_BF16, skip = pvthreshd != nullptr;
-#define SPARGE_F16PV(DD, C, S, T) \
-  launch_attn<DD, C, S, T, 1, true>(tq, tk, tv, o, lut, valid, pvthreshd, q_scale, k_scale, nullptr, dev_status, BH, H, N, sl2, o_stride_b, o_stride_h, o_stride_n, pv_count, q_block_ranges, q_blocks_max, st)
-#define SPARGE_F16PV_T(DD, C, S) (bf ? SPARGE_F16PV(DD, C, S, __nv_bfloat16) : SPARGE_F16PV(DD, C, S, __half))
-#define SPARGE_F16PV_S(DD, C) (skip ? SPARGE_F16PV_T(DD, C, 1) : SPARGE_F16PV_T(DD, C, 0))
-#define SPARGE_F16PV_C(DD) (causal ? SPARGE_F16PV_S(DD, true) : SPARGE_F16PV_S(DD, false))
-  return D == 64 ? SPARGE_F16PV_C(64) : SPARGE_F16PV_C(128);
-#undef SPARGE_F16PV_C
-#undef SPARGE_F16PV_S
-#undef SPARGE_F16PV_T
-#undef SPARGE_F16PV
+  AttnArgs a = {};
+  a.q8 = q_int8, a.k8 = k_int8, a.v = v_f16, a.v_f16 = true, a.o = o;
+  a.v_st[0] = (long long)H * N * D, a.v_st[1] = (long long)N * D, a.v_st[2] = D;
+  a.o_st[0] = o_stride_b, a.o_st[1] = o_stride_h, a.o_st[2] = o_stride_n;
+  a.lut = lut, a.valid = valid, a.pvthr = pvthreshd, a.q_scale = q_scale, a.k_scale = k_scale;
+  a.dev_status = dev_status, a.pv_count = pv_count, a.q_ranges = q_block_ranges, a.q_blocks_max = q_blocks_max;
+  a.B = B, a.H = H, a.N = N, a.D = D, a.out_dtype = out_dtype, a.causal = is_causal, a.gran = 1;
+  a.pv_mode = pvthreshd != nullptr, a.sm_scale = sm_scale;
+  return attn_launch(a, (cudaStream_t)stream);
 }
 
 extern "C" int sparge_attn_fwd_rows(const int8_t* q_int8, const int8_t* k_int8, const uint8_t* v8, void* o,

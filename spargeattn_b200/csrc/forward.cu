@@ -1,28 +1,28 @@
 // One call for the whole path of spas_sage2_attn_meansim_topk_cuda / spas_sage2_attn_meansim_cuda
-// (spas_sage_attn/core.py:39-169): K mean, pooling + self-similarity + INT8 quantisation of Q and K, block
-// selection + LUT, FP8 quantisation of V, block-sparse attention -- the sequence a host otherwise issues entry by
-// entry, here on one stream with every intermediate tensor carved out of one caller-provided workspace. It exists
-// for small problems, where issuing the nine launches from an interpreter costs more than running them.
-#include "common.cuh"
+// (spas_sage_attn/core.py:39-169), of their fp16-PV counterparts (:235-319) and of block_sparse_sage2_attn_cuda
+// (:171-233): K mean, pooling + self-similarity + INT8 quantisation of Q and K, V quantiser, block selection + LUT,
+// block-sparse attention, on one stream with every intermediate tensor carved out of one workspace. Four launches (five
+// from 2 049 tokens on), each a programmatic dependent of the one before it; issued entry by entry the path takes ten.
+#include "attn.cuh"
+#include "forward.cuh"
+#include "prep.cuh"
+#include "select.cuh"
 
 namespace sparge {
 
-enum { kWsKm, kWsScratch, kWsPq, kWsPk, kWsSimQ, kWsSimK, kWsQ8, kWsK8, kWsQs, kWsKs, kWsLut, kWsValid, kWsV8, kWsVs, kWsCount };
-
 static size_t round_up_256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Offsets of the workspace parts (each 256-byte aligned); returns the total size.
-static size_t forward_layout(int B, int H, int N, int D, size_t* off) {
+size_t forward_layout(int B, int H, int N, int D, int v_bytes_per_value, size_t* off) {
   const size_t BH = (size_t)B * H, nq = ((size_t)N + 127) / 128, nk = ((size_t)N + 63) / 64, npad = nq * 128;
   const size_t bytes[kWsCount] = {
       BH * D * 2,                                  // km
-      sparge_k_mean_scratch_bytes(B, H, N, D),     // k-mean partial sums
+      prep_scratch_bytes(B * H, N, D),             // partial sums and maxima
       BH * nq * D * 2, BH * nk * D * 2,            // pooled q, pooled k
       BH * nq, BH * nk,                            // self-similarity flags
       BH * (size_t)N * D, BH * (size_t)N * D,      // q_int8, k_int8
       BH * nq * 4, BH * nk * 4,                    // q_scale, k_scale
       BH * nq * nk * 4, BH * nq * 4,               // lut, valid
-      BH * npad * D, BH * D * 4};                  // v8, v_scale
+      BH * npad * D * v_bytes_per_value, BH * D * 4};   // v8 (or the fp16 copy of V), v_scale
   size_t total = 0;
   for (int i = 0; i < kWsCount; i++) {
     if (off) off[i] = total;
@@ -31,17 +31,79 @@ static size_t forward_layout(int B, int H, int N, int D, size_t* off) {
   return total;
 }
 
+int forward(const ForwardArgs& a, cudaStream_t st) {
+  if (!a.q || !a.k || !a.v || !a.o || !a.workspace) return SPARGE_ERR_NULL;
+  const bool select = a.mask == nullptr;
+  if (select && !a.simthr) return SPARGE_ERR_NULL;
+  if (select && (a.cdf == nullptr) == (a.topk == nullptr)) return SPARGE_ERR_INVALID_ARG;   // exactly one selection rule
+  if (a.B <= 0 || a.H <= 0 || a.N < 128 || (a.D != 64 && a.D != 128)) return SPARGE_ERR_INVALID_ARG;
+  if ((a.dtype != SPARGE_F16 && a.dtype != SPARGE_BF16) || (a.v_dtype != SPARGE_F16 && a.v_dtype != SPARGE_BF16))
+    return SPARGE_ERR_INVALID_ARG;
+  if (!select && a.mask_elem_size != 1 && a.mask_elem_size != 2 && a.mask_elem_size != 4 && a.mask_elem_size != 8)
+    return SPARGE_ERR_INVALID_ARG;
+  if (!(a.sm_scale > 0.f) || (a.q_ranges && a.q_blocks_max <= 0)) return SPARGE_ERR_INVALID_ARG;
+  if ((long long)a.B * a.H > 65535) return SPARGE_ERR_TOO_LARGE;
+  if (!strides_ok(a.q, a.q_st[0], a.q_st[1], a.q_st[2]) || !strides_ok(a.k, a.k_st[0], a.k_st[1], a.k_st[2]) ||
+      !strides_ok(a.v, a.v_st[0], a.v_st[1], a.v_st[2]) || !strides_ok(a.o, a.o_st[0], a.o_st[1], a.o_st[2]))
+    return SPARGE_ERR_INVALID_ARG;
+  if (reinterpret_cast<uintptr_t>(a.workspace) & 255) return SPARGE_ERR_INVALID_ARG;
+  const bool copy_v = forward_copies_v(a.pv_fp16, a.v_dtype, a.v_st);
+  size_t off[kWsCount];
+  if (a.workspace_bytes < forward_layout(a.B, a.H, a.N, a.D, copy_v ? 2 : a.pv_fp16 ? 0 : 1, off)) return SPARGE_ERR_INVALID_ARG;
+  uint8_t* ws = static_cast<uint8_t*>(a.workspace);
+  const int nq = (a.N + 127) / 128, nk = (a.N + 63) / 64;
+  int32_t *lut = (int32_t*)(ws + off[kWsLut]), *valid = (int32_t*)(ws + off[kWsValid]);
+
+  PrepArgs p = {};
+  p.q = a.q, p.k = a.k, p.v = a.v;
+  for (int i = 0; i < 3; i++) p.q_st[i] = a.q_st[i], p.k_st[i] = a.k_st[i], p.v_st[i] = a.v_st[i];
+  p.simthr = select ? a.simthr : nullptr;
+  p.pq = ws + off[kWsPq], p.pk = ws + off[kWsPk], p.sim_q = ws + off[kWsSimQ], p.sim_k = ws + off[kWsSimK];
+  p.q8 = (int8_t*)(ws + off[kWsQ8]), p.k8 = (int8_t*)(ws + off[kWsK8]);
+  p.qs = (float*)(ws + off[kWsQs]), p.ks = (float*)(ws + off[kWsKs]);
+  p.v_out = ws + off[kWsV8], p.v_scale = (float*)(ws + off[kWsVs]), p.km = ws + off[kWsKm], p.scratch = ws + off[kWsScratch];
+  p.BH = a.B * a.H, p.H = a.H, p.N = a.N, p.D = a.D, p.dtype = a.dtype, p.v_dtype = a.v_dtype, p.smooth_k = a.smooth_k;
+  p.v_mode = copy_v ? kVHalf : a.pv_fp16 ? kVNone : kVFp8;
+  int rc = prep_launch(p, st);
+  if (rc != SPARGE_OK) return rc;
+
+  if (select) {
+    // the skip test exempts the last two live blocks of the visiting order: best-first order only without it
+    const SelectArgs s = {p.pq, p.pk, p.sim_q, p.sim_k, a.topk, a.cdf, nullptr, lut, valid, p.BH, a.H, nq, nk, a.D, a.dtype,
+                          a.is_causal, a.sink, a.pvthr == nullptr, true};
+    rc = select_launch(s, st);
+  } else {
+    rc = mask_to_lut_launch(a.mask, a.mask_elem_size, lut, valid, (long long)p.BH * nq, nk, true, st);
+  }
+  if (rc != SPARGE_OK) return rc;
+
+  AttnArgs t = {};
+  t.q8 = p.q8, t.k8 = p.k8, t.o = a.o, t.lut = lut, t.valid = valid, t.pvthr = a.pvthr;
+  t.q_scale = p.qs, t.k_scale = p.ks, t.v_scale = p.v_scale, t.dev_status = a.dev_status;
+  t.v_f16 = a.pv_fp16;
+  t.v = a.pv_fp16 && !copy_v ? a.v : p.v_out;
+  const long long packed[3] = {(long long)a.H * a.N * a.D, (long long)a.N * a.D, a.D};
+  for (int i = 0; i < 3; i++) {
+    t.o_st[i] = a.o_st[i];
+    t.v_st[i] = copy_v ? packed[i] : a.v_st[i];
+  }
+  t.q_ranges = a.q_ranges, t.q_blocks_max = a.q_blocks_max, t.B = a.B, t.H = a.H, t.N = a.N, t.D = a.D;
+  t.out_dtype = a.dtype, t.causal = a.kernel_causal, t.gran = 1, t.pv_mode = a.pvthr != nullptr, t.dependent = true;
+  t.sm_scale = a.sm_scale;
+  return attn_launch(t, st);
+}
+
 }  // namespace sparge
 
 extern "C" size_t sparge_forward_workspace_bytes(int B, int H, int N, int D) {
   if (B <= 0 || H <= 0 || N <= 0 || (D != 64 && D != 128)) return 0;
-  return sparge::forward_layout(B, H, N, D, nullptr);
+  return sparge::forward_layout(B, H, N, D, 1, nullptr);
 }
 
 extern "C" int sparge_forward_workspace_layout(int B, int H, int N, int D, size_t* offsets, int n_offsets) {
   if (!offsets) return SPARGE_ERR_NULL;
   if (B <= 0 || H <= 0 || N <= 0 || (D != 64 && D != 128) || n_offsets != sparge::kWsCount) return SPARGE_ERR_INVALID_ARG;
-  sparge::forward_layout(B, H, N, D, offsets);
+  sparge::forward_layout(B, H, N, D, 1, offsets);
   return SPARGE_OK;
 }
 
@@ -51,41 +113,12 @@ extern "C" int sparge_meansim_forward(const void* q, const void* k, const void* 
                                       int v_dtype, int is_causal, int kernel_causal, int attention_sink, int smooth_k,
                                       float sm_scale, const long long* q_strides, const long long* k_strides,
                                       const long long* v_strides, const long long* o_strides, sparge_stream_t stream) {
-  using namespace sparge;
-  if (!q || !k || !v || !o || !simthreshd1 || !workspace || !q_strides || !k_strides || !v_strides || !o_strides)
-    return SPARGE_ERR_NULL;
-  if ((cdfthreshd == nullptr) == (topk == nullptr)) return SPARGE_ERR_INVALID_ARG;   // exactly one selection rule
-  if (B <= 0 || H <= 0 || N < 128 || (D != 64 && D != 128)) return SPARGE_ERR_INVALID_ARG;
-  if (reinterpret_cast<uintptr_t>(workspace) & 255) return SPARGE_ERR_INVALID_ARG;
-  size_t off[kWsCount];
-  if (workspace_bytes < forward_layout(B, H, N, D, off)) return SPARGE_ERR_INVALID_ARG;
-  uint8_t* ws = static_cast<uint8_t*>(workspace);
-  void* km = ws + off[kWsKm];
-  const int nq = (N + 127) / 128, nk = (N + 63) / 64;
-  int rc = SPARGE_OK;
-  if (smooth_k) {
-    rc = sparge_k_mean_strided(k, km, ws + off[kWsScratch], B, H, N, D, dtype, k_strides[0], k_strides[1], k_strides[2], stream);
-    if (rc != SPARGE_OK) return rc;
-  }
-  rc = sparge_pool_quant_strided(q, nullptr, simthreshd1, ws + off[kWsPq], ws + off[kWsSimQ], (int8_t*)(ws + off[kWsQ8]),
-                                 (float*)(ws + off[kWsQs]), B, H, N, D, 128, dtype, q_strides[0], q_strides[1], q_strides[2],
-                                 stream);
-  if (rc != SPARGE_OK) return rc;
-  rc = sparge_pool_quant_strided(k, smooth_k ? km : nullptr, simthreshd1, ws + off[kWsPk], ws + off[kWsSimK],
-                                 (int8_t*)(ws + off[kWsK8]), (float*)(ws + off[kWsKs]), B, H, N, D, 64, dtype, k_strides[0],
-                                 k_strides[1], k_strides[2], stream);
-  if (rc != SPARGE_OK) return rc;
-  // the skip test exempts the last two live blocks of the visiting order: best-first order only without it
-  rc = sparge_select(ws + off[kWsPq], ws + off[kWsPk], ws + off[kWsSimQ], ws + off[kWsSimK], topk, cdfthreshd, nullptr,
-                     (int32_t*)(ws + off[kWsLut]), (int32_t*)(ws + off[kWsValid]), B, H, nq, nk, D, dtype, is_causal,
-                     attention_sink, pvthreshd ? SPARGE_LUT_ASCENDING : SPARGE_LUT_BEST_FIRST, stream);
-  if (rc != SPARGE_OK) return rc;
-  rc = sparge_quant_v_strided(v, ws + off[kWsV8], (float*)(ws + off[kWsVs]), B, H, N, D, v_dtype, v_strides[0], v_strides[1],
-                              v_strides[2], stream);
-  if (rc != SPARGE_OK) return rc;
-  return sparge_attn_fwd_strided((const int8_t*)(ws + off[kWsQ8]), (const int8_t*)(ws + off[kWsK8]), ws + off[kWsV8], o,
-                                 (const int32_t*)(ws + off[kWsLut]), (const int32_t*)(ws + off[kWsValid]), pvthreshd,
-                                 (const float*)(ws + off[kWsQs]), (const float*)(ws + off[kWsKs]),
-                                 (const float*)(ws + off[kWsVs]), dev_status, B, H, N, D, dtype, kernel_causal, sm_scale,
-                                 o_strides[0], o_strides[1], o_strides[2], stream);
+  if (!simthreshd1 || !q_strides || !k_strides || !v_strides || !o_strides) return SPARGE_ERR_NULL;
+  sparge::ForwardArgs a = {};
+  a.q = q, a.k = k, a.v = v, a.o = o, a.simthr = simthreshd1, a.cdf = cdfthreshd, a.topk = topk, a.pvthr = pvthreshd;
+  for (int i = 0; i < 3; i++) a.q_st[i] = q_strides[i], a.k_st[i] = k_strides[i], a.v_st[i] = v_strides[i], a.o_st[i] = o_strides[i];
+  a.workspace = workspace, a.workspace_bytes = workspace_bytes, a.dev_status = dev_status;
+  a.B = B, a.H = H, a.N = N, a.D = D, a.dtype = dtype, a.v_dtype = v_dtype, a.is_causal = is_causal;
+  a.kernel_causal = kernel_causal, a.sink = attention_sink, a.smooth_k = smooth_k, a.sm_scale = sm_scale;
+  return sparge::forward(a, (cudaStream_t)stream);
 }

@@ -3,7 +3,7 @@
 // Replaces `k.mean(dim=-2, keepdim=True)` at spas_sage_attn/core.py:119-120.
 #include <mutex>
 
-#include "common.cuh"
+#include "column_passes.cuh"
 
 namespace sparge {
 
@@ -15,48 +15,15 @@ constexpr int kMeanRowsPerCta = 512;
 constexpr size_t kStaticScratchDoubles = SPARGE_K_MEAN_STATIC_MAX_BYTES / sizeof(double);
 static __device__ __align__(256) double g_kmean_static_scratch[kStaticScratchDoubles];
 
-// grid (chunks, B*H), 256 threads. Each thread owns 8 channels of every (256 / (D/8))-th row.
+// grid (chunks, B*H), 256 threads.
 template <typename T, int D>
-__global__ void __launch_bounds__(256) kmean_partial_kernel(const T* __restrict__ k, double* __restrict__ part, int N, int H,
-                                                            long long sb, long long sh, long long sn) {
-  constexpr int TPR = D / 8;        // threads per row
-  constexpr int RPP = 256 / TPR;    // rows per pass
-  __shared__ double red[RPP][D];
-  const int tid = threadIdx.x, cg = tid % TPR, r0 = tid / TPR;
-  const int chunk = blockIdx.x, bh = blockIdx.y, chunks = gridDim.x;
-  const int row_begin = chunk * kMeanRowsPerCta;
-  const int row_end = min(N, row_begin + kMeanRowsPerCta);
-  const T* base = k + (size_t)(bh / H) * sb + (size_t)(bh % H) * sh;
-  double acc[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) acc[i] = 0.0;
-  // Eight 128-bit loads in flight per thread: with one load per trip the kernel waited on memory with half of its
-  // issue slots idle (33.6 -> 27.5 us for a 100 MB tensor, 165 -> 137 us = 5.4 TB/s for an 890 MB one).
-  constexpr int KMEAN_UNROLL = 8;
-  int row = row_begin + r0;
-  for (; row + (KMEAN_UNROLL - 1) * RPP < row_end; row += KMEAN_UNROLL * RPP) {
-    Pack8<T> p[KMEAN_UNROLL];
-#pragma unroll
-    for (int u = 0; u < KMEAN_UNROLL; u++) p[u] = *reinterpret_cast<const Pack8<T>*>(base + (size_t)(row + u * RPP) * sn + cg * 8);
-#pragma unroll
-    for (int u = 0; u < KMEAN_UNROLL; u++)
-#pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] += (double)Elem<T>::to_float(p[u].v[i]);
-  }
-  for (; row < row_end; row += RPP) {
-    Pack8<T> p = *reinterpret_cast<const Pack8<T>*>(base + (size_t)row * sn + cg * 8);
-#pragma unroll
-    for (int i = 0; i < 8; i++) acc[i] += (double)Elem<T>::to_float(p.v[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < 8; i++) red[r0][cg * 8 + i] = acc[i];
-  __syncthreads();
-  if (tid < D) {
-    double s = 0.0;
-#pragma unroll 4
-    for (int r = 0; r < RPP; r++) s += red[r][tid];
-    part[((size_t)bh * chunks + chunk) * D + tid] = s;
-  }
+__global__ void __launch_bounds__(kPassThreads) kmean_partial_kernel(const T* __restrict__ k, double* __restrict__ part, int N, int H,
+                                                                     long long sb, long long sh, long long sn) {
+  __shared__ double red[PassShape<D>::kRowsPerPass][D];
+  const int chunk = blockIdx.x, bh = blockIdx.y, row_begin = chunk * kMeanRowsPerCta;
+  const double s = column_sum<T, D>(red, k + (size_t)(bh / H) * sb + (size_t)(bh % H) * sh, row_begin,
+                                    min(N, row_begin + kMeanRowsPerCta), sn);
+  if (threadIdx.x < D) part[((size_t)bh * gridDim.x + chunk) * D + threadIdx.x] = s;
 }
 
 // grid (B*H), D threads.
@@ -72,7 +39,7 @@ template <typename T, int D>
 static int launch_kmean(const void* k, void* km, void* scratch, int BH, int H, int N, long long sb, long long sh,
                         long long sn, cudaStream_t st) {
   const int chunks = (N + kMeanRowsPerCta - 1) / kMeanRowsPerCta;
-  kmean_partial_kernel<T, D><<<dim3(chunks, BH), 256, 0, st>>>((const T*)k, (double*)scratch, N, H, sb, sh, sn);
+  kmean_partial_kernel<T, D><<<dim3(chunks, BH), kPassThreads, 0, st>>>((const T*)k, (double*)scratch, N, H, sb, sh, sn);
   kmean_final_kernel<T, D><<<BH, D, 0, st>>>((const double*)scratch, (T*)km, N, chunks);
   return launch_status();
 }

@@ -9,120 +9,43 @@
 // Output is token-major [B,H,N_pad,D] with zero rows beyond N: the tcgen05 PV MMA takes V as an
 // MN-major B operand straight from that layout, so no transposed copy is made.
 // An all-zero channel is emitted as zeros (the reference produces NaN there).
-#include "common.cuh"
-#include "sm100_ptx.cuh"
+#include "column_passes.cuh"
 
 namespace sparge {
 
 constexpr int kVRowsPerCta = 256;
-constexpr float kVScaleMax = 2.25f;   // spas_sage_attn/core.py:151
-
-// a / b as fused.cu computes it under --use_fast_math
-__device__ __forceinline__ float div_approx(float a, float b) {
-  float q;
-  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(a), "f"(b));
-  return q;
-}
 
 __global__ void div_approx_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = div_approx(a[i], b[i]);
 }
 
-template <typename T>
-__device__ __forceinline__ float to_f16_value(T v);
-template <>
-__device__ __forceinline__ float to_f16_value<__half>(__half v) { return __half2float(v); }
-template <>
-__device__ __forceinline__ float to_f16_value<__nv_bfloat16>(__nv_bfloat16 v) {
-  return __half2float(__float2half_rn(__bfloat162float(v)));
-}
-
 // grid (chunks, B*H), 256 threads. amax accumulates as the bit pattern of a non-negative float.
 template <typename T, int D>
-__global__ void __launch_bounds__(256) v_amax_kernel(const T* __restrict__ v, unsigned int* __restrict__ amax_bits, int N, int H,
-                                                     long long sb, long long sh, long long sn) {
-  constexpr int TPR = D / 8, RPP = 256 / TPR;
-  __shared__ float red[RPP][D];
-  const int tid = threadIdx.x, cg = tid % TPR, r0 = tid / TPR;
-  const int bh = blockIdx.y;
-  const int row_begin = blockIdx.x * kVRowsPerCta, row_end = min(N, row_begin + kVRowsPerCta);
-  const T* base = v + (size_t)(bh / H) * sb + (size_t)(bh % H) * sh;
-  float mx[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) mx[i] = 0.f;
-#ifndef VQ_UNROLL
-#define VQ_UNROLL 4
-#endif
-  int row = row_begin + r0;
-  for (; row + (VQ_UNROLL - 1) * RPP < row_end; row += VQ_UNROLL * RPP) {   // several 128-bit loads in flight per thread
-    Pack8<T> p[VQ_UNROLL];
-#pragma unroll
-    for (int u = 0; u < VQ_UNROLL; u++) p[u] = *reinterpret_cast<const Pack8<T>*>(base + (size_t)(row + u * RPP) * sn + cg * 8);
-#pragma unroll
-    for (int u = 0; u < VQ_UNROLL; u++)
-#pragma unroll
-      for (int i = 0; i < 8; i++) mx[i] = fmaxf(mx[i], fabsf(to_f16_value<T>(p[u].v[i])));
-  }
-  for (; row < row_end; row += RPP) {
-    Pack8<T> p = *reinterpret_cast<const Pack8<T>*>(base + (size_t)row * sn + cg * 8);
-#pragma unroll
-    for (int i = 0; i < 8; i++) mx[i] = fmaxf(mx[i], fabsf(to_f16_value<T>(p.v[i])));
-  }
-#pragma unroll
-  for (int i = 0; i < 8; i++) red[r0][cg * 8 + i] = mx[i];
-  __syncthreads();
-  if (tid < D) {
-    float m = 0.f;
-#pragma unroll 4
-    for (int r = 0; r < RPP; r++) m = fmaxf(m, red[r][tid]);
-    atomicMax(amax_bits + (size_t)bh * D + tid, __float_as_uint(m));
-  }
+__global__ void __launch_bounds__(kPassThreads) v_amax_kernel(const T* __restrict__ v, unsigned int* __restrict__ amax_bits, int N,
+                                                              int H, long long sb, long long sh, long long sn) {
+  __shared__ float red[PassShape<D>::kRowsPerPass][D];
+  const int bh = blockIdx.y, row_begin = blockIdx.x * kVRowsPerCta;
+  const float m = column_amax<T, D>(red, v + (size_t)(bh / H) * sb + (size_t)(bh % H) * sh, row_begin,
+                                    min(N, row_begin + kVRowsPerCta), sn);
+  if (threadIdx.x < D) atomicMax(amax_bits + (size_t)bh * D + threadIdx.x, __float_as_uint(m));
 }
 
 // grid (ceil(N_pad / rows), B*H), 256 threads.
 template <typename T, int D>
-__global__ void __launch_bounds__(256) v_quant_kernel(const T* __restrict__ v, const float* __restrict__ amax,
-                                                      uint8_t* __restrict__ v8, int N, int N_pad, int H,
-                                                      long long sb, long long sh, long long sn) {
-  constexpr int TPR = D / 8, RPP = 256 / TPR;
-  const int tid = threadIdx.x, cg = tid % TPR, r0 = tid / TPR;
-#ifndef VQ_REVERSE
-#define VQ_REVERSE 1
-#endif
+__global__ void __launch_bounds__(kPassThreads) v_quant_kernel(const T* __restrict__ v, const float* __restrict__ amax,
+                                                               uint8_t* __restrict__ v8, int N, int N_pad, int H,
+                                                               long long sb, long long sh, long long sn) {
+  const int cg = threadIdx.x % PassShape<D>::kThreadsPerRow;
   // The amax pass has just read V front to back; this pass walks it back to front, so that it starts with the
   // rows that are still in L2 (a tensor larger than the cache would be re-read from DRAM in full either way).
-  const int bh = VQ_REVERSE ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
-  const int chunk = VQ_REVERSE ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
-  const int row_begin = chunk * kVRowsPerCta, row_end = min(N_pad, row_begin + kVRowsPerCta);
-  float r[8];
+  const int bh = gridDim.y - 1 - blockIdx.y;
+  const int row_begin = (gridDim.x - 1 - blockIdx.x) * kVRowsPerCta;
+  float r8[8];
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const float a = amax[(size_t)bh * D + cg * 8 + i];
-    r[i] = a > 0.f ? div_approx(kVScaleMax, a) : 0.f;
-  }
-  const T* base = v + (size_t)(bh / H) * sb + (size_t)(bh % H) * sh;
-  uint8_t* out = v8 + (size_t)bh * N_pad * D;
-  auto quantise = [&](const Pack8<T>& p) {
-    float f[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) f[i] = __fmul_rn(to_f16_value<T>(p.v[i]), r[i]);
-    return make_uint2(cvt_e4m3x4(f[0], f[1], f[2], f[3]), cvt_e4m3x4(f[4], f[5], f[6], f[7]));
-  };
-  int row = row_begin + r0;
-  const int full_end = min(row_end, N);                  // rows below N hold data, the rest of the pad is zeros
-  for (; row + (VQ_UNROLL - 1) * RPP < full_end; row += VQ_UNROLL * RPP) {
-    Pack8<T> p[VQ_UNROLL];
-#pragma unroll
-    for (int u = 0; u < VQ_UNROLL; u++) p[u] = *reinterpret_cast<const Pack8<T>*>(base + (size_t)(row + u * RPP) * sn + cg * 8);
-#pragma unroll
-    for (int u = 0; u < VQ_UNROLL; u++) *reinterpret_cast<uint2*>(out + (size_t)(row + u * RPP) * D + cg * 8) = quantise(p[u]);
-  }
-  for (; row < row_end; row += RPP) {
-    uint2 w = make_uint2(0u, 0u);
-    if (row < N) w = quantise(*reinterpret_cast<const Pack8<T>*>(base + (size_t)row * sn + cg * 8));
-    *reinterpret_cast<uint2*>(out + (size_t)row * D + cg * 8) = w;
-  }
+  for (int i = 0; i < 8; i++) r8[i] = v_multiplier(amax[(size_t)bh * D + cg * 8 + i]);
+  v_quant_rows<T, D>(v + (size_t)(bh / H) * sb + (size_t)(bh % H) * sh, v8 + (size_t)bh * N_pad * D, r8, row_begin,
+                     min(N_pad, row_begin + kVRowsPerCta), N, sn);
 }
 
 __global__ void v_scale_final_kernel(float* __restrict__ v_scale, int n) {
@@ -135,8 +58,8 @@ static int launch_quant_v(const void* v, uint8_t* v8, float* v_scale, int BH, in
                           long long sn, cudaStream_t st) {
   const int N_pad = (N + 127) / 128 * 128;
   if (cudaMemsetAsync(v_scale, 0, (size_t)BH * D * sizeof(float), st) != cudaSuccess) return SPARGE_ERR_CUDA;
-  v_amax_kernel<T, D><<<dim3((N + kVRowsPerCta - 1) / kVRowsPerCta, BH), 256, 0, st>>>((const T*)v, (unsigned int*)v_scale, N, H, sb, sh, sn);
-  v_quant_kernel<T, D><<<dim3((N_pad + kVRowsPerCta - 1) / kVRowsPerCta, BH), 256, 0, st>>>((const T*)v, v_scale, v8, N, N_pad, H, sb, sh, sn);
+  v_amax_kernel<T, D><<<dim3((N + kVRowsPerCta - 1) / kVRowsPerCta, BH), kPassThreads, 0, st>>>((const T*)v, (unsigned int*)v_scale, N, H, sb, sh, sn);
+  v_quant_kernel<T, D><<<dim3((N_pad + kVRowsPerCta - 1) / kVRowsPerCta, BH), kPassThreads, 0, st>>>((const T*)v, v_scale, v8, N, N_pad, H, sb, sh, sn);
   v_scale_final_kernel<<<(BH * D + 255) / 256, 256, 0, st>>>(v_scale, BH * D);
   return launch_status();
 }

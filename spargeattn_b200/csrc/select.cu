@@ -20,7 +20,8 @@
 //            probabilities themselves agree; clamped to [1, nk].
 #include <cfloat>
 
-#include "common.cuh"
+#include "launch.cuh"
+#include "select.cuh"
 
 namespace sparge {
 
@@ -113,6 +114,7 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
               uint8_t* __restrict__ mask, int32_t* __restrict__ lut, int32_t* __restrict__ valid, int H, int nq, int nk,
               int is_causal, int sink, int rows_per_cta, int best_first, int scan_log_nx, int cdf_len) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int qi = blockIdx.x * rows_per_cta + warp, bh = blockIdx.y, h = bh % H;
   const bool active = warp < rows_per_cta && qi < nq;       // inactive warps still help to stage K tiles
@@ -321,6 +323,7 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
     lrow[r] = vv;
   }
   if (lane == 0) valid[(size_t)bh * nq + qi] = live_seen;
+  pdl_trigger();
 }
 
 // One CTA per mask row: compaction of a user block mask into the LUT.
@@ -353,18 +356,20 @@ __global__ void __launch_bounds__(kSelThreads) mask_to_lut_kernel(const uint8_t*
   }
   __syncthreads();
   write_lut_row(s_idx, live_seen, nk, lut + row * (size_t)nk, valid + row);
+  // nothing here depends on the kernels before this one, but the kernel after it relies on them too: it is released by
+  // this one's end
+  pdl_wait();
+  pdl_trigger();
 }
 
 template <typename T, int D>
-static int launch_select(const void* pq, const void* pk, const uint8_t* sim_q, const uint8_t* sim_k, const float* topk,
-                         const float* cdf, uint8_t* mask, int32_t* lut, int32_t* valid, int BH, int H, int nq, int nk,
-                         int causal, int sink, int best_first, cudaStream_t st) {
+static int launch_select(const SelectArgs& a, cudaStream_t st) {
   // cdf mode reproduces torch.cumsum over the [B*H*nq, nk] matrix of sorted probabilities: the scan's chunking
   // depends on both extents
-  const int scan_log_nx = aten_scan_log_threads_x((uint32_t)BH * (uint32_t)nq, (uint32_t)nk);
+  const int scan_log_nx = aten_scan_log_threads_x((uint32_t)a.BH * (uint32_t)a.nq, (uint32_t)a.nk);
   const int scan_w = 2 << scan_log_nx;
-  const int cdf_len = cdf ? (nk + scan_w - 1) / scan_w * scan_w : 0;
-  const size_t row_bytes = select_row_bytes(nk, D, cdf_len);
+  const int cdf_len = a.cdf ? (a.nk + scan_w - 1) / scan_w * scan_w : 0;
+  const size_t row_bytes = select_row_bytes(a.nk, D, cdf_len);
   const size_t tile_bytes = 32 * (D * sizeof(T) + 16);
   const size_t budget = 200 * 1024 - tile_bytes;
   if (row_bytes > budget) return SPARGE_ERR_TOO_LARGE;
@@ -375,10 +380,28 @@ static int launch_select(const void* pq, const void* pk, const uint8_t* sim_q, c
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return SPARGE_ERR_CUDA;
   }
-  kern<<<dim3((nq + rows - 1) / rows, BH), kSelRowsPerCta * 32, smem, st>>>(
-      (const T*)pq, (const T*)pk, sim_q, sim_k, topk, cdf, mask, lut, valid, H, nq, nk, causal, sink, rows, best_first,
-      scan_log_nx, cdf_len);
-  return launch_status();
+  const cudaError_t e = launch(kern, dim3((a.nq + rows - 1) / rows, a.BH), kSelRowsPerCta * 32, smem, st, a.dependent,
+                               (const T*)a.pq, (const T*)a.pk, a.sim_q, a.sim_k, a.topk, a.cdf, a.mask, a.lut, a.valid, a.H, a.nq,
+                               a.nk, a.causal, a.sink, rows, a.best_first, scan_log_nx, cdf_len);
+  return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
+}
+
+int select_launch(const SelectArgs& a, cudaStream_t st) {
+  if (a.dtype == SPARGE_F16) return a.D == 64 ? launch_select<__half, 64>(a, st) : launch_select<__half, 128>(a, st);
+  return a.D == 64 ? launch_select<__nv_bfloat16, 64>(a, st) : launch_select<__nv_bfloat16, 128>(a, st);
+}
+
+int mask_to_lut_launch(const void* mask, int elem_size, int32_t* lut, int32_t* valid, long long rows, int nk, bool dependent,
+                       cudaStream_t st) {
+  const size_t smem = (size_t)nk * sizeof(int);
+  if (smem > 200 * 1024 || rows > 2147483647LL) return SPARGE_ERR_TOO_LARGE;
+  if (smem > 48 * 1024) {
+    if (cudaFuncSetAttribute(mask_to_lut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return SPARGE_ERR_CUDA;
+  }
+  const cudaError_t e = launch(mask_to_lut_kernel, dim3((unsigned)rows), kSelThreads, smem, st, dependent, (const uint8_t*)mask,
+                               elem_size, lut, valid, nk);
+  return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
 }
 
 }  // namespace sparge
@@ -393,13 +416,9 @@ extern "C" int sparge_select(const void* pq, const void* pk, const uint8_t* sim_
   if (B <= 0 || H <= 0 || nq <= 0 || nk <= 0 || (D != 64 && D != 128) || (dtype != SPARGE_F16 && dtype != SPARGE_BF16))
     return SPARGE_ERR_INVALID_ARG;
   if ((long long)B * H > 65535) return SPARGE_ERR_TOO_LARGE;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int BH = B * H;
-#define SPARGE_SEL(T, DD) \
-  launch_select<T, DD>(pq, pk, sim_q, sim_k, topk, cdfthreshd, mask, lut, valid, BH, H, nq, nk, is_causal, attention_sink, lut_order != 0, st)
-  if (dtype == SPARGE_F16) return D == 64 ? SPARGE_SEL(__half, 64) : SPARGE_SEL(__half, 128);
-  return D == 64 ? SPARGE_SEL(__nv_bfloat16, 64) : SPARGE_SEL(__nv_bfloat16, 128);
-#undef SPARGE_SEL
+  const SelectArgs a = {pq, pk, sim_q, sim_k, topk, cdfthreshd, mask, lut, valid, B * H, H, nq, nk, D, dtype, is_causal,
+                        attention_sink, lut_order != 0, false};
+  return select_launch(a, (cudaStream_t)stream);
 }
 
 extern "C" int sparge_mask_to_lut(const void* mask, int elem_size, int32_t* lut, int32_t* valid, int B, int H, int nq,
@@ -408,15 +427,5 @@ extern "C" int sparge_mask_to_lut(const void* mask, int elem_size, int32_t* lut,
   if (!mask || !lut || !valid) return SPARGE_ERR_NULL;
   if (B <= 0 || H <= 0 || nq <= 0 || nk <= 0 || (elem_size != 1 && elem_size != 2 && elem_size != 4 && elem_size != 8))
     return SPARGE_ERR_INVALID_ARG;
-  const size_t smem = (size_t)nk * sizeof(int);
-  if (smem > 200 * 1024) return SPARGE_ERR_TOO_LARGE;
-  const long long rows = (long long)B * H * nq;
-  if (rows > 2147483647LL) return SPARGE_ERR_TOO_LARGE;
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(mask_to_lut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return SPARGE_ERR_CUDA;
-  }
-  mask_to_lut_kernel<<<(unsigned)rows, kSelThreads, smem, (cudaStream_t)stream>>>((const uint8_t*)mask, elem_size, lut,
-                                                                                    valid, nk);
-  return launch_status();
+  return mask_to_lut_launch(mask, elem_size, lut, valid, (long long)B * H * nq, nk, false, (cudaStream_t)stream);
 }

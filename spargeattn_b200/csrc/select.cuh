@@ -1,0 +1,21 @@
+// Launches of the block selection (select.cu) for the C entry points.
+#pragma once
+#include "common.cuh"
+
+namespace sparge {
+
+struct SelectArgs {
+  const void *pq, *pk;              // pooled [B,H,nq,D], [B,H,nk,D]
+  const uint8_t *sim_q, *sim_k;
+  const float *topk, *cdf;          // [H], exactly one
+  uint8_t* mask;                    // [B,H,nq,nk] or NULL
+  int32_t *lut, *valid;
+  int BH, H, nq, nk, D, dtype, causal, sink, best_first;
+  bool dependent;                   // programmatic launch behind the kernel before it on the stream
+};
+int select_launch(const SelectArgs& a, cudaStream_t st);
+
+int mask_to_lut_launch(const void* mask, int elem_size, int32_t* lut, int32_t* valid, long long rows, int nk, bool dependent,
+                       cudaStream_t st);
+
+}  // namespace sparge
