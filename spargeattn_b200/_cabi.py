@@ -16,6 +16,10 @@ if not os.path.exists(LIB_PATH):
 
 lib = ctypes.CDLL(LIB_PATH)
 
+import torch  # noqa: E402,F401  (its libraries have to be loaded before the binding's)
+
+from . import _binding  # noqa: E402,F401  (a missing module raises here: it is built beside the library)
+
 _p, _i, _f, _sz, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_size_t, ctypes.c_longlong
 
 # name -> (restype, argtypes); must list every symbol of include/sparge_b200.h

@@ -1,4 +1,5 @@
-"""Builds libsparge_b200.so in-tree with nvcc for sm_100a (no other architecture is targeted).
+"""Builds libsparge_b200.so in-tree with nvcc for sm_100a (no other architecture is targeted), and _binding.so, the host
+code between Python and it, with g++ against PyTorch's headers.
 
     python spargeattn_b200/build.py [--force] [--verbose]
 """
@@ -10,6 +11,7 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libsparge_b200.so")
+BINDING = os.path.join(HERE, "_binding.so")
 SOURCES = ["cabi.cu", "kmean.cu", "pool_quant.cu", "prep.cu", "select.cu", "quant_v.cu", "attn_sm100.cu", "peer.cu", "tensor_peak.cu",
            "forward.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
@@ -26,6 +28,23 @@ def _stale(target, deps):
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _build_binding(headers, force):
+    src = os.path.join(CSRC, "binding.cpp")
+    if not (force or _stale(BINDING, [src] + headers)):
+        return
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [f"-isystem{p}" for p in include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]]
+    cmd += [src, "-o", BINDING, LIB, "-Wl,-rpath,$ORIGIN"] + [f"-L{p}" for p in library_paths()]
+    cmd += ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for binding.cpp:\n{r.stdout}\n{r.stderr}")
 
 
 def build(force=False, verbose=False):
@@ -48,9 +67,10 @@ def build(force=False, verbose=False):
     with ThreadPoolExecutor(max_workers=6) as ex:
         objs = list(ex.map(compile_one, SOURCES))
     if force or _stale(LIB, objs):
-        r = subprocess.run([_nvcc(), "-shared", "-o", LIB] + objs + ["-lcudart"], capture_output=True, text=True)
+        r = subprocess.run([_nvcc(), "-shared", "-Xlinker", "-soname=libsparge_b200.so", "-o", LIB] + objs + ["-lcudart"], capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_binding(headers, force)
     return LIB
 
 

@@ -13,6 +13,7 @@ Differences from the reference, all deliberate:
 import torch
 
 from . import ops
+from ._cabi import _binding
 
 # The reference's Sage2 entry points pass the literal False in the kernel's is_causal slot
 # (spas_sage_attn/core.py:154-158, :221-225): causality is enforced per block by the predictor
@@ -109,9 +110,10 @@ _SIDE_STREAMS = {}
 # worsen. Hence the window, in (batch * heads * tokens) rows.
 CONCURRENT_PREP_MIN_ROWS = 16384
 CONCURRENT_PREP_MAX_ROWS = 163840
-# Below the window the whole path is issued by one C call (sparge_meansim_forward): 0.14 ms of a [1, 4, 2048, 64] call
-# were the interpreter walking through nine wrappers.
-SINGLE_CALL_MAX_ROWS = CONCURRENT_PREP_MIN_ROWS
+# Calls of fewer (batch * heads * tokens) rows than this are issued by one native call (forward.cu: four or five launches
+# on one workspace) -- all of them: it is faster at every size (0.067 -> 0.03 ms at [1, 4, 2048, 64]). The sequence of
+# separate entries below it gives the same bytes; it is what a caller composes who wants the intermediate tensors.
+SINGLE_CALL_MAX_ROWS = 1 << 62
 
 
 def _side_streams(device):
@@ -196,12 +198,9 @@ def block_map_lut_triton(block_map):
     return ops.mask_to_lut(block_map)
 
 
-def _sparsity(valid_block_num, lut, causal_denominator):
-    """spas_sage_attn/core.py:162-167, :229-231."""
-    if not causal_denominator:
-        denom = lut.size(3) * lut.size(2) * lut.size(0) * lut.size(1)
-    else:
-        denom = (lut.size(3) + 2) // 2 * lut.size(2) * lut.size(0) * lut.size(1)
+def _sparsity(valid_block_num, nk, causal_denominator):
+    """spas_sage_attn/core.py:162-167, :229-231. valid_block_num: [B, H, query blocks]; nk: key blocks."""
+    denom = ((nk + 2) // 2 if causal_denominator else nk) * valid_block_num.numel()
     return (1 - (valid_block_num.float().sum()) / denom).item()
 
 
@@ -216,25 +215,20 @@ def _meansim_attention(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthre
     headdim = q.size(-1)
     assert headdim in [64, 128], "headdim should be in [64, 128]. For other headdim, you can use padding and specify the softmax scale."
     rows = q.size(0) * q.size(1) * q.size(2)
-    if rows < SINGLE_CALL_MAX_ROWS and q_block_ranges is None and not pv_fp16:
-        # a handful of short launches: issued by one C call, the interpreter's share of the time is what matters here
-        B_, H_, N_, _ = q.shape
-        thr = hyperparameter_check(simthreshd1, H_, q.device)
-        cdf = None if cdfthreshd is None else hyperparameter_check(cdfthreshd, H_, q.device)
-        tk = None if topk is None else hyperparameter_check(topk, H_, q.device)
-        assert (cdf is None) != (tk is None), "Only one of cdfthreshd and topk can be set."
+    if rows < SINGLE_CALL_MAX_ROWS:
+        H_, nq, nk = q.size(1), (q.size(2) + 127) // 128, (q.size(2) + 63) // 64
+        ready = lambda x: None if x is None else hyperparameter_check(x, H_, q.device)
+        assert (cdfthreshd is None) != (topk is None), "Only one of cdfthreshd and topk can be set."
         pv = _pv_threshold_tensor(pvthreshd, H_, q.device)
-        o, ws, offs = ops.meansim_forward(q, k, v, _empty_like_layout(q), thr, cdf, tk, pv,
-                                          scale if scale is not None else 1.0 / (headdim ** 0.5), bool(is_causal),
-                                          kernel_causal, attention_sink, smooth_k)
-        if tensor_layout == 'NHD':
-            o = o.transpose(-2, -3)
-        if return_sparsity:
-            nq, nk = (N_ + 127) // 128, (N_ + 63) // 64
-            valid = ws[offs["valid"]:offs["valid"] + B_ * H_ * nq * 4].view(torch.int32)
-            denom = nk * nq * B_ * H_ if is_causal is False else (nk + 2) // 2 * nq * B_ * H_     # core.py:162-167
-            return o, (1 - valid.float().sum() / denom).item()
-        return o
+        ops.device_status_word(q.device)
+        r = _binding.forward(q, k, v, None, ready(simthreshd1), ready(cdfthreshd), ready(topk),
+                             PV_SKIP_NEVER_FIRES_FROM if pv is None else pv, scale, bool(is_causal), kernel_causal,
+                             attention_sink, smooth_k, pv_fp16, "HND", q_block_ranges, q_blocks_max, return_sparsity)
+        if r is not None:
+            o, valid = r if return_sparsity else (r, None)
+            if tensor_layout == 'NHD':
+                o = o.transpose(-2, -3)
+            return (o, _sparsity(valid, nk, is_causal is not False)) if return_sparsity else o
     beside = CONCURRENT_PREP_MIN_ROWS <= rows <= CONCURRENT_PREP_MAX_ROWS
     s_q, s_v = _side_streams(q.device) if beside else (None, None)
     if pv_fp16:
@@ -265,72 +259,116 @@ def _meansim_attention(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthre
     if tensor_layout == 'NHD':
         o = o.transpose(-2, -3)
     if return_sparsity:
-        return o, _sparsity(valid_block_num, lut, is_causal is not False)
+        return o, _sparsity(valid_block_num, lut.size(3), is_causal is not False)
     return o
 
 
-@torch.compiler.disable
+# The public functions hand their arguments to the native call as they are; it takes the ordinary ones (fp16 / bf16 CUDA
+# tensors that can be read in place, knobs that are numbers or ready tensors) and returns None for everything else, which
+# the general path then converts, or complains about. The general path is closed to the tracing compiler; the public
+# frames are skipped by it, which costs a call nothing.
+_meansim_general = torch.compiler.disable(_meansim_attention)
+_skip_frame = torch.compiler.disable(recursive=False)
+
+
+@_skip_frame
 def spas_sage2_attn_meansim_cuda(q, k, v, attn_mask=None, dropout_p=0.0, is_causal=False, scale=None, smooth_k=True,
                                  simthreshd1=0.6, cdfthreshd=0.98, pvthreshd=50, attention_sink=False,
                                  tensor_layout="HND", output_dtype=torch.float16, return_sparsity=False):
     """spas_sage_attn/core.py:39-103 -- cdf-threshold selection, INT8 QK / FP8 PV."""
-    return _meansim_attention(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, None, pvthreshd,
-                              attention_sink, tensor_layout, return_sparsity,
-                              bool(is_causal) and SAGE2_TOKEN_LEVEL_CAUSAL)
+    kernel_causal = SAGE2_TOKEN_LEVEL_CAUSAL and bool(is_causal)
+    if not return_sparsity and SINGLE_CALL_MAX_ROWS:
+        o = _binding.forward(q, k, v, None, simthreshd1, cdfthreshd, None, pvthreshd, scale, is_causal, kernel_causal,
+                             attention_sink, smooth_k, False, tensor_layout, None, 0, False)
+        if o is not None:
+            return o
+    return _meansim_general(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, None, pvthreshd, attention_sink,
+                            tensor_layout, return_sparsity, kernel_causal)
 
 
-@torch.compiler.disable
+@_skip_frame
 def spas_sage2_attn_meansim_topk_cuda(q, k, v, attn_mask=None, dropout_p=0.0, is_causal=False, scale=None,
                                       smooth_k=True, simthreshd1=-0.1, cdfthreshd=None, topk=0.5, pvthreshd=50,
                                       attention_sink=False, tensor_layout="HND", output_dtype=torch.float16,
                                       return_sparsity=False):
     """spas_sage_attn/core.py:105-169 -- top-k selection, INT8 QK / FP8 PV."""
-    return _meansim_attention(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, topk, pvthreshd,
-                              attention_sink, tensor_layout, return_sparsity,
-                              bool(is_causal) and SAGE2_TOKEN_LEVEL_CAUSAL)
+    kernel_causal = SAGE2_TOKEN_LEVEL_CAUSAL and bool(is_causal)
+    if not return_sparsity and SINGLE_CALL_MAX_ROWS:
+        o = _binding.forward(q, k, v, None, simthreshd1, cdfthreshd, topk, pvthreshd, scale, is_causal, kernel_causal,
+                             attention_sink, smooth_k, False, tensor_layout, None, 0, False)
+        if o is not None:
+            return o
+    return _meansim_general(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, topk, pvthreshd, attention_sink,
+                            tensor_layout, return_sparsity, kernel_causal)
 
 
 @torch.compiler.disable
+def _block_sparse_general(q, k, v, mask_id, scale, smooth_k, pvthreshd, tensor_layout, return_sparsity):
+    q, k, v = _prologue(q, k, v, tensor_layout)
+    headdim = q.size(-1)
+    assert mask_id is not None, "mask_id is required"
+    assert mask_id.dim() == 4 and mask_id.is_contiguous()
+    assert headdim in [64, 128], "headdim should be in [64, 128]. For other headdim, you can use padding and specify the softmax scale."
+    if mask_id.dtype.is_floating_point:
+        mask_id = mask_id != 0                            # -0.0 must count as false
+    pvthreshd = _pv_threshold_tensor(pvthreshd, q.size(-3), q.device)
+    ops.device_status_word(q.device)
+    r = _binding.forward(q, k, v, mask_id, None, None, None, PV_SKIP_NEVER_FIRES_FROM if pvthreshd is None else pvthreshd, scale,
+                         False, False, False, smooth_k, False, "HND", None, 0, return_sparsity)
+    if r is not None:
+        o, valid_block_num = r if return_sparsity else (r, None)
+    else:                                                 # e.g. a mask of another shape than this problem's
+        km = ops.k_mean(k) if smooth_k else None
+        q_int8, q_scale, k_int8, k_scale = get_vanilla_qk_quant(q, k, km, 128, 64)
+        lut, valid_block_num = block_map_lut_triton(block_map=mask_id)
+        v_fp8, v_scale = ops.quant_v(v)
+        o = ops.attn_fwd(q_int8, k_int8, v_fp8, lut, valid_block_num, pvthreshd, q_scale, k_scale, v_scale,
+                         1.0 / (headdim ** 0.5) if scale is None else scale, False, q.dtype, out=_empty_like_layout(q))
+    if tensor_layout == 'NHD':
+        o = o.transpose(-2, -3)
+    # core.py:229-231 always uses the causal denominator
+    return (o, _sparsity(valid_block_num, mask_id.size(3), True)) if return_sparsity else o
+
+
+@_skip_frame
 def block_sparse_sage2_attn_cuda(q, k, v, mask_id=None, dropout_p=0.0, scale=None, smooth_k=True, pvthreshd=50,
                                  attention_sink=False, tensor_layout="HND", output_dtype=torch.float16,
                                  return_sparsity=False):
     """spas_sage_attn/core.py:171-233 -- attention under a user-supplied 128x64 block mask."""
-    q, k, v = _prologue(q, k, v, tensor_layout)
-    km = ops.k_mean(k) if smooth_k else None
-    headdim = q.size(-1)
-    q_int8, q_scale, k_int8, k_scale = get_vanilla_qk_quant(q, k, km, 128, 64)
-    assert mask_id is not None, "mask_id is required"
-    lut, valid_block_num = block_map_lut_triton(block_map=mask_id)
-    if scale is None:
-        scale = 1.0 / (headdim ** 0.5)
-    assert headdim in [64, 128], "headdim should be in [64, 128]. For other headdim, you can use padding and specify the softmax scale."
-    pvthreshd = _pv_threshold_tensor(pvthreshd, q.size(-3), q.device)
-    v_fp8, v_scale = ops.quant_v(v)
-    o = ops.attn_fwd(q_int8, k_int8, v_fp8, lut, valid_block_num, pvthreshd, q_scale, k_scale, v_scale, scale, False,
-                     q.dtype, out=_empty_like_layout(q))
-    if tensor_layout == 'NHD':
-        o = o.transpose(-2, -3)
-    if return_sparsity:
-        return o, _sparsity(valid_block_num, lut, True)   # core.py:229-231 always uses the causal denominator
-    return o
+    if not return_sparsity and mask_id is not None:
+        o = _binding.forward(q, k, v, mask_id, None, None, None, pvthreshd, scale, False, False, False, smooth_k, False,
+                             tensor_layout, None, 0, False)
+        if o is not None:
+            return o
+    return _block_sparse_general(q, k, v, mask_id, scale, smooth_k, pvthreshd, tensor_layout, return_sparsity)
 
 
-@torch.compiler.disable
+@_skip_frame
 def spas_sage_attn_meansim_cuda(q, k, v, attn_mask=None, dropout_p=0.0, is_causal=False, scale=None, smooth_k=True,
                                 simthreshd1=0.6, cdfthreshd=0.98, pvthreshd=50, attention_sink=False,
                                 tensor_layout="HND", output_dtype=torch.float16, return_sparsity=False):
     """spas_sage_attn/core.py:235-276 -- Sage1 signature (cdf selection).  The reference runs its fp16-PV
     mma.sync kernel here on unquantised fp16 V and forwards is_causal to it; this build runs the fp16-PV
     variant of the tcgen05 kernel (SAGE1_FP16_PV = False: the FP8-PV kernel) with token-level causal masking."""
-    return _meansim_attention(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, None, pvthreshd,
-                              attention_sink, tensor_layout, return_sparsity, bool(is_causal), pv_fp16=SAGE1_FP16_PV)
+    if not return_sparsity and SINGLE_CALL_MAX_ROWS:
+        o = _binding.forward(q, k, v, None, simthreshd1, cdfthreshd, None, pvthreshd, scale, is_causal, is_causal,
+                             attention_sink, smooth_k, SAGE1_FP16_PV, tensor_layout, None, 0, False)
+        if o is not None:
+            return o
+    return _meansim_general(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, None, pvthreshd, attention_sink,
+                            tensor_layout, return_sparsity, bool(is_causal), pv_fp16=SAGE1_FP16_PV)
 
 
-@torch.compiler.disable
+@_skip_frame
 def spas_sage_attn_meansim_topk_cuda(q, k, v, attn_mask=None, dropout_p=0.0, is_causal=False, scale=None,
                                      smooth_k=True, simthreshd1=-0.1, cdfthreshd=None, topk=0.5, pvthreshd=50,
                                      attention_sink=False, tensor_layout="HND", output_dtype=torch.float16,
                                      return_sparsity=False):
     """spas_sage_attn/core.py:278-319 -- Sage1 signature (top-k selection), token-level causal, fp16 P.V."""
-    return _meansim_attention(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, topk, pvthreshd,
-                              attention_sink, tensor_layout, return_sparsity, bool(is_causal), pv_fp16=SAGE1_FP16_PV)
+    if not return_sparsity and SINGLE_CALL_MAX_ROWS:
+        o = _binding.forward(q, k, v, None, simthreshd1, cdfthreshd, topk, pvthreshd, scale, is_causal, is_causal,
+                             attention_sink, smooth_k, SAGE1_FP16_PV, tensor_layout, None, 0, False)
+        if o is not None:
+            return o
+    return _meansim_general(q, k, v, is_causal, scale, smooth_k, simthreshd1, cdfthreshd, topk, pvthreshd, attention_sink,
+                            tensor_layout, return_sparsity, bool(is_causal), pv_fp16=SAGE1_FP16_PV)
