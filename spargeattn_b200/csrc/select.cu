@@ -1,5 +1,5 @@
 // Mask predictor back end: pooled QK^T row -> softmax -> stable top-k (or cdf) selection ->
-// forced blocks / causal / sink -> block mask + delta-encoded LUT, one CTA per (b, h, q-block) row.
+// forced blocks / causal / sink -> block mask + delta-encoded LUT, one warp per one or two (b, h, q-block) rows.
 // Replaces spas_sage_attn/utils.py:386-420 (bmm, masked fills, softmax, sort, cumsum,
 // triton_fill_block_map_kernel :282-292, triton_fill_causal_mask :304-311) and
 // triton_block_map_to_lut_kernel (utils.py:54-74).
@@ -72,15 +72,23 @@ __device__ __forceinline__ float key_value<__nv_bfloat16>(uint32_t k) {
   return __bfloat162float(__ushort_as_bfloat16((unsigned short)k));
 }
 
-// ---- warp-per-row predictor --------------------------------------------------------------------
-// One warp owns one (b, h, q-block) row; a CTA holds up to 4 consecutive rows of one head, so the
-// pooled K rows it streams are shared through L1. Everything is warp-synchronous (shuffles and
-// ballots), there is no block-wide barrier.
-// dynamic smem: [32][D*2+16] byte staging tile of pooled K rows (shared by the CTA's rows), then per
-// row: int idx[nk] (first the fp32 scores) | float q[D] | uint16 key[nk].  The fp64 exponentials are
-// evaluated twice (once for the sum, once for the probabilities) instead of being stored: at long
-// sequences shared memory per row, not arithmetic, limits how many rows an SM can hold.
-constexpr int kSelRowsPerCta = 4;
+// ---- predictor -----------------------------------------------------------------------------------
+// A warp owns RW rows (b, h, q-block) of one head, a CTA WARPS * RW consecutive ones.
+//   1  scores: the CTA streams pooled K through shared memory in tiles of 64 rows; lane l of a warp runs the fp32 FMA
+//      chains of keys j0 + l and j0 + 32 + l for each of its rows as one packed f32x2 chain (each half rounds on its own).
+//      A score is a 16-bit value and is kept as one: two bytes per key and row are all that a row holds, and they become
+//      in turn the softmax key, the sort buffer's source and the list of live blocks. (With 32-bit scores, an index list
+//      and separate keys a row of 1 861 blocks took 12 KB, three warps fitted per scheduler, and the kernel waited:
+//      2.26 ms for 24 heads of 931 x 1861 blocks, 1.14 ms now.)
+//   2  per row, by its warp alone (shuffles and ballots): fp64 softmax, selection threshold by bisection over the 16 key
+//      bits with eight keys per lane and load, final map and LUT.
+// What bounds it: instruction issue of the score chains (1.3 per score and channel), then the fp64 pipe; a short row is a
+// chain of dependent reductions.
+constexpr int kSelTileKeys = 64;
+// Marks of a block that is not self-similar: in place of its score, and in place of its probability (zero, with the sign
+// bit telling that the block is live whatever the selection says).
+constexpr uint16_t kNotSimilarScore = 0xffff, kNotSimilarKey = 0x8000;
+
 __host__ __device__ inline int next_pow2(int n) {
   int p = 1;
   while (p < n) p <<= 1;
@@ -96,233 +104,410 @@ __host__ __device__ inline int aten_scan_log_threads_x(uint32_t num_rows, uint32
   v = v < 4u ? 4u : v;
   return (int)(v > 9u ? 9u : v);
 }
-// per-row shared memory: sort / index / score words [next_pow2(nk)] | q [D] floats | keys [nk] | cdf [cdf_len] 16-bit
-__host__ __device__ inline size_t select_row_bytes(int nk, int D, int cdf_len) {
-  return (((size_t)next_pow2(nk) * 4 + (size_t)D * 4 + (size_t)nk * 2 + (size_t)cdf_len * 2) + 15) / 16 * 16;
+
+// Shared memory of one row, in bytes: keys (16-bit, padded to whole 256-key groups of the bisection); the duplicated
+// query (freed after the scores) or, in cdf mode, the sort buffer in the same place; the scanned probabilities.
+struct SelectRow {
+  int keys, work, cdf;
+  __host__ __device__ int total() const { return keys + work + cdf; }
+};
+__host__ __device__ inline SelectRow select_row(int nk, int D, int cdf_len) {
+  SelectRow r;
+  r.keys = (nk + 255) / 256 * 512;
+  const int sort = cdf_len ? next_pow2(nk) * 2 : 0;
+  r.work = ((D * 8 > sort ? D * 8 : sort) + 15) / 16 * 16;
+  r.cdf = (cdf_len * 2 + 15) / 16 * 16;
+  return r;
 }
 
-__device__ __forceinline__ int warp_sum_int(int x) {
+// exp(x) for x <= 0: x = n ln 2 + r, Taylor polynomial of degree 11 in r (remainder below 7e-15), exponent added. Where
+// exp(x) is below 1e-304 it is zero: no sum or 16-bit probability can tell.
+__device__ __forceinline__ double exp_nonpositive(double x) {
+  if (x < -700.0) return 0.0;
+  constexpr double kLn2Hi = 0.6931471824645996, kLn2Lo = -1.90465429995776804525e-09;   // the nearest float (n * hi is exact) + the rest
+  const float nf = rintf((float)x * 1.44269504f);
+  double r = fma((double)nf, -kLn2Hi, x);
+  r = fma((double)nf, -kLn2Lo, r);
+  double p = 1.0 / 39916800.0;
+  p = fma(p, r, 1.0 / 3628800.0);
+  p = fma(p, r, 1.0 / 362880.0);
+  p = fma(p, r, 1.0 / 40320.0);
+  p = fma(p, r, 1.0 / 5040.0);
+  p = fma(p, r, 1.0 / 720.0);
+  p = fma(p, r, 1.0 / 120.0);
+  p = fma(p, r, 1.0 / 24.0);
+  p = fma(p, r, 1.0 / 6.0);
+  p = fma(p, r, 0.5);
+  p = fma(p, r, 1.0);
+  p = fma(p, r, 1.0);
+  return __hiloint2double(__double2hiint(p) + ((int)nf << 20), __double2loint(p));
+}
+
+// number of a lane's keys (8 in a 128-bit word) that are >= cand, both halves of cand2 holding cand: non-negative 16-bit
+// floats order like their bit patterns
+template <typename T>
+__device__ __forceinline__ int count_ge(uint4 w, uint32_t cand2);
+template <>
+__device__ __forceinline__ int count_ge<__half>(uint4 w, uint32_t cand2) {
+  const __half2 c = *reinterpret_cast<const __half2*>(&cand2);
+  const __half2 s = __hadd2(__hadd2(__hge2(*reinterpret_cast<const __half2*>(&w.x), c), __hge2(*reinterpret_cast<const __half2*>(&w.y), c)),
+                            __hadd2(__hge2(*reinterpret_cast<const __half2*>(&w.z), c), __hge2(*reinterpret_cast<const __half2*>(&w.w), c)));
+  return (int)__low2float(s) + (int)__high2float(s);
+}
+template <>
+__device__ __forceinline__ int count_ge<__nv_bfloat16>(uint4 w, uint32_t cand2) {
+  const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162*>(&cand2);
+  const __nv_bfloat162 s =
+      __hadd2(__hadd2(__hge2(*reinterpret_cast<const __nv_bfloat162*>(&w.x), c), __hge2(*reinterpret_cast<const __nv_bfloat162*>(&w.y), c)),
+              __hadd2(__hge2(*reinterpret_cast<const __nv_bfloat162*>(&w.z), c), __hge2(*reinterpret_cast<const __nv_bfloat162*>(&w.w), c)));
+  return (int)__low2float(s) + (int)__high2float(s);
+}
+
+template <typename T>
+__device__ __forceinline__ uint16_t add16(uint16_t a, uint16_t b) {
+  return (uint16_t)key_bits<T>(Elem<T>::from_float(__fadd_rn(key_value<T>(a), key_value<T>(b))));
+}
+
+// Descending bitonic sort of P2 16-bit keys (two per word, unsigned order) by one warp in shared memory. The position of
+// equal keys does not matter: only the sequence of values is used.
+__device__ __forceinline__ void sort_descending(uint32_t* buf, int P2, int lane) {
+  const int words = P2 / 2;
+  for (int kk = 2; kk <= P2; kk <<= 1) {
+    for (int jj = kk >> 1; jj > 1; jj >>= 1) {   // partners in different words
+      const int jw = jj / 2;
+      for (int t = lane; t < words / 2; t += 32) {
+        const int i = ((t & ~(jw - 1)) << 1) | (t & (jw - 1)), ip = i | jw;
+        const uint32_t a = buf[i], b = buf[ip];
+        const uint32_t mx = __vmaxu2(a, b), mn = __vminu2(a, b);
+        const bool down = ((2 * i) & kk) == 0;
+        buf[i] = down ? mx : mn;
+        buf[ip] = down ? mn : mx;
+      }
+      __syncwarp();
+    }
+    for (int i = lane; i < words; i += 32) {     // partners in one word
+      const uint32_t a = buf[i], lo = min(a & 0xffffu, a >> 16), hi = max(a & 0xffffu, a >> 16);
+      buf[i] = ((2 * i) & kk) == 0 ? (hi | (lo << 16)) : (lo | (hi << 16));
+    }
+    __syncwarp();
+  }
+}
+
+// ATen's cumsum of nk sorted 16-bit values (see the contract above): chunks of W = 32 V values, the running total enters
+// the first value of a chunk, Sklansky combine steps, each sum rounded to the 16-bit type. In registers: value i of a
+// chunk is v[i / 32] of lane i % 32.
+template <typename T, int V>
+__device__ __forceinline__ void scan_chunks(const uint16_t* sorted, uint16_t* cdf, int nk, int lane) {
+  uint16_t total = 0;
+  for (int c0 = 0; c0 < nk; c0 += 32 * V) {
+    uint16_t v[V];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
+    for (int i = 0; i < V; i++) v[i] = (c0 + 32 * i + lane < nk) ? sorted[c0 + 32 * i + lane] : (uint16_t)0;
+    if (lane == 0) v[0] = add16<T>(v[0], total);
+#pragma unroll
+    for (int mm = 0; mm < 5; mm++) {
+#pragma unroll
+      for (int i = 0; i < V; i++) {
+        const uint16_t o = (uint16_t)__shfl_sync(0xffffffffu, (int)v[i], (lane & ~((2 << mm) - 1)) + (1 << mm) - 1);
+        if (lane & (1 << mm)) v[i] = add16<T>(v[i], o);
+      }
+    }
+#pragma unroll
+    for (int g = 1; g < V; g <<= 1) {
+#pragma unroll
+      for (int i = 0; i < V; i++)
+        if (i & g) v[i] = add16<T>(v[i], (uint16_t)__shfl_sync(0xffffffffu, (int)v[(i & ~(2 * g - 1)) + g - 1], 31));
+    }
+#pragma unroll
+    for (int i = 0; i < V; i++) cdf[c0 + 32 * i + lane] = v[i];
+    total = (uint16_t)__shfl_sync(0xffffffffu, (int)v[V - 1], 31);
+  }
+  __syncwarp();
+}
+// the same for wider chunks, in shared memory
+template <typename T>
+__device__ __forceinline__ void scan_chunks_wide(const uint16_t* sorted, uint16_t* cdf, int nk, int log_nx, int lane) {
+  const int nx = 1 << log_nx, W = 2 * nx;
+  uint16_t total = 0;
+  for (int c0 = 0; c0 < nk; c0 += W) {
+    uint16_t* buf = cdf + c0;
+    for (int i = lane; i < W; i += 32) buf[i] = (c0 + i < nk) ? sorted[c0 + i] : (uint16_t)0;
+    __syncwarp();
+    if (lane == 0) buf[0] = add16<T>(buf[0], total);
+    __syncwarp();
+    for (int mm = 0; mm <= log_nx; mm++) {
+      const int sgm = 1 << mm;
+      for (int t = lane; t < nx; t += 32) {
+        const int a = ((t >> mm) << (mm + 1)) | sgm;
+        const int ti = a + (t & (sgm - 1)), si = a - 1;
+        buf[ti] = add16<T>(buf[ti], buf[si]);
+      }
+      __syncwarp();
+    }
+    total = buf[W - 1];
+    __syncwarp();
+  }
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kSelRowsPerCta * 32)
+template <typename T, int D, int RW, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t* __restrict__ sim_q,
               const uint8_t* __restrict__ sim_k, const float* __restrict__ topk, const float* __restrict__ cdfthr,
               uint8_t* __restrict__ mask, int32_t* __restrict__ lut, int32_t* __restrict__ valid, int H, int nq, int nk,
-              int is_causal, int sink, int rows_per_cta, int best_first, int scan_log_nx, int cdf_len) {
+              int is_causal, int sink, int best_first, int scan_log_nx, int cdf_len) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  pdl_wait();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int qi = blockIdx.x * rows_per_cta + warp, bh = blockIdx.y, h = bh % H;
-  const bool active = warp < rows_per_cta && qi < nq;       // inactive warps still help to stage K tiles
   constexpr int kTileRowBytes = D * (int)sizeof(T) + 16;   // 16-byte pad: conflict-free 128-bit reads, one row per lane
-  unsigned char* s_tile = smem_raw;
-  const size_t row_bytes = select_row_bytes(nk, D, cdf_len);
-  const int P2 = next_pow2(nk);
-  unsigned char* base = smem_raw + 32 * kTileRowBytes + (size_t)(active ? warp : 0) * row_bytes;
-  int* s_idx = reinterpret_cast<int*>(base);
-  float* s_s = reinterpret_cast<float*>(s_idx);            // scores share storage with the index list
-  uint32_t* s_sort = reinterpret_cast<uint32_t*>(s_idx);   // ... and with the sort keys of the cdf mode
-  float* s_q = reinterpret_cast<float*>(s_idx + P2);
-  uint16_t* s_key = reinterpret_cast<uint16_t*>(s_q + D);
-  uint16_t* s_cdf = s_key + nk;
-  const int k_limit = is_causal ? min(nk, (qi + 1) * (kBlockQ / kBlockK)) : nk;   // causal: k < (q+1)*2
+  constexpr int kChunksPerRow = D * (int)sizeof(T) / 16;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q0 = (blockIdx.x * WARPS + warp) * RW, bh = blockIdx.y, h = bh % H;   // this warp's first row
+  const SelectRow layout = select_row(nk, D, cdf_len);
+  unsigned char* base = smem_raw + kSelTileKeys * kTileRowBytes + (size_t)warp * RW * layout.total();
+  auto keys_of = [&](int r) { return reinterpret_cast<uint16_t*>(base + r * layout.total()); };
+  auto work_of = [&](int r) { return base + r * layout.total() + layout.keys; };
+  // causal: a row sees the key blocks k < 2 (q + 1)
+  auto limit_of = [&](int q) { return is_causal ? min(nk, (q + 1) * (kBlockQ / kBlockK)) : nk; };
+  pdl_wait();
+  // asked for here, needed long after: a row is a chain of short steps, and a load in it would stall all of them
+  const float n_or_thr = cdfthr ? cdfthr[h] : topk[h];
+  uint8_t q_similar[RW];
+#pragma unroll
+  for (int r = 0; r < RW; r++) q_similar[r] = sim_q[(size_t)bh * nq + min(q0 + r, nq - 1)];
 
-  if (active)
-    for (int dd = lane; dd < D; dd += 32) s_q[dd] = Elem<T>::to_float(pq[((size_t)bh * nq + qi) * D + dd]);
-  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < RW; r++) {   // the query, each value twice: a packed FMA takes it as it is
+    float2* s_q = reinterpret_cast<float2*>(work_of(r));
+    for (int d = lane; d < D; d += 32) {
+      const float v = q0 + r < nq ? Elem<T>::to_float(pq[((size_t)bh * nq + q0 + r) * D + d]) : 0.f;
+      s_q[d] = make_float2(v, v);
+    }
+  }
 
-  // ---- scores: the CTA streams pooled K through shared memory in tiles of 32 rows (coalesced
-  // 128-bit loads); lane l of every active warp then runs the fp32 FMA chain for key block j0 + l.
+  // ---- 1: scores
   const float scale = (D == 64) ? 0.125f : 0.08838834764831845f;   // float(D ** -0.5)
   const T* pkb = pk + (size_t)bh * nk * D;
   const uint8_t* simk = sim_k + (size_t)bh * nk;
-  constexpr int kChunksPerRow = D * (int)sizeof(T) / 16;
-  float m = -INFINITY;
-  for (int j0 = 0; j0 < nk; j0 += 32) {
-    __syncthreads();                                       // previous tile fully consumed
-    for (int i = threadIdx.x; i < 32 * kChunksPerRow; i += blockDim.x) {
-      const int r = i / kChunksPerRow, c = i % kChunksPerRow;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (j0 + r < nk) val = *reinterpret_cast<const uint4*>(pkb + (size_t)(j0 + r) * D + c * 8);
-      *reinterpret_cast<uint4*>(s_tile + r * kTileRowBytes + c * 16) = val;
-    }
-    __syncthreads();
-    const int j = j0 + lane;
-    if (active && j < nk) {
-      float sc = -INFINITY;
-      if (j < k_limit && simk[j]) {
-        float acc = 0.f;
-        const unsigned char* row = s_tile + lane * kTileRowBytes;
-#pragma unroll 4
-        for (int c = 0; c < kChunksPerRow; c++) {
-          const Pack8<T> p = *reinterpret_cast<const Pack8<T>*>(row + c * 16);
+  const int cta_limit = limit_of(min(nq, ((int)blockIdx.x + 1) * WARPS * RW) - 1);   // keys any row of the CTA sees
+  const T minus_inf = Elem<T>::from_float(-INFINITY);
+  float m[RW];
 #pragma unroll
-          for (int i = 0; i < 8; i++) acc = __fmaf_rn(s_q[c * 8 + i], Elem<T>::to_float(p.v[i]), acc);
-        }
-        sc = Elem<T>::to_float(Elem<T>::from_float(acc));
-        sc = Elem<T>::to_float(Elem<T>::from_float(__fmul_rn(sc, scale)));
+  for (int r = 0; r < RW; r++) m[r] = -INFINITY;
+  for (int j0 = 0; j0 < nk; j0 += kSelTileKeys) {
+    const bool seen = j0 < cta_limit;
+    uint8_t similar[2];
+#pragma unroll
+    for (int hf = 0; hf < 2; hf++) similar[hf] = j0 + 32 * hf + lane < nk ? simk[j0 + 32 * hf + lane] : 0;
+    if (seen) {
+      __syncthreads();                                       // previous tile fully consumed
+      for (int i = threadIdx.x; i < kSelTileKeys * kChunksPerRow; i += WARPS * 32) {
+        const int row = i / kChunksPerRow, c = i % kChunksPerRow;
+        uint4 val = make_uint4(0, 0, 0, 0);
+        if (j0 + row < nk) val = *reinterpret_cast<const uint4*>(pkb + (size_t)(j0 + row) * D + c * 8);
+        *reinterpret_cast<uint4*>(smem_raw + row * kTileRowBytes + c * 16) = val;
       }
-      s_s[j] = sc;
-      m = fmaxf(m, sc);
+      __syncthreads();
     }
-  }
-  if (!active) return;                                     // no block-wide barrier below this line
-  m = warp_max(m);
-
-  // ---- fp64 softmax -> 16-bit keys (p >= 0, so the bit pattern orders like the value)
-  double Z = 0.0;
-  for (int j = lane; j < nk; j += 32) {
-    const float sc = s_s[j];
-    Z += (sc == -INFINITY) ? 0.0 : exp((double)sc - (double)m);
-  }
-  Z = warp_sum(Z);
-  const bool empty_row = (m == -INFINITY);
-  for (int j = lane; j < nk; j += 32) {
-    const float sc = s_s[j];
-    const double e = (sc == -INFINITY) ? 0.0 : exp((double)sc - (double)m);
-    s_key[j] = empty_row ? (uint16_t)0 : (uint16_t)key_bits<T>(Elem<T>::from_float((float)(e / Z)));
-  }
-  __syncwarp();
-
-  // ---- how many blocks to select
-  int n_sel;
-  if (cdfthr == nullptr) {
-    n_sel = (int)__fmul_rn(topk[h], (float)nk);            // top-k mode: same count for every row of a head
-  } else {
-    // cdf mode. Step 1: the stable descending order (ties -> lower block index) as an explicit sequence: a
-    // bitonic sort of (probability bits << 16 | 0xFFFF - index) in shared memory by this warp.
-    const float thr = cdfthr[h];
-    for (int i = lane; i < P2; i += 32) s_sort[i] = (i < nk) ? (((uint32_t)s_key[i] << 16) | (uint32_t)(0xFFFF - i)) : 0u;
-    __syncwarp();
-    for (int kk = 2; kk <= P2; kk <<= 1) {
-      for (int jj = kk >> 1; jj > 0; jj >>= 1) {
-        for (int i = lane; i < P2; i += 32) {
-          const int ixj = i ^ jj;
-          if (ixj > i) {
-            const uint32_t a = s_sort[i], b = s_sort[ixj];
-            const bool first_larger = (i & kk) == 0;
-            if (first_larger ? (a < b) : (a > b)) {
-              s_sort[i] = b;
-              s_sort[ixj] = a;
-            }
+    float2 acc[RW];
+#pragma unroll
+    for (int r = 0; r < RW; r++) acc[r] = make_float2(0.f, 0.f);
+    if (seen) {
+      const unsigned char* ka = smem_raw + lane * kTileRowBytes;
+      const unsigned char* kb = ka + 32 * kTileRowBytes;
+#pragma unroll 2
+      for (int c = 0; c < kChunksPerRow; c++) {
+        const Pack8<T> a = *reinterpret_cast<const Pack8<T>*>(ka + c * 16), b = *reinterpret_cast<const Pack8<T>*>(kb + c * 16);
+        float2 k2[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) k2[i] = make_float2(Elem<T>::to_float(a.v[i]), Elem<T>::to_float(b.v[i]));
+#pragma unroll
+        for (int r = 0; r < RW; r++) {
+          const float4* qv = reinterpret_cast<const float4*>(work_of(r)) + c * 4;
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const float4 q2 = qv[i];
+            acc[r] = __ffma2_rn(make_float2(q2.x, q2.y), k2[2 * i], acc[r]);
+            acc[r] = __ffma2_rn(make_float2(q2.z, q2.w), k2[2 * i + 1], acc[r]);
           }
         }
-        __syncwarp();
       }
-    }
-    // Step 2: ATen's cumsum of the sorted 16-bit values: chunks of W = 2 * nx values; the running total enters
-    // the first value of a chunk; Sklansky combine steps, each sum rounded to the 16-bit type.
-    const int nx = 1 << scan_log_nx, W = 2 * nx;
-    auto add16 = [](uint16_t a, uint16_t b) -> uint16_t {
-      return (uint16_t)key_bits<T>(Elem<T>::from_float(__fadd_rn(key_value<T>(a), key_value<T>(b))));
-    };
-    uint16_t total = 0;
-    for (int c0 = 0; c0 < nk; c0 += W) {
-      uint16_t* buf = s_cdf + c0;
-      for (int i = lane; i < W; i += 32) buf[i] = (c0 + i < nk) ? (uint16_t)(s_sort[c0 + i] >> 16) : (uint16_t)0;
-      __syncwarp();
-      if (lane == 0) buf[0] = add16(buf[0], total);
-      __syncwarp();
-      for (int mm = 0; mm <= scan_log_nx; mm++) {
-        const int sgm = 1 << mm;
-        for (int t = lane; t < nx; t += 32) {
-          const int a = ((t >> mm) << (mm + 1)) | sgm;
-          const int ti = a + (t & (sgm - 1)), si = a - 1;
-          buf[ti] = add16(buf[ti], buf[si]);
-        }
-        __syncwarp();
-      }
-      total = buf[W - 1];
-      __syncwarp();
-    }
-    // Step 3: torch.searchsorted(..., right=True): upper-bound binary search, 16-bit cdf compared in fp32
-    int lo_i = 0, hi_i = nk;
-    while (lo_i < hi_i) {
-      const int mid = lo_i + ((hi_i - lo_i) >> 1);
-      if (!(key_value<T>(s_cdf[mid]) > thr)) lo_i = mid + 1; else hi_i = mid;
-    }
-    n_sel = lo_i;
-    __syncwarp();
-  }
-  n_sel = max(1, min(n_sel, nk));
-
-  // ---- n_sel-th largest key by bisection over the 16 key bits
-  uint32_t thr_key = 0;
-#pragma unroll 1
-  for (int bit = 15; bit >= 0; bit--) {
-    const uint32_t cand = thr_key | (1u << bit);
-    int c = 0;
-    for (int j = lane; j < nk; j += 32) c += (s_key[j] >= cand);
-    c = warp_sum_int(c);
-    if (c >= n_sel) thr_key = cand;
-  }
-  int above = 0;
-  for (int j = lane; j < nk; j += 32) above += (s_key[j] > thr_key);
-  above = warp_sum_int(above);
-  const int remaining = n_sel - above;
-
-  // ---- final map in index order (ties -> lower index) and compaction into idx[]
-  const bool row_forced = sim_q[(size_t)bh * nq + qi] == 0;
-  uint8_t* mrow = mask ? mask + ((size_t)bh * nq + qi) * nk : nullptr;
-  int eq_seen = 0, live_seen = 0;
-  __syncwarp();                                            // scores are dead from here on: idx[] may overwrite them
-  for (int j0 = 0; j0 < nk; j0 += 32) {
-    const int j = j0 + lane;
-    const bool in = j < nk;
-    const uint32_t key = in ? s_key[j] : 0u;
-    const bool is_eq = in && key == thr_key;
-    const unsigned eq_b = __ballot_sync(0xffffffffu, is_eq);
-    const int eq_rank = eq_seen + __popc(eq_b & ((1u << lane) - 1u));
-    eq_seen += __popc(eq_b);
-    bool live = false;
-    if (in) {
-      live = (key > thr_key) || (is_eq && eq_rank < remaining) || row_forced || (simk[j] == 0);
-      if (is_causal) live = live && (j < k_limit);
-      if (sink && j == 0) live = true;
-      if (mrow) mrow[j] = live ? 1 : 0;
-    }
-    const unsigned lv_b = __ballot_sync(0xffffffffu, live);
-    if (live) s_idx[live_seen + __popc(lv_b & ((1u << lane) - 1u))] = j;
-    live_seen += __popc(lv_b);
-  }
-  __syncwarp();
-  int32_t* lrow = lut + ((size_t)bh * nq + qi) * nk;
-  // Visiting order. Reference order: ascending block index. Best-first: the live block with the largest
-  // pooled probability (lowest index on ties) is moved to the front and the rest stay ascending; the
-  // deltas may then be negative. Attention is order-independent, but starting at the block that most
-  // likely holds the row maxima makes later rescales of the running output rare.
-  int rbest = 0;
-  if (best_first && live_seen > 1) {
-    uint32_t bk = 0;
-    int bpos = 0x7fffffff;
-    for (int r = lane; r < live_seen; r += 32) {
-      const uint32_t key = s_key[s_idx[r]];
-      if (key > bk || (key == bk && r < bpos)) { bk = key; bpos = r; }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const uint32_t ok_ = __shfl_xor_sync(0xffffffffu, bk, o);
-      const int op = __shfl_xor_sync(0xffffffffu, bpos, o);
-      if (ok_ > bk || (ok_ == bk && op < bpos)) { bk = ok_; bpos = op; }
+    for (int hf = 0; hf < 2; hf++) {
+      const int j = j0 + 32 * hf + lane;
+      const bool in = j < nk;
+#pragma unroll
+      for (int r = 0; r < RW; r++) {
+        T sc = minus_inf;
+        if (similar[hf] && j < limit_of(q0 + r)) {
+          sc = Elem<T>::from_float(hf ? acc[r].y : acc[r].x);
+          sc = Elem<T>::from_float(__fmul_rn(Elem<T>::to_float(sc), scale));
+          m[r] = fmaxf(m[r], Elem<T>::to_float(sc));
+        }
+        if (in) keys_of(r)[j] = similar[hf] ? (uint16_t)key_bits<T>(sc) : kNotSimilarScore;
+      }
     }
-    rbest = (bpos == 0x7fffffff) ? 0 : bpos;
   }
-  const int jbest = (live_seen > 0) ? s_idx[rbest] : 0;
-  for (int r = lane; r < nk; r += 32) {
-    int vv = 0;
-    if (r < live_seen) {
-      // element at visiting position r: jbest first, then the ascending list without it
-      const int cur = (r == 0) ? jbest : s_idx[r <= rbest ? r - 1 : r];
-      const int prev = (r == 0) ? 0 : ((r == 1) ? jbest : s_idx[(r - 1) <= rbest ? r - 2 : r - 1]);
-      vv = cur - prev;
+  __syncwarp();
+
+  // ---- 2: row by row (no block-wide barrier below this line)
+#pragma unroll 1
+  for (int r = 0; r < RW; r++) {
+    const int qi = q0 + r;
+    if (qi >= nq) break;
+    uint16_t* s_key = keys_of(r);
+    const int k_limit = limit_of(qi);
+    const float mx = warp_max(m[0]);
+    const bool row_forced = q_similar[0] == 0;
+#pragma unroll
+    for (int i = 0; i + 1 < RW; i++) {                       // the next row's values, without indexing registers
+      m[i] = m[i + 1];
+      q_similar[i] = q_similar[i + 1];
     }
-    lrow[r] = vv;
+
+    // fp64 softmax -> 16-bit keys (p >= 0, so the bit pattern orders like the value). The exponentials are evaluated
+    // twice, once for the sum and once for the probabilities, instead of being stored.
+    double Z = 0.0;
+    for (int j = lane; j < nk; j += 32) {
+      const uint16_t raw = s_key[j];
+      const float sc = key_value<T>(raw);
+      if (raw != kNotSimilarScore && sc != -INFINITY) Z += exp_nonpositive((double)sc - (double)mx);
+    }
+    Z = warp_sum(Z);
+    const double rz = 1.0 / Z;
+    const int padded = (nk + 255) / 256 * 256;
+    for (int j = lane; j < padded; j += 32) {
+      uint16_t key = 0;
+      if (j < nk) {
+        const uint16_t raw = s_key[j];
+        const float sc = key_value<T>(raw);
+        if (raw == kNotSimilarScore) key = kNotSimilarKey;
+        else if (sc != -INFINITY) key = (uint16_t)key_bits<T>(Elem<T>::from_float((float)(exp_nonpositive((double)sc - (double)mx) * rz)));
+      }
+      s_key[j] = key;
+    }
+    __syncwarp();
+
+    // how many blocks to select
+    int n_sel;
+    if (cdfthr == nullptr) {
+      n_sel = (int)__fmul_rn(n_or_thr, (float)nk);           // top-k mode: same count for every row of a head
+    } else {
+      // cdf mode: the probabilities in descending order, ATen's cumsum of them, then torch.searchsorted(..., right=True):
+      // upper-bound binary search, 16-bit cdf compared in fp32
+      const float thr = n_or_thr;
+      const int P2 = next_pow2(nk);
+      uint16_t* sorted = reinterpret_cast<uint16_t*>(work_of(r));
+      uint16_t* s_cdf = reinterpret_cast<uint16_t*>(work_of(r) + layout.work);
+      for (int i = lane; i < P2; i += 32) sorted[i] = i < nk ? (uint16_t)(s_key[i] & 0x7fff) : (uint16_t)0;
+      __syncwarp();
+      sort_descending(reinterpret_cast<uint32_t*>(sorted), P2, lane);
+      if (scan_log_nx == 4) scan_chunks<T, 1>(sorted, s_cdf, nk, lane);
+      else if (scan_log_nx == 5) scan_chunks<T, 2>(sorted, s_cdf, nk, lane);
+      else scan_chunks_wide<T>(sorted, s_cdf, nk, scan_log_nx, lane);
+      int lo_i = 0, hi_i = nk;
+      while (lo_i < hi_i) {
+        const int mid = lo_i + ((hi_i - lo_i) >> 1);
+        if (!(key_value<T>(s_cdf[mid]) > thr)) lo_i = mid + 1; else hi_i = mid;
+      }
+      n_sel = lo_i;
+    }
+    n_sel = max(1, min(n_sel, nk));
+
+    // n_sel-th largest key, two of its 15 value bits per round (three candidates counted at once: the rounds are a chain of
+    // reductions); padding and not-similar keys count as zero
+    const uint4* groups = reinterpret_cast<const uint4*>(s_key);
+    const uint4 own = groups[lane];                          // all there is of a row of up to 256 blocks
+    auto count = [&](uint32_t cand) {
+      const uint32_t cand2 = cand | (cand << 16);
+      int c = count_ge<T>(own, cand2);
+      for (int i = lane + 32; i < padded / 8; i += 32) c += count_ge<T>(groups[i], cand2);
+      return (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
+    };
+    uint32_t thr_key = count(1u << 14) >= n_sel ? 1u << 14 : 0u;
+#pragma unroll 1
+    for (int bit = 12; bit >= 0; bit -= 2) {
+      const int c1 = count(thr_key | (1u << bit)), c2 = count(thr_key | (2u << bit)), c3 = count(thr_key | (3u << bit));
+      thr_key |= (uint32_t)((c1 >= n_sel) + (c2 >= n_sel) + (c3 >= n_sel)) << bit;
+    }
+    const int remaining = n_sel - count(thr_key + 1);
+
+    // final map in index order (ties -> lower index), compacted in place into the list of live blocks: a lane takes eight
+    // consecutive keys of a 256-key group, and a position of the list never lies past the keys already read. The best
+    // block of the list (largest probability, lowest index) is found on the way.
+    uint8_t* mrow = mask ? mask + ((size_t)bh * nq + qi) * nk : nullptr;
+    int eq_seen = 0, live_seen = 0;
+    uint32_t best = 0;                                       // (probability + 1) << 16 | 0xffff - position in the list
+    for (int g0 = 0; g0 < nk; g0 += 256) {
+      const int jb = g0 + lane * 8;
+      const uint4 w = *reinterpret_cast<const uint4*>(s_key + jb);
+      const uint32_t word[4] = {w.x, w.y, w.z, w.w};
+      uint32_t eq = 0, live = 0;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const uint32_t key = (word[i >> 1] >> (16 * (i & 1))) & 0xffffu;
+        eq |= (jb + i < nk && (key & 0x7fff) == thr_key) ? 1u << i : 0u;
+      }
+      int eq_incl = __popc(eq);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, eq_incl, o);
+        if (lane >= o) eq_incl += t;
+      }
+      int eq_rank = eq_seen + eq_incl - __popc(eq);
+      eq_seen += __shfl_sync(0xffffffffu, eq_incl, 31);
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int j = jb + i;
+        const uint32_t key = (word[i >> 1] >> (16 * (i & 1))) & 0xffffu;
+        bool on = false;
+        if (j < nk) {
+          const bool is_eq = (eq >> i) & 1;
+          on = key > thr_key || (is_eq && eq_rank < remaining) || row_forced;   // (a not-similar key has the top bit)
+          eq_rank += is_eq ? 1 : 0;
+          if (is_causal) on = on && j < k_limit;
+          if (sink && j == 0) on = true;
+          if (mrow) mrow[j] = on ? 1 : 0;
+        }
+        live |= on ? 1u << i : 0u;
+      }
+      int incl = __popc(live);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      int pos = live_seen + incl - __popc(live);
+      live_seen += __shfl_sync(0xffffffffu, incl, 31);
+      __syncwarp();                                          // the whole group has been read
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        if ((live >> i) & 1) {
+          const uint32_t key = (word[i >> 1] >> (16 * (i & 1))) & 0xffffu;
+          best = max(best, (((key & 0x7fff) + 1) << 16) | (uint32_t)(0xffff - pos));
+          s_key[pos++] = (uint16_t)(jb + i);
+        }
+      }
+    }
+    __syncwarp();
+    // Visiting order. Reference order: ascending block index. Best-first: the live block with the largest
+    // pooled probability (lowest index on ties) is moved to the front and the rest stay ascending; the
+    // deltas may then be negative. Attention is order-independent, but starting at the block that most
+    // likely holds the row maxima makes later rescales of the running output rare.
+    const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+    const int rbest = (best_first && live_seen > 0) ? 0xffff - (int)(top & 0xffffu) : 0;
+    const int jbest = live_seen > 0 ? s_key[rbest] : 0;
+    int32_t* lrow = lut + ((size_t)bh * nq + qi) * nk;
+    for (int i = lane; i < nk; i += 32) {
+      int v = 0;
+      if (i < live_seen) {
+        // element at visiting position i: jbest first, then the ascending list without it
+        const int cur = i == 0 ? jbest : s_key[i <= rbest ? i - 1 : i];
+        const int prev = i == 0 ? 0 : i == 1 ? jbest : s_key[i - 1 <= rbest ? i - 2 : i - 1];
+        v = cur - prev;
+      }
+      lrow[i] = v;
+    }
+    if (lane == 0) valid[(size_t)bh * nq + qi] = live_seen;
   }
-  if (lane == 0) valid[(size_t)bh * nq + qi] = live_seen;
   pdl_trigger();
 }
 
@@ -362,33 +547,42 @@ __global__ void __launch_bounds__(kSelThreads) mask_to_lut_kernel(const uint8_t*
   pdl_trigger();
 }
 
-template <typename T, int D>
+template <typename T, int D, int RW, int WARPS>
 static int launch_select(const SelectArgs& a, cudaStream_t st) {
   // cdf mode reproduces torch.cumsum over the [B*H*nq, nk] matrix of sorted probabilities: the scan's chunking
   // depends on both extents
   const int scan_log_nx = aten_scan_log_threads_x((uint32_t)a.BH * (uint32_t)a.nq, (uint32_t)a.nk);
   const int scan_w = 2 << scan_log_nx;
   const int cdf_len = a.cdf ? (a.nk + scan_w - 1) / scan_w * scan_w : 0;
-  const size_t row_bytes = select_row_bytes(a.nk, D, cdf_len);
-  const size_t tile_bytes = 32 * (D * sizeof(T) + 16);
-  const size_t budget = 200 * 1024 - tile_bytes;
-  if (row_bytes > budget) return SPARGE_ERR_TOO_LARGE;
-  const int rows = (int)min((size_t)kSelRowsPerCta, budget / row_bytes);
-  const size_t smem = tile_bytes + rows * row_bytes;
-  auto kern = select_kernel<T, D>;
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return SPARGE_ERR_CUDA;
-  }
-  const cudaError_t e = launch(kern, dim3((a.nq + rows - 1) / rows, a.BH), kSelRowsPerCta * 32, smem, st, a.dependent,
+  const size_t smem = kSelTileKeys * (D * sizeof(T) + 16) + (size_t)WARPS * RW * select_row(a.nk, D, cdf_len).total();
+  if (smem > 200 * 1024) return SPARGE_ERR_TOO_LARGE;
+  auto kern = select_kernel<T, D, RW, WARPS>;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return SPARGE_ERR_CUDA;
+  const cudaError_t e = launch(kern, dim3((a.nq + WARPS * RW - 1) / (WARPS * RW), a.BH), WARPS * 32, smem, st, a.dependent,
                                (const T*)a.pq, (const T*)a.pk, a.sim_q, a.sim_k, a.topk, a.cdf, a.mask, a.lut, a.valid, a.H, a.nq,
-                               a.nk, a.causal, a.sink, rows, a.best_first, scan_log_nx, cdf_len);
+                               a.nk, a.causal, a.sink, a.best_first, scan_log_nx, cdf_len);
   return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
 }
 
+// Two rows per warp share every K value and its conversion, but then a row's steps run behind the other's: worth it where
+// the scores are most of the work and rows are plenty. One against two rows per warp, top-k mode, us: 59 / 71 at 21 rows
+// per SM (12 heads of 256 x 512 blocks), 124 / 114 at 55 (32 heads), 69 / 63 at 56 (60 heads of 139 x 278, D = 64); cdf
+// mode, whose sort and scan are per row: 84 / 108, 178 / 208, 117 / 120.
+constexpr long long kSelPairRows = 148 * 32;
+template <typename T, int D>
+static int dispatch_select(const SelectArgs& a, cudaStream_t st) {
+  if (a.nk > 65535) return SPARGE_ERR_TOO_LARGE;             // block indices are kept in 16 bits
+  int rc = SPARGE_ERR_TOO_LARGE;
+  if (!a.cdf && (long long)a.BH * a.nq >= kSelPairRows) rc = launch_select<T, D, 2, 8>(a, st);
+  if (rc == SPARGE_ERR_TOO_LARGE) rc = launch_select<T, D, 1, 4>(a, st);
+  if (rc == SPARGE_ERR_TOO_LARGE) rc = launch_select<T, D, 1, 1>(a, st);   // very long rows: one fits an SM
+  return rc;
+}
+
 int select_launch(const SelectArgs& a, cudaStream_t st) {
-  if (a.dtype == SPARGE_F16) return a.D == 64 ? launch_select<__half, 64>(a, st) : launch_select<__half, 128>(a, st);
-  return a.D == 64 ? launch_select<__nv_bfloat16, 64>(a, st) : launch_select<__nv_bfloat16, 128>(a, st);
+  if (a.dtype == SPARGE_F16) return a.D == 64 ? dispatch_select<__half, 64>(a, st) : dispatch_select<__half, 128>(a, st);
+  return a.D == 64 ? dispatch_select<__nv_bfloat16, 64>(a, st) : dispatch_select<__nv_bfloat16, 128>(a, st);
 }
 
 int mask_to_lut_launch(const void* mask, int elem_size, int32_t* lut, int32_t* valid, long long rows, int nk, bool dependent,

@@ -1,0 +1,88 @@
+"""Sizes at which the selection and the fused preparation change shape: edges of their tiles and groups, the smallest and
+largest member of each dispatch, against the oracle or the path that the other tests compare with it."""
+import pytest
+import torch
+
+import sparge_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _pooled(BH, nq, nk, D, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    pq, pk = torch.randn(1, BH, nq, D, generator=g) * 0.7, torch.randn(1, BH, nk, D, generator=g)
+    sim_q, sim_k = (torch.rand(1, BH, nq, generator=g) > 0.2), (torch.rand(1, BH, nk, generator=g) > 0.1)
+    return pq.to(dtype), pk.to(dtype), sim_q, sim_k
+
+
+# key blocks around the 64-row score tile, the 256-key group and the 16-byte load; 1 024 and 2 049 with few rows take the
+# widest cumsum chunks, 63 with many rows the narrowest
+@pytest.mark.parametrize("BH,nq,nk", [(1, 1, 1), (2, 3, 7), (1, 5, 63), (2, 4, 64), (3, 3, 65), (1, 6, 255), (2, 2, 256), (1, 3, 257),
+                                      (24, 32, 63), (1, 2, 1024), (1, 1, 2049)])
+@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 128), (torch.float16, 64)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_selection_at_tile_edges(BH, nq, nk, dtype, D, causal):
+    from spargeattn_b200 import ops
+    pq, pk, sim_q, sim_k = _pooled(BH, nq, nk, D, dtype, 100 * nk + nq)
+    p = O.pooled_probs(pq, pk, sim_k, causal)
+    dev = [t.cuda() for t in (pq, pk, sim_q.to(torch.uint8), sim_k.to(torch.uint8))]
+    for topk, cdf in ((0.37, None), (None, 0.9)):
+        knob = torch.full((BH,), topk or cdf)
+        want = O.select_blocks(p, sim_q, sim_k, knob if topk else None, knob if cdf else None, causal, nk > 64)
+        lut, valid, mask = ops.select_blocks(*dev, knob.cuda() if topk else None, knob.cuda() if cdf else None, causal, nk > 64, True)
+        assert torch.equal(mask.cpu().bool(), want)
+        lut_o, valid_o = O.block_map_to_lut(want)
+        assert torch.equal(lut.cpu(), lut_o) and torch.equal(valid.cpu(), valid_o)
+
+
+@pytest.mark.parametrize("BH,nq,nk", [(40, 119, 238), (37, 128, 31)])
+@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 64), (torch.float16, 128)])
+def test_selection_with_two_rows_per_warp(BH, nq, nk, dtype, D):
+    """Problems of many rows run two rows per warp; a single head of them runs one."""
+    from spargeattn_b200 import ops
+    dev = [t.cuda() for t in _pooled(BH, nq, nk, D, dtype, 7)]
+    dev[2:] = [t.to(torch.uint8) for t in dev[2:]]
+    knob = torch.linspace(0.1, 0.9, BH).cuda()
+    for causal in (False, True):
+        lut, valid, mask = ops.select_blocks(*dev, knob, None, causal, True, True, best_first=True)
+        for h in (0, BH // 2, BH - 1):
+            one = ops.select_blocks(*[t[:, h:h + 1].contiguous() for t in dev], knob[h:h + 1], None, causal, True, True, best_first=True)
+            for a, b in zip((lut, valid, mask), one):
+                assert torch.equal(a[:, h:h + 1], b)
+
+
+# around the 256-token span, the block sizes inside it and the size from which partial results are combined by a kernel
+@pytest.mark.parametrize("N", [128, 129, 255, 256, 257, 511, 2048, 2049, 2300])
+@pytest.mark.parametrize("D,dtype,v_dtype", [(64, torch.bfloat16, torch.bfloat16), (128, torch.float16, torch.float16),
+                                             (128, torch.bfloat16, torch.float16)])
+def test_fused_preparation_equals_the_separate_kernels(N, D, dtype, v_dtype):
+    import spargeattn_b200 as S
+    from spargeattn_b200 import core, ops
+    g = torch.Generator().manual_seed(N + D)
+    q, k, v = (torch.randn(2, 3, N, D, generator=g).cuda().to(t) for t in (dtype, dtype, v_dtype))
+    k = k + 2
+    # token-major V of one dtype with Q: what the fp16-PV path reads through its strides
+    v_nhd = v.transpose(1, 2).contiguous().transpose(1, 2)
+    calls = [lambda: S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=0.5, pvthreshd=6.0),
+             lambda: S.spas_sage2_attn_meansim_topk_cuda(q, k, v_nhd, topk=0.5, smooth_k=False, is_causal=True),
+             lambda: S.spas_sage_attn_meansim_topk_cuda(q, k, v, topk=0.5),
+             lambda: S.spas_sage_attn_meansim_topk_cuda(q, k, v_nhd, topk=0.5, is_causal=True),
+             lambda: S.spas_sage_attn_meansim_topk_cuda(q, k, v[:, :1].expand(2, 3, N, D), topk=0.5)]
+    one = [f() for f in calls]
+    limit = core.SINGLE_CALL_MAX_ROWS
+    try:
+        core.SINGLE_CALL_MAX_ROWS = 0
+        sep = [f() for f in calls]
+    finally:
+        core.SINGLE_CALL_MAX_ROWS = limit
+    for a, b in zip(one, sep):
+        assert torch.equal(a, b)
+    # block mask: composed from the separate entries
+    mask = torch.rand(2, 3, (N + 127) // 128, (N + 63) // 64, generator=g) < 0.6
+    for m in (mask.cuda(), mask.to(torch.int64).cuda()):
+        o = S.block_sparse_sage2_attn_cuda(q, k, v, mask_id=m)
+        q8, qs, k8, ks = core.get_vanilla_qk_quant(q, k, ops.k_mean(k))
+        lut, valid = ops.mask_to_lut(m)
+        v8, vs = ops.quant_v(v)
+        assert torch.equal(o, ops.attn_fwd(q8, k8, v8, lut, valid, None, qs, ks, vs, D ** -0.5, False, dtype))
+    ops.check_device_status()
