@@ -85,33 +85,26 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t* w) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
 
-// Row maximum of a block's 64 scores, in log2 units. klim: keys with block-local index >= klim are masked.
-template <bool MASKED>
-__device__ __forceinline__ float block_rowmax(const uint32_t* sr, float c, int klim) {
-  if (!MASKED) {
-    int m[4];   // four chains of 3-input maxima: short latency
+// Row maximum of a block's 64 scores, in log2 units.
+__device__ __forceinline__ float block_rowmax(const uint32_t* sr, float c) {
+  int m[4];   // four chains of 3-input maxima: short latency
 #pragma unroll
-    for (int g = 0; g < 4; g++) {
-      m[g] = __vimax3_s32((int)sr[16 * g], (int)sr[16 * g + 1], (int)sr[16 * g + 2]);
+  for (int g = 0; g < 4; g++) {
+    m[g] = __vimax3_s32((int)sr[16 * g], (int)sr[16 * g + 1], (int)sr[16 * g + 2]);
 #pragma unroll
-      for (int k = 3; k < 15; k += 2) m[g] = __vimax3_s32(m[g], (int)sr[16 * g + k], (int)sr[16 * g + k + 1]);
-    }
-    m[0] = __vimax3_s32(m[0], m[1], (int)sr[15]);
-    m[2] = __vimax3_s32(m[2], m[3], (int)sr[31]);
-    m[0] = __vimax3_s32(m[0], m[2], (int)sr[47]);
-    return __int2float_rn(max(m[0], (int)sr[63])) * c;   // c > 0: max commutes with the scaling
-  } else {
-    int mx = INT_MIN;
-#pragma unroll
-    for (int k = 0; k < 64; k++) mx = (k < klim) ? max(mx, (int)sr[k]) : mx;
-    return (klim > 0) ? __int2float_rn(mx) * c : kMaskValue;
+    for (int k = 3; k < 15; k += 2) m[g] = __vimax3_s32(m[g], (int)sr[16 * g + k], (int)sr[16 * g + k + 1]);
   }
+  m[0] = __vimax3_s32(m[0], m[1], (int)sr[15]);
+  m[2] = __vimax3_s32(m[2], m[3], (int)sr[31]);
+  m[0] = __vimax3_s32(m[0], m[2], (int)sr[47]);
+  return __int2float_rn(max(m[0], (int)sr[63])) * c;   // c > 0: max commutes with the scaling
 }
 
-// Per-thread granularity (QuantGranularity::kPerThread, qk_int_sv_f8_cuda_sm89.cuh:116-136): key column n of a
+// The same with masks and per-column scales: keys with block-local index >= klim are masked. Per-thread granularity
+// (QuantGranularity::kPerThread, qk_int_sv_f8_cuda_sm89.cuh:116-136): key column n of a
 // block is scaled by entry (n % 8) / 2 of the block's four K scales, so a thread's 64 scores carry four different
 // factors c4[0..3] and the integer maximum no longer commutes with the scaling: one maximum per factor.
-__device__ __forceinline__ float block_rowmax_g(const uint32_t* sr, const float* c4, int klim) {
+__device__ __forceinline__ float block_rowmax_masked(const uint32_t* sr, const float* c4, int klim) {
   int mx[4] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN};
 #pragma unroll
   for (int k = 0; k < 64; k++) mx[(k & 7) >> 1] = (k < klim) ? max(mx[(k & 7) >> 1], (int)sr[k]) : mx[(k & 7) >> 1];
@@ -356,7 +349,11 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
         }
       }
       if (lane == 0) {
-        if (s + 1 < nsteps) load_k(s + 1, na, nb, make_int4(na, max(nb, 0), __float_as_int(ka), __float_as_int(kb)));
+        if (s + 1 < nsteps) {
+          // the top bit marks a block whose keys need masks; a second block that there is not has it too
+          auto marked = [&](int j) { return ((j * 64 + 64 > N) || (CAUSAL && (j * 64 + 63 > qi * 128))) ? j | INT_MIN : j; };
+          load_k(s + 1, na, nb, make_int4(marked(na), nb < 0 ? INT_MIN : marked(nb), __float_as_int(ka), __float_as_int(kb)));
+        }
         if (ok && s >= 0) load_v(2 * s, ja);
         if (ok && s >= 0 && jb >= 0) load_v(2 * s + 1, jb);
       }
@@ -488,51 +485,48 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     const int rsw = row & 7;
     float m = kMaskValue, d = 0.f;
     int npv = 0;   // PV products issued for this query block (all of them unless the skip test fires)
-    for (int s = 0; s < nsteps; s++) {
-      const bool two = cnt - 2 * s >= 2;                          // the last step of an odd count has one block
-      mbar_wait_or_flag(&bar_s_full, s & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+    mbar_wait_or_flag(&bar_s_full, 0, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+    for (int s = 0; s < nsteps; s++) {   // S of step s is complete
       tc_fence_after();
       uint32_t sr[128];
       tmem_ld32(tS, sr);
       tmem_ld32(tS + 32, sr + 32);
-      if (two) {
-        tmem_ld32(tS + 64, sr + 64);
-        tmem_ld32(tS + 96, sr + 96);
-      }
-      // the blocks and their scales (published by the producer warp before the step's K tiles were requested)
-      const int4 mt = s_meta[s & 7];
-      tmem_wait_ld();
-      // S is in registers: the MMA warp may overwrite it with the next step's scores
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_s_free);
-
+      tmem_ld32(tS + 64, sr + 64);
+      tmem_ld32(tS + 96, sr + 96);
+      const int4 mt = s_meta[s & 7];   // published by the producer warp before the step's K tiles were requested
+      const bool two = cnt - 2 * s >= 2;                          // the last step of an odd count has one block
+      // Key masks, or one block only: the general path for both blocks. One test, made while the scores travel, keeps the
+      // ordinary step free of branches (with a test per block after the load: 2.44 instead of 2.33 ms at [1,12,32760,128]).
+      const bool plain = !GRAN3 && __all_sync(0xffffffffu, (mt.x | mt.y) >= 0);
       float cc[2][4];   // scale of each block's scores (per-thread granularity: of each pair of key columns)
-      int klim[2];      // keys with block-local index >= klim are masked
-      bool exact[2];
+      int klim[2] = {64, 64};   // keys with block-local index >= klim are masked
 #pragma unroll
       for (int b = 0; b < 2; b++) {
-        const int key0 = (b ? mt.y : mt.x) * 64;
-        if (GRAN3) {
-          const float4 k4 = *reinterpret_cast<const float4*>(ks_row + (size_t)(b ? mt.y : mt.x) * 4);
-          cc[b][0] = qs * k4.x; cc[b][1] = qs * k4.y; cc[b][2] = qs * k4.z; cc[b][3] = qs * k4.w;
-        } else {
-          cc[b][0] = cc[b][1] = cc[b][2] = cc[b][3] = qs * __int_as_float(b ? mt.w : mt.z);
-        }
-        klim[b] = 64;
-        exact[b] = __any_sync(0xffffffffu, (key0 + 64 > N) || (CAUSAL && (key0 + 63 > qi * 128)));
-        if (exact[b]) {
+        cc[b][0] = cc[b][1] = cc[b][2] = cc[b][3] = qs * __int_as_float(b ? mt.w : mt.z);
+        if (!plain) {
+          const int j = (b ? mt.y : mt.x) & INT_MAX, key0 = j * 64;
+          if (GRAN3) {
+            const float4 k4 = *reinterpret_cast<const float4*>(ks_row + (size_t)j * 4);
+            cc[b][0] = qs * k4.x; cc[b][1] = qs * k4.y; cc[b][2] = qs * k4.z; cc[b][3] = qs * k4.w;
+          }
           klim[b] = min(64, N - key0);
           if (CAUSAL) klim[b] = min(klim[b], qrow - key0 + 1);
           klim[b] = max(klim[b], 0);
         }
       }
+      tmem_wait_ld();
+      // S is in registers: the MMA warp may overwrite it with the next step's scores
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_s_free);
       float r[2];
-#pragma unroll
-      for (int b = 0; b < 2; b++)
-        r[b] = (b == 1 && !two) ? m
-               : GRAN3 ? block_rowmax_g(sr + 64 * b, cc[b], klim[b])
-               : exact[b] ? block_rowmax<true>(sr + 64 * b, cc[b][0], klim[b]) : block_rowmax<false>(sr + 64 * b, cc[b][0], 64);
+      if (plain) {
+        r[0] = block_rowmax(sr, cc[0][0]);
+        r[1] = block_rowmax(sr + 64, cc[1][0]);
+      } else {
+        r[0] = block_rowmax_masked(sr, cc[0], klim[0]);
+        r[1] = two ? block_rowmax_masked(sr + 64, cc[1], klim[1]) : m;
+      }
       const float m1 = fmaxf(m, r[0]);                            // maximum after block A
       const float m2 = fmaxf(m1, r[1]);
       // PV-skip test (qk_int_sv_f8_cuda_sm89.cuh:317-353), per 64-key block as in the reference: a block is dropped
@@ -559,19 +553,19 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       if (Shape::kBuffersP == 1 && s > 0) mbar_wait_or_flag(&bar_o_done[(s - 1) & 1], ((s - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
       const uint32_t pb = prow + (s % Shape::kBuffersP) * Shape::kTileP;
       float sum[2] = {0.f, 0.f};
-#pragma unroll
-      for (int b = 0; b < 2; b++) {
-        if (b == 1 && !two) break;
-        // A 32-row group that drops its block in per-warp mode still writes its rows of P (as zeros, through the
-        // exact path with no visible key): the other groups' rows of the same block may be multiplied.
-        if (pv_per_warp && own_skip[b]) klim[b] = 0;
-        const uint32_t dst = pb + (PVF16 ? b * 16384u : 0u);
-        const int chunk0 = PVF16 ? 0 : 4 * b;
-        if (GRAN3 || exact[b] || (pv_per_warp && own_skip[b]))
-          sum[b] = block_exp<true, PVF16>(sr + 64 * b, cc[b], m, klim[b], dst, chunk0, rsw);
-        else
-          sum[b] = block_exp<false, PVF16>(sr + 64 * b, cc[b], m, 64, dst, chunk0, rsw);
+      const uint32_t pb1 = pb + (PVF16 ? 16384u : 0u);
+      constexpr int chunkB = PVF16 ? 0 : 4;
+      if (plain && !(pv_per_warp && (own_skip[0] || own_skip[1]))) {
+        sum[0] = block_exp<false, PVF16>(sr, cc[0], m, 64, pb, 0, rsw);
+        sum[1] = block_exp<false, PVF16>(sr + 64, cc[1], m, 64, pb1, chunkB, rsw);
+      } else {
+        // A 32-row group that drops its block in per-warp mode still writes its rows of P (as zeros, no key being
+        // visible): the other groups' rows of the same block may be multiplied.
+        sum[0] = block_exp<true, PVF16>(sr, cc[0], m, pv_per_warp && own_skip[0] ? 0 : klim[0], pb, 0, rsw);
+        if (two) sum[1] = block_exp<true, PVF16>(sr + 64, cc[1], m, pv_per_warp && own_skip[1] ? 0 : klim[1], pb1, chunkB, rsw);
       }
+      // asked here, needed at the end of the step: the answer's latency is hidden
+      const bool next_ready = s + 1 < nsteps && mbar_test(&bar_s_full, (s + 1) & 1);
       // A wait names a phase by its parity, so the waiter must know that the phase before it is complete: PV(s-3), the
       // previous user of this barrier, is (see above). With one barrier for all steps that would not hold.
       if (need_rescale) {   // some row of this warp raised its maximum: O must hold everything up to PV(s-1)
@@ -620,6 +614,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_p_ready[s & 1]);   // (two barriers: a warp may be a step ahead of another)
+      if (s + 1 < nsteps && !__all_sync(0xffffffffu, next_ready))
+        mbar_wait_or_flag(&bar_s_full, (s + 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
     }
     mbar_wait_or_flag(&bar_o_done[(nsteps - 1) & 1], ((nsteps - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
     tc_fence_after();
