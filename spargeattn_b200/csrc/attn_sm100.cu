@@ -42,7 +42,7 @@ constexpr float kMaskValue = -5000000.0f;  // csrc/qattn/attn_utils.cuh:348-352
 // (csrc/qattn/qk_int_sv_f16_cuda_sm80.cuh), which its Sage1-signature entry points run. V then is the caller's fp16
 // tensor itself (no quantiser); a 64-key V tile is D/64 sub-tiles of [64 keys x 128 bytes] (64 channels each, 128B
 // swizzle), P is two sub-tiles of [128 rows x 128 bytes], one per block of a pair. The tiles are twice as large,
-// so P has one buffer and the rings are shorter (see kKTiles) to keep two CTAs per SM.
+// so the rings are shorter (see kKTiles), and at D = 128 P has one buffer, to keep two CTAs per SM.
 template <int D, bool PVF16 = false>
 struct AttnShape {
   // K ring of single tiles (fp16 variant at D = 128): three 64-key tile slots instead of two pair slots bring the CTA
@@ -50,13 +50,13 @@ struct AttnShape {
   // adjacent and QK^T is issued as two N = 64 instruction groups.
   static constexpr bool kKTiles = PVF16 && D == 128;
   static constexpr int kStagesK = kKTiles ? 3 : (D == 128 || PVF16) ? 2 : 4;   // ring slots: PAIRS of 64-key tiles (tiles if kKTiles)
-  static constexpr int kSlotsV = PVF16 ? (D == 128 ? 2 : 4) : (D == 128 ? 3 : 8);   // single 64-key tiles
+  static constexpr int kSlotsV = PVF16 ? 2 : (D == 128 ? 3 : 8);   // single 64-key tiles
   static constexpr int kTileQ = 128 * D;
   static constexpr int kTileKV = 64 * D;
   static constexpr int kPairKV = 2 * kTileKV;
   static constexpr int kTileV = PVF16 ? 2 * kTileKV : kTileKV;
   static constexpr int kTileP = PVF16 ? 2 * 128 * 128 : 128 * 128;   // 128 rows x 128 keys of e4m3 / fp16
-  static constexpr int kBuffersP = PVF16 ? 1 : 2;
+  static constexpr int kBuffersP = PVF16 && D == 128 ? 1 : 2;
   static constexpr int kRingK = kStagesK * (kKTiles ? kTileKV : kPairKV);
   static constexpr int kSmemBytes = 1024 + kTileQ + kBuffersP * kTileP + kRingK + kSlotsV * kTileV;
   static constexpr int kTmemCols = 256;
@@ -548,19 +548,29 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       const float alpha = (s > 0) ? ex2_approx(m - m2) : 0.f;
       const bool need_rescale = (s > 0) && __any_sync(0xffffffffu, m2 > m);
       m = m2;
-      // PV of the step that used this P buffer must have retired before the buffer is overwritten. With two buffers that
-      // is step s - 2, whose products were issued before QK^T of this step, so S being complete shows it.
-      if (Shape::kBuffersP == 1 && s > 0) mbar_wait_or_flag(&bar_o_done[(s - 1) & 1], ((s - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+      // P.V of the step that used this P buffer must have retired before the buffer is overwritten. With two buffers that
+      // is step s - 2, whose products were issued before QK^T of this step, so S being complete shows it. With one buffer it
+      // is the step before, block by block: its V tile is handed back when its product is done.
+      auto wait_p = [&](int b) {
+        if (Shape::kBuffersP == 1 && s > 0) {
+          const int n = 2 * (s - 1) + b;
+          mbar_wait_or_flag(&bar_v_empty[n % NV], (n / NV) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+        }
+      };
       const uint32_t pb = prow + (s % Shape::kBuffersP) * Shape::kTileP;
       float sum[2] = {0.f, 0.f};
       const uint32_t pb1 = pb + (PVF16 ? 16384u : 0u);
       constexpr int chunkB = PVF16 ? 0 : 4;
       if (plain && !(pv_per_warp && (own_skip[0] || own_skip[1]))) {
+        wait_p(0);
         sum[0] = block_exp<false, PVF16>(sr, cc[0], m, 64, pb, 0, rsw);
+        wait_p(1);
         sum[1] = block_exp<false, PVF16>(sr + 64, cc[1], m, 64, pb1, chunkB, rsw);
       } else {
         // A 32-row group that drops its block in per-warp mode still writes its rows of P (as zeros, no key being
         // visible): the other groups' rows of the same block may be multiplied.
+        wait_p(0);
+        wait_p(1);
         sum[0] = block_exp<true, PVF16>(sr, cc[0], m, pv_per_warp && own_skip[0] ? 0 : klim[0], pb, 0, rsw);
         if (two) sum[1] = block_exp<true, PVF16>(sr + 64, cc[1], m, pv_per_warp && own_skip[1] ? 0 : klim[1], pb1, chunkB, rsw);
       }
@@ -569,7 +579,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       // A wait names a phase by its parity, so the waiter must know that the phase before it is complete: PV(s-3), the
       // previous user of this barrier, is (see above). With one barrier for all steps that would not hold.
       if (need_rescale) {   // some row of this warp raised its maximum: O must hold everything up to PV(s-1)
-        if (Shape::kBuffersP > 1) mbar_wait_or_flag(&bar_o_done[(s - 1) & 1], ((s - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
+        mbar_wait_or_flag(&bar_o_done[(s - 1) & 1], ((s - 1) >> 1) & 1, &s_fail, SPARGE_DEV_TIMEOUT_SOFTMAX);
         tc_fence_after();
         const float2 al2 = make_float2(alpha, alpha);
 #pragma unroll
