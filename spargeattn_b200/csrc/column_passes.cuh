@@ -16,14 +16,16 @@ struct PassShape {
   static constexpr int kThreadsPerRow = D / 8, kRowsPerPass = kPassThreads / kThreadsPerRow;
 };
 
-// fp16(v) as a float: the value the V quantiser sees whatever the input type
+// fp16(v) of two neighbouring values: what the V quantiser sees whatever the input type. Pairs all through: converting,
+// comparing and scaling one value at a time took a third more instructions.
 template <typename T>
-__device__ __forceinline__ float to_f16_value(T v);
+__device__ __forceinline__ __half2 to_half2(const T* v);
 template <>
-__device__ __forceinline__ float to_f16_value<__half>(__half v) { return __half2float(v); }
+__device__ __forceinline__ __half2 to_half2<__half>(const __half* v) { return *reinterpret_cast<const __half2*>(v); }
 template <>
-__device__ __forceinline__ float to_f16_value<__nv_bfloat16>(__nv_bfloat16 v) {
-  return __half2float(__float2half_rn(__bfloat162float(v)));
+__device__ __forceinline__ __half2 to_half2<__nv_bfloat16>(const __nv_bfloat16* v) {
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(v);
+  return __float22half2_rn(make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)));
 }
 
 // a / b as fused.cu computes it under --use_fast_math
@@ -79,15 +81,19 @@ template <typename T, int D>
 __device__ __forceinline__ float column_amax(float (*red)[D], const T* __restrict__ head, int row_begin, int row_end, long long sn) {
   constexpr int TPR = PassShape<D>::kThreadsPerRow, RPP = PassShape<D>::kRowsPerPass;
   const int tid = threadIdx.x, cg = tid % TPR, r0 = tid / TPR;
-  float mx[8];
+  __half2 mx[4];
 #pragma unroll
-  for (int i = 0; i < 8; i++) mx[i] = 0.f;
+  for (int i = 0; i < 4; i++) mx[i] = __floats2half2_rn(0.f, 0.f);
   for_rows<T, D, 8>(head, row_begin, row_end, sn, [&](int, const Pack8<T>& p) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) mx[i] = fmaxf(mx[i], fabsf(to_f16_value<T>(p.v[i])));
+    for (int i = 0; i < 4; i++) mx[i] = __hmax2(mx[i], __habs2(to_half2<T>(p.v + 2 * i)));
   });
 #pragma unroll
-  for (int i = 0; i < 8; i++) red[r0][cg * 8 + i] = mx[i];
+  for (int i = 0; i < 4; i++) {
+    const float2 f = __half22float2(mx[i]);
+    red[r0][cg * 8 + 2 * i] = f.x;
+    red[r0][cg * 8 + 2 * i + 1] = f.y;
+  }
   __syncthreads();
   float m = 0.f;
   if (tid < D) {
@@ -104,11 +110,11 @@ __device__ __forceinline__ void v_quant_rows(const T* __restrict__ head, uint8_t
   constexpr int TPR = PassShape<D>::kThreadsPerRow, RPP = PassShape<D>::kRowsPerPass;
   const int cg = threadIdx.x % TPR, r0 = threadIdx.x / TPR;
   for_rows<T, D, 4>(head, row_begin, min(row_end, N), sn, [&](int row, const Pack8<T>& p) {
-    float f[8];
+    float2 f[4];
 #pragma unroll
-    for (int i = 0; i < 8; i++) f[i] = __fmul_rn(to_f16_value<T>(p.v[i]), r8[i]);
+    for (int i = 0; i < 4; i++) f[i] = __fmul2_rn(__half22float2(to_half2<T>(p.v + 2 * i)), make_float2(r8[2 * i], r8[2 * i + 1]));
     *reinterpret_cast<uint2*>(out + (size_t)row * D + cg * 8) =
-        make_uint2(cvt_e4m3x4(f[0], f[1], f[2], f[3]), cvt_e4m3x4(f[4], f[5], f[6], f[7]));
+        make_uint2(cvt_e4m3x4(f[0].x, f[0].y, f[1].x, f[1].y), cvt_e4m3x4(f[2].x, f[2].y, f[3].x, f[3].y));
   });
   for (int row = max(row_begin, N) + r0; row < row_end; row += RPP)   // padding rows are zeros
     *reinterpret_cast<uint2*>(out + (size_t)row * D + cg * 8) = make_uint2(0u, 0u);
@@ -120,10 +126,10 @@ __device__ __forceinline__ void v_half_rows(const T* __restrict__ head, __half* 
                                             long long sn) {
   const int cg = threadIdx.x % PassShape<D>::kThreadsPerRow;
   for_rows<T, D, 8>(head, row_begin, row_end, sn, [&](int row, const Pack8<T>& p) {
-    Pack8<__half> h;
+    alignas(16) __half2 h[4];
 #pragma unroll
-    for (int i = 0; i < 8; i++) h.v[i] = __float2half_rn(Elem<T>::to_float(p.v[i]));
-    *reinterpret_cast<Pack8<__half>*>(out + (size_t)row * D + cg * 8) = h;
+    for (int i = 0; i < 4; i++) h[i] = to_half2<T>(p.v + 2 * i);
+    *reinterpret_cast<uint4*>(out + (size_t)row * D + cg * 8) = *reinterpret_cast<const uint4*>(h);
   });
 }
 

@@ -49,6 +49,19 @@ __device__ __forceinline__ uint32_t pack2_rn<__half>(float2 v) {
   const __half2 h = __float22half2_rn(v);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
+// per-half max(a, |b|) of 16-bit pairs, a >= 0
+template <typename T>
+__device__ __forceinline__ uint32_t max_abs2(uint32_t a, uint32_t b);
+template <>
+__device__ __forceinline__ uint32_t max_abs2<__nv_bfloat16>(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&b)));
+  return *reinterpret_cast<const uint32_t*>(&m);
+}
+template <>
+__device__ __forceinline__ uint32_t max_abs2<__half>(uint32_t a, uint32_t b) {
+  const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&a), __habs2(*reinterpret_cast<const __half2*>(&b)));
+  return *reinterpret_cast<const uint32_t*>(&m);
+}
 // {sat8(hi), sat8(lo)} into the low half of the result, the low half of `upper` into its high half
 __device__ __forceinline__ uint32_t pack_s8x2(int hi, int lo, uint32_t upper) {
   uint32_t d;
@@ -114,7 +127,7 @@ __device__ __forceinline__ void pool_quant_blocks(PoolQuantShared<D, BS, NSUB, W
   }
 
   // ---- pass 1: mean subtraction in the 16-bit type, amax, pooled sums, partial sums of squares
-  float amax = 0.f;
+  uint32_t amax2[2] = {0u, 0u};   // pairs of 16-bit maxima
   float2 pacc[4];
   float ss[8];
 #pragma unroll
@@ -135,8 +148,8 @@ __device__ __forceinline__ void pool_quant_blocks(PoolQuantShared<D, BS, NSUB, W
         raw[i] = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
-    amax = fmaxf(amax, fmaxf(fmaxf(fmaxf(fabsf(v[0].x), fabsf(v[0].y)), fmaxf(fabsf(v[1].x), fabsf(v[1].y))),
-                             fmaxf(fmaxf(fabsf(v[2].x), fabsf(v[2].y)), fmaxf(fabsf(v[3].x), fabsf(v[3].y)))));
+#pragma unroll
+    for (int c = 0; c < 4; c++) amax2[c & 1] = max_abs2<T>(amax2[c & 1], w[c]);
     if (WANT_POOL) {
       float q = 0.f;
 #pragma unroll
@@ -188,7 +201,11 @@ __device__ __forceinline__ void pool_quant_blocks(PoolQuantShared<D, BS, NSUB, W
 
   // ---- block amax -> scale
   // the flag for an all-zero row travels in the sign bit of the warp's maximum, so that one barrier serves both
-  amax = warp_max(amax);
+  float amax;
+  {
+    const float2 a = unpack2<T>(max_abs2<T>(amax2[0], amax2[1]));
+    amax = warp_max(fmaxf(a.x, a.y));
+  }
   const bool warp_zero = __any_sync(0xffffffffu, zero_row);
   if (lane == 0) sm.amax[warp] = warp_zero ? __uint_as_float(__float_as_uint(amax) | 0x80000000u) : amax;
   if (WANT_POOL) {
