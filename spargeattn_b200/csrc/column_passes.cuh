@@ -8,12 +8,23 @@
 
 namespace sparge {
 
+// What the FP8 quantisation of V needs once the column maxima are known.
+struct VQuantArgs {
+  const void* v;                    // [B,H,N,D] view; NULL: nothing to do
+  long long st[3];                  // strides of (batch, head, token) in elements
+  void* out;                        // [B,H,N_pad,D] e4m3
+  float* v_scale;                   // [B,H,D]
+  const float* vmax;                // [B*H, parts, D]
+  int parts, spans, N, H, dtype;
+};
+
 constexpr int kPassThreads = 256;
+constexpr int kSpan = 256;   // tokens of one head that a CTA takes
 constexpr float kVScaleMax = 2.25f;   // spas_sage_attn/core.py:151
 
-template <int D>
+template <int D, int THREADS = kPassThreads>
 struct PassShape {
-  static constexpr int kThreadsPerRow = D / 8, kRowsPerPass = kPassThreads / kThreadsPerRow;
+  static constexpr int kThreadsPerRow = D / 8, kRowsPerPass = THREADS / kThreadsPerRow;
 };
 
 // fp16(v) of two neighbouring values: what the V quantiser sees whatever the input type. Pairs all through: converting,
@@ -38,9 +49,9 @@ __device__ __forceinline__ float div_approx(float a, float b) {
 __device__ __forceinline__ float v_multiplier(float amax) { return amax > 0.f ? div_approx(kVScaleMax, amax) : 0.f; }
 
 // f(row, values) for the rows of [row_begin, row_end) that this thread owns, UNROLL loads in flight
-template <typename T, int D, int UNROLL, typename F>
+template <typename T, int D, int UNROLL, int THREADS = kPassThreads, typename F>
 __device__ __forceinline__ void for_rows(const T* __restrict__ head, int row_begin, int row_end, long long sn, F f) {
-  constexpr int TPR = PassShape<D>::kThreadsPerRow, RPP = PassShape<D>::kRowsPerPass;
+  constexpr int TPR = PassShape<D, THREADS>::kThreadsPerRow, RPP = PassShape<D, THREADS>::kRowsPerPass;
   const int cg = threadIdx.x % TPR;
   int row = row_begin + threadIdx.x / TPR;
   for (; row + (UNROLL - 1) * RPP < row_end; row += UNROLL * RPP) {
@@ -104,12 +115,12 @@ __device__ __forceinline__ float column_amax(float (*red)[D], const T* __restric
 }
 
 // FP8 quantisation of rows [row_begin, row_end) of the padded output; r8: multipliers of this thread's 8 channels
-template <typename T, int D>
+template <typename T, int D, int THREADS = kPassThreads>
 __device__ __forceinline__ void v_quant_rows(const T* __restrict__ head, uint8_t* __restrict__ out, const float* r8, int row_begin,
                                              int row_end, int N, long long sn) {
-  constexpr int TPR = PassShape<D>::kThreadsPerRow, RPP = PassShape<D>::kRowsPerPass;
+  constexpr int TPR = PassShape<D, THREADS>::kThreadsPerRow, RPP = PassShape<D, THREADS>::kRowsPerPass;
   const int cg = threadIdx.x % TPR, r0 = threadIdx.x / TPR;
-  for_rows<T, D, 4>(head, row_begin, min(row_end, N), sn, [&](int row, const Pack8<T>& p) {
+  for_rows<T, D, 4, THREADS>(head, row_begin, min(row_end, N), sn, [&](int row, const Pack8<T>& p) {
     float2 f[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) f[i] = __fmul2_rn(__half22float2(to_half2<T>(p.v + 2 * i)), make_float2(r8[2 * i], r8[2 * i + 1]));
@@ -118,6 +129,27 @@ __device__ __forceinline__ void v_quant_rows(const T* __restrict__ head, uint8_t
   });
   for (int row = max(row_begin, N) + r0; row < row_end; row += RPP)   // padding rows are zeros
     *reinterpret_cast<uint2*>(out + (size_t)row * D + cg * 8) = make_uint2(0u, 0u);
+}
+
+// FP8 quantisation of one span of one head by a CTA of THREADS threads, from the head's column maxima
+template <int D, int THREADS>
+__device__ __forceinline__ void v_quant_span(const VQuantArgs& a, float (&s_mul)[D], int span, int bh) {
+  const int tid = threadIdx.x, n_pad = (a.N + 127) / 128 * 128, r0 = span * kSpan, r1 = min(n_pad, r0 + kSpan);
+  for (int d = tid; d < D; d += THREADS) {
+    float m = 0.f;
+#pragma unroll 8
+    for (int c = 0; c < a.parts; c++) m = fmaxf(m, a.vmax[((size_t)bh * a.parts + c) * D + d]);
+    s_mul[d] = v_multiplier(m);
+    if (span == 0) a.v_scale[(size_t)bh * D + d] = div_approx(m, kVScaleMax);
+  }
+  __syncthreads();
+  float r8[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) r8[i] = s_mul[(tid % PassShape<D>::kThreadsPerRow) * 8 + i];
+  uint8_t* out = (uint8_t*)a.out + (size_t)bh * n_pad * D;
+  const size_t head = (size_t)(bh / a.H) * a.st[0] + (size_t)(bh % a.H) * a.st[1];
+  if (a.dtype == SPARGE_F16) v_quant_rows<__half, D, THREADS>((const __half*)a.v + head, out, r8, r0, r1, a.N, a.st[2]);
+  else v_quant_rows<__nv_bfloat16, D, THREADS>((const __nv_bfloat16*)a.v + head, out, r8, r0, r1, a.N, a.st[2]);
 }
 
 // fp16 copy of rows [row_begin, row_end)

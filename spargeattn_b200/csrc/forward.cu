@@ -64,13 +64,19 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
   p.v_out = ws + off[kWsV8], p.v_scale = (float*)(ws + off[kWsVs]), p.km = ws + off[kWsKm], p.scratch = ws + off[kWsScratch];
   p.BH = a.B * a.H, p.H = a.H, p.N = a.N, p.D = a.D, p.dtype = a.dtype, p.v_dtype = a.v_dtype, p.smooth_k = a.smooth_k;
   p.v_mode = copy_v ? kVHalf : a.pv_fp16 ? kVNone : kVFp8;
-  int rc = prep_launch(p, st);
+  // While the selection has at most eight rows per SM it is a chain of latencies that leaves the memory system idle: V is
+  // quantised beside it. From there on it fills the chip, and V is cheaper beside K, where its rows are still in L2.
+  // Whole call, us, beside K / beside the selection: 39.4 / 36.9 (2 x 8 heads of 1000), 181.0 / 179.6 (24 of 4608),
+  // 416.5 / 415.5 (16 of 8191), but 2 541 / 2 543 (12 of 32760) and 3 586 / 3 606 (60 of 17776, D = 64).
+  VQuantArgs v_later = {};
+  const bool v_beside_selection = select && (long long)p.BH * nq <= 8 * 148;
+  int rc = prep_launch(p, v_beside_selection ? &v_later : nullptr, st);
   if (rc != SPARGE_OK) return rc;
 
   if (select) {
     // the skip test exempts the last two live blocks of the visiting order: best-first order only without it
     const SelectArgs s = {p.pq, p.pk, p.sim_q, p.sim_k, a.topk, a.cdf, nullptr, lut, valid, p.BH, a.H, nq, nk, a.D, a.dtype,
-                          a.is_causal, a.sink, a.pvthr == nullptr, true};
+                          a.is_causal, a.sink, a.pvthr == nullptr, true, v_later};
     rc = select_launch(s, st);
   } else {
     rc = mask_to_lut_launch(a.mask, a.mask_elem_size, lut, valid, (long long)p.BH * nq, nk, true, st);

@@ -2,6 +2,7 @@
 //   1  Q pooled and quantised | column sums of K | column maxima of V        (one read of each tensor)
 //   1b partial sums and maxima combined, when there are many of them
 //   2  K pooled and quantised with its mean taken out | V quantised to FP8   (a second read of K and V)
+//      (beside a short selection V's part runs in the selection's grid instead: see forward.cu)
 // The arithmetic is that of the standalone entries (kmean.cu, pool_quant.cu, quant_v.cu), so the bytes are the same.
 //
 // Why one launch for three tensors: pooling is bound by instruction issue and the column passes by memory, so their
@@ -15,7 +16,6 @@
 
 namespace sparge {
 
-constexpr int kSpan = 256;
 // Up to this many partial results per head are combined by every CTA that needs them (8 KB from L2 at D = 128); from
 // there on a kernel of its own does it once per head.
 constexpr int kDirectParts = 8;
@@ -118,11 +118,12 @@ __global__ void __launch_bounds__(1024) prep_combine_kernel(PrepScratch s, int s
   pdl_trigger();
 }
 
-// grid (spans * units, B*H), 256 threads. kp, vp: `parts` partial results per head. Walks the tensors back to front:
+// grid (spans * units, B*H), 256 threads. kp: `parts` partial results per head. Walks the tensors back to front:
 // what the first kernel read last is still in L2.
 template <typename T, int D, bool SMOOTH_K, bool WANT_POOL>
 __global__ void __launch_bounds__(kPassThreads, 3)
-prep_second_kernel(const __grid_constant__ PrepArgs a, const double* __restrict__ kp, const float* __restrict__ vp, int parts, int spans) {
+prep_second_kernel(const __grid_constant__ PrepArgs a, const __grid_constant__ VQuantArgs vq, const double* __restrict__ kp, int parts,
+                   int spans) {
   using Shape = PrepShape<D>;
   constexpr int KU = Shape::kKUnits;
   __shared__ PoolQuantShared<D, 64, Shape::kKBlocks, WANT_POOL> sm;
@@ -150,33 +151,20 @@ prep_second_kernel(const __grid_constant__ PrepArgs a, const double* __restrict_
     }
   } else {
     pdl_wait();
-    const int n_pad = (a.N + 127) / 128 * 128, r0 = span * kSpan, r1 = min(n_pad, r0 + kSpan);
-    if (tid < D) {
-      float m = 0.f;
-      for (int c = 0; c < parts; c++) m = fmaxf(m, vp[((size_t)bh * parts + c) * D + tid]);
-      s_mul[tid] = v_multiplier(m);
-      if (span == 0) a.v_scale[(size_t)bh * D + tid] = div_approx(m, kVScaleMax);
-    }
-    __syncthreads();
-    float r8[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) r8[i] = s_mul[(tid % PassShape<D>::kThreadsPerRow) * 8 + i];
-    uint8_t* out = (uint8_t*)a.v_out + (size_t)bh * n_pad * D;
-    if (a.v_dtype == SPARGE_F16) v_quant_rows<__half, D>(head_of<__half>(a.v, a.v_st, bh, a.H), out, r8, r0, r1, a.N, a.v_st[2]);
-    else v_quant_rows<__nv_bfloat16, D>(head_of<__nv_bfloat16>(a.v, a.v_st, bh, a.H), out, r8, r0, r1, a.N, a.v_st[2]);
+    v_quant_span<D, kPassThreads>(vq, s_mul, span, bh);
   }
   pdl_trigger();
 }
 
 template <typename T, int D>
-static int prep_launch_t(const PrepArgs& a, cudaStream_t st) {
+static int prep_launch_t(const PrepArgs& a, VQuantArgs* v_later, cudaStream_t st) {
   using Shape = PrepShape<D>;
   PrepScratch s;
   prep_scratch(a.BH, a.N, D, a.scratch, &s);
   const int spans = (a.N + kSpan - 1) / kSpan;
   const bool want = a.simthr != nullptr, smooth = a.smooth_k != 0, v8 = a.v_mode == kVFp8;
   const int units1 = Shape::kQUnits + (smooth ? 1 : 0) + (a.v_mode != kVNone ? 1 : 0);
-  const int units2 = Shape::kKUnits + (v8 ? 1 : 0);
+  const int units2 = Shape::kKUnits + (v8 && !v_later ? 1 : 0);
   cudaError_t e = launch(want ? prep_first_kernel<T, D, true> : prep_first_kernel<T, D, false>, dim3(spans * units1, a.BH),
                          kPassThreads, 0, st, false, a, s, spans);
   const double* kp = s.kpart;
@@ -190,13 +178,15 @@ static int prep_launch_t(const PrepArgs& a, cudaStream_t st) {
   }
   auto second = smooth ? (want ? prep_second_kernel<T, D, true, true> : prep_second_kernel<T, D, true, false>)
                        : (want ? prep_second_kernel<T, D, false, true> : prep_second_kernel<T, D, false, false>);
-  if (e == cudaSuccess) e = launch(second, dim3(spans * units2, a.BH), kPassThreads, 0, st, true, a, kp, vp, parts, spans);
+  const VQuantArgs vq = {a.v, {a.v_st[0], a.v_st[1], a.v_st[2]}, a.v_out, a.v_scale, vp, parts, spans, a.N, a.H, a.v_dtype};
+  if (v_later && v8) *v_later = vq;
+  if (e == cudaSuccess) e = launch(second, dim3(spans * units2, a.BH), kPassThreads, 0, st, true, a, vq, kp, parts, spans);
   return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
 }
 
-int prep_launch(const PrepArgs& a, cudaStream_t st) {
-  if (a.dtype == SPARGE_F16) return a.D == 64 ? prep_launch_t<__half, 64>(a, st) : prep_launch_t<__half, 128>(a, st);
-  return a.D == 64 ? prep_launch_t<__nv_bfloat16, 64>(a, st) : prep_launch_t<__nv_bfloat16, 128>(a, st);
+int prep_launch(const PrepArgs& a, VQuantArgs* v_later, cudaStream_t st) {
+  if (a.dtype == SPARGE_F16) return a.D == 64 ? prep_launch_t<__half, 64>(a, v_later, st) : prep_launch_t<__half, 128>(a, v_later, st);
+  return a.D == 64 ? prep_launch_t<__nv_bfloat16, 64>(a, v_later, st) : prep_launch_t<__nv_bfloat16, 128>(a, v_later, st);
 }
 
 }  // namespace sparge

@@ -1,6 +1,6 @@
 // What precedes the selection and the attention kernel of a call, in two launches (three for long sequences).
 #pragma once
-#include "common.cuh"
+#include "column_passes.cuh"
 
 namespace sparge {
 
@@ -22,6 +22,8 @@ struct PrepArgs {
 };
 
 size_t prep_scratch_bytes(int BH, int N, int D);
-int prep_launch(const PrepArgs& a, cudaStream_t st);
+// v_later: if not NULL, the FP8 quantisation of V is left to the caller, who gets what it needs (v stays NULL if V is not to
+// be quantised).
+int prep_launch(const PrepArgs& a, VQuantArgs* v_later, cudaStream_t st);
 
 }  // namespace sparge

@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t* __restrict__ sim_q,
               const uint8_t* __restrict__ sim_k, const float* __restrict__ topk, const float* __restrict__ cdfthr,
               uint8_t* __restrict__ mask, int32_t* __restrict__ lut, int32_t* __restrict__ valid, int H, int nq, int nk,
-              int is_causal, int sink, int best_first, int scan_log_nx, int cdf_len) {
+              int is_causal, int sink, int best_first, int scan_log_nx, int cdf_len, const __grid_constant__ VQuantArgs vq, int row_ctas) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int kTileRowBytes = D * (int)sizeof(T) + 16;   // 16-byte pad: conflict-free 128-bit reads, one row per lane
   constexpr int kChunksPerRow = D * (int)sizeof(T) / 16;
@@ -267,6 +267,14 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
   // causal: a row sees the key blocks k < 2 (q + 1)
   auto limit_of = [&](int q) { return is_causal ? min(nk, (q + 1) * (kBlockQ / kBlockK)) : nk; };
   pdl_wait();
+  // The grid's other blocks quantise V, which only the attention kernel waits for: a row is a chain of latencies or bound by
+  // issue, V's pass is bound by memory.
+  if ((int)blockIdx.x >= row_ctas) {
+    __shared__ float s_mul[D];
+    v_quant_span<D, WARPS * 32>(vq, s_mul, blockIdx.x - row_ctas, bh);
+    pdl_trigger();
+    return;
+  }
   // asked for here, needed long after: a row is a chain of short steps, and a load in it would stall all of them
   const float n_or_thr = cdfthr ? cdfthr[h] : topk[h];
   uint8_t q_similar[RW];
@@ -559,9 +567,10 @@ static int launch_select(const SelectArgs& a, cudaStream_t st) {
   auto kern = select_kernel<T, D, RW, WARPS>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return SPARGE_ERR_CUDA;
-  const cudaError_t e = launch(kern, dim3((a.nq + WARPS * RW - 1) / (WARPS * RW), a.BH), WARPS * 32, smem, st, a.dependent,
+  const int row_ctas = (a.nq + WARPS * RW - 1) / (WARPS * RW);
+  const cudaError_t e = launch(kern, dim3(row_ctas + (a.vq.v ? a.vq.spans : 0), a.BH), WARPS * 32, smem, st, a.dependent,
                                (const T*)a.pq, (const T*)a.pk, a.sim_q, a.sim_k, a.topk, a.cdf, a.mask, a.lut, a.valid, a.H, a.nq,
-                               a.nk, a.causal, a.sink, a.best_first, scan_log_nx, cdf_len);
+                               a.nk, a.causal, a.sink, a.best_first, scan_log_nx, cdf_len, a.vq, row_ctas);
   return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
 }
 
@@ -611,7 +620,7 @@ extern "C" int sparge_select(const void* pq, const void* pk, const uint8_t* sim_
     return SPARGE_ERR_INVALID_ARG;
   if ((long long)B * H > 65535) return SPARGE_ERR_TOO_LARGE;
   const SelectArgs a = {pq, pk, sim_q, sim_k, topk, cdfthreshd, mask, lut, valid, B * H, H, nq, nk, D, dtype, is_causal,
-                        attention_sink, lut_order != 0, false};
+                        attention_sink, lut_order != 0, false, {}};
   return select_launch(a, (cudaStream_t)stream);
 }
 

@@ -1,6 +1,6 @@
 // Launches of the block selection (select.cu) for the C entry points.
 #pragma once
-#include "common.cuh"
+#include "column_passes.cuh"
 
 namespace sparge {
 
@@ -12,6 +12,7 @@ struct SelectArgs {
   int32_t *lut, *valid;
   int BH, H, nq, nk, D, dtype, causal, sink, best_first;
   bool dependent;                   // programmatic launch behind the kernel before it on the stream
+  VQuantArgs vq;                    // V quantised beside the selection; v == NULL: none
 };
 int select_launch(const SelectArgs& a, cudaStream_t st);
 
