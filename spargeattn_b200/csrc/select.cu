@@ -18,6 +18,8 @@
 //            half an ulp). The kernel runs the same scan in the same order and the same binary search with
 //            the fp32 comparison torch uses, so n_sel equals the reference's wherever the 16-bit
 //            probabilities themselves agree; clamped to [1, nk].
+//   a row with a score of +inf or NaN (a 16-bit score overflows from 65 520 in fp16) has NaN probabilities only, all equal
+//            in the order: its first n_sel blocks, in cdf mode all of them.
 #include <cfloat>
 
 #include "launch.cuh"
@@ -381,6 +383,9 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
     }
     Z = warp_sum(Z);
     const double rz = 1.0 / Z;
+    // An infinite or NaN score makes all probabilities of its row NaN, which a descending order takes as equal: the first
+    // n_sel blocks. Zeros are equal too, and the comparisons below can count them.
+    const bool undefined = Z != Z;
     const int padded = (nk + 255) / 256 * 256;
     for (int j = lane; j < padded; j += 32) {
       uint16_t key = 0;
@@ -388,7 +393,7 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
         const uint16_t raw = s_key[j];
         const float sc = key_value<T>(raw);
         if (raw == kNotSimilarScore) key = kNotSimilarKey;
-        else if (sc != -INFINITY) key = (uint16_t)key_bits<T>(Elem<T>::from_float((float)(exp_nonpositive((double)sc - (double)mx) * rz)));
+        else if (sc != -INFINITY && !undefined) key = (uint16_t)key_bits<T>(Elem<T>::from_float((float)(exp_nonpositive((double)sc - (double)mx) * rz)));
       }
       s_key[j] = key;
     }
@@ -416,7 +421,7 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
         const int mid = lo_i + ((hi_i - lo_i) >> 1);
         if (!(key_value<T>(s_cdf[mid]) > thr)) lo_i = mid + 1; else hi_i = mid;
       }
-      n_sel = lo_i;
+      n_sel = undefined ? nk : lo_i;                         // no sum of NaNs exceeds the threshold
     }
     n_sel = max(1, min(n_sel, nk));
 

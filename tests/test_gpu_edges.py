@@ -86,3 +86,24 @@ def test_fused_preparation_equals_the_separate_kernels(N, D, dtype, v_dtype):
         v8, vs = ops.quant_v(v)
         assert torch.equal(o, ops.attn_fwd(q8, k8, v8, lut, valid, None, qs, ks, vs, D ** -0.5, False, dtype))
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf"), 6e4])
+def test_selection_of_rows_without_defined_probabilities(dtype, causal, value):
+    """NaN, infinite and (6e4 in fp16) overflowing scores: the first blocks of the row are selected, not all of them."""
+    from spargeattn_b200 import ops
+    pq, pk, sim_q, sim_k = _pooled(2, 40, 70, 64, dtype, 3)
+    sim_q[:] = True
+    pq[0, 0, 30, 5] = value
+    pk[0, 1, 9] = value
+    dev = [t.cuda() for t in (pq, pk, sim_q.to(torch.uint8), sim_k.to(torch.uint8))]
+    p = O.pooled_probs(pq, pk, sim_k, causal)
+    for topk, cdf in ((0.1, None), (None, 0.7)):
+        knob = torch.full((2,), topk or cdf)
+        want = O.select_blocks(p, sim_q, sim_k, knob if topk else None, knob if cdf else None, causal, False)
+        lut, valid, mask = ops.select_blocks(*dev, knob.cuda() if topk else None, knob.cuda() if cdf else None, causal, False, True)
+        assert torch.equal(mask.cpu().bool(), want)
+        lut_o, valid_o = O.block_map_to_lut(want)
+        assert torch.equal(lut.cpu(), lut_o) and torch.equal(valid.cpu(), valid_o)
