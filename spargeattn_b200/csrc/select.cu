@@ -272,8 +272,8 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
   // The grid's other blocks quantise V, which only the attention kernel waits for: a row is a chain of latencies or bound by
   // issue, V's pass is bound by memory.
   if ((int)blockIdx.x >= row_ctas) {
-    __shared__ float s_mul[D];
-    v_quant_span<D, WARPS * 32>(vq, s_mul, blockIdx.x - row_ctas, bh);
+    // in the tile's place: the kernel has no static shared memory, which would count against the 48 KB of launch_select
+    v_quant_span<D, WARPS * 32>(vq, *reinterpret_cast<float(*)[D]>(smem_raw), blockIdx.x - row_ctas, bh);
     pdl_trigger();
     return;
   }

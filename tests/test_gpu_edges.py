@@ -1,5 +1,8 @@
 """Sizes at which the selection and the fused preparation change shape: edges of their tiles and groups, the smallest and
 largest member of each dispatch, against the oracle or the path that the other tests compare with it."""
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -107,3 +110,26 @@ def test_selection_of_rows_without_defined_probabilities(dtype, causal, value):
         assert torch.equal(mask.cpu().bool(), want)
         lut_o, valid_o = O.block_map_to_lut(want)
         assert torch.equal(lut.cpu(), lut_o) and torch.equal(valid.cpu(), valid_o)
+
+
+def _in_new_process(call):
+    """Kernel attributes outlive a call: what a launch needs shows only where no larger one came before it."""
+    r = subprocess.run([sys.executable, "-c", f"import sys; sys.path[:0] = {sys.path!r}; import test_gpu_edges as t; t.{call}"],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+
+
+def _check_cdf_selection(BH, nq, nk):
+    from spargeattn_b200 import ops
+    pq, pk, sim_q, sim_k = _pooled(BH, nq, nk, 64, torch.float16, nk)
+    knob = torch.full((BH,), 0.9)
+    want = O.select_blocks(O.pooled_probs(pq, pk, sim_k, False), sim_q, sim_k, None, knob, False, False)
+    dev = [t.cuda() for t in (pq, pk, sim_q.to(torch.uint8), sim_k.to(torch.uint8))]
+    assert torch.equal(ops.select_blocks(*dev, None, knob.cuda(), False, False, True)[2].cpu().bool(), want)
+
+
+# four rows take exactly 48 KB of dynamic shared memory from 1 281 to 1 408 blocks (with the scan's chunk, which follows the
+# number of rows), the first size above it is 1 409
+@pytest.mark.parametrize("BH,nq,nk", [(2, 64, 1281), (2, 64, 1408), (2, 64, 1409), (1, 600, 1345), (3, 700, 1377)])
+def test_cdf_selection_where_dynamic_shared_memory_reaches_48_kb(BH, nq, nk):
+    _in_new_process(f"_check_cdf_selection({BH}, {nq}, {nk})")
