@@ -525,13 +525,14 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
 }
 
 // One CTA per mask row: compaction of a user block mask into the LUT.
-// dynamic smem: int idx[nk]
+// dynamic smem: int per warp, int idx[nk]
+constexpr int kMaskWarps = kSelThreads / 32;
 __global__ void __launch_bounds__(kSelThreads) mask_to_lut_kernel(const uint8_t* __restrict__ mask, int elem_size,
                                                                   int32_t* __restrict__ lut, int32_t* __restrict__ valid,
                                                                   int nk) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  int* s_idx = reinterpret_cast<int*>(smem_raw);
-  __shared__ int s_warp[kSelThreads / 32];
+  int* s_warp = reinterpret_cast<int*>(smem_raw);   // not static: that would count against the 48 KB of the launch too
+  int* s_idx = s_warp + kMaskWarps;
   const size_t row = blockIdx.x;
   const uint8_t* mrow = mask + row * (size_t)nk * elem_size;
   int live_seen = 0;
@@ -601,8 +602,8 @@ int select_launch(const SelectArgs& a, cudaStream_t st) {
 
 int mask_to_lut_launch(const void* mask, int elem_size, int32_t* lut, int32_t* valid, long long rows, int nk, bool dependent,
                        cudaStream_t st) {
-  const size_t smem = (size_t)nk * sizeof(int);
-  if (smem > 200 * 1024 || rows > 2147483647LL) return SPARGE_ERR_TOO_LARGE;
+  if (nk > 50 * 1024 || rows > 2147483647LL) return SPARGE_ERR_TOO_LARGE;
+  const size_t smem = ((size_t)kMaskWarps + nk) * sizeof(int);
   if (smem > 48 * 1024) {
     if (cudaFuncSetAttribute(mask_to_lut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return SPARGE_ERR_CUDA;

@@ -133,3 +133,17 @@ def _check_cdf_selection(BH, nq, nk):
 @pytest.mark.parametrize("BH,nq,nk", [(2, 64, 1281), (2, 64, 1408), (2, 64, 1409), (1, 600, 1345), (3, 700, 1377)])
 def test_cdf_selection_where_dynamic_shared_memory_reaches_48_kb(BH, nq, nk):
     _in_new_process(f"_check_cdf_selection({BH}, {nq}, {nk})")
+
+
+def _check_mask_to_lut(nk):
+    from spargeattn_b200 import ops
+    m = torch.rand(1, 1, 2, nk, generator=torch.Generator().manual_seed(nk)) < 0.5
+    lut, valid = ops.mask_to_lut(m.cuda())
+    lut_o, valid_o = O.block_map_to_lut(m)
+    assert torch.equal(lut.cpu(), lut_o) and torch.equal(valid.cpu(), valid_o)
+
+
+# around the 48 KB that a launch may ask for without the attribute, and the longest row
+@pytest.mark.parametrize("nk", [12280, 12281, 12288, 12289, 51200])
+def test_block_mask_rows_where_dynamic_shared_memory_reaches_48_kb(nk):
+    _in_new_process(f"_check_mask_to_lut({nk})")
