@@ -28,23 +28,15 @@ SAGE2_TOKEN_LEVEL_CAUSAL = False
 SAGE1_FP16_PV = True
 
 
-_knob_cache = {}
-
-
 def hyperparameter_check(hyper, H, device):
     """spas_sage_attn/utils.py:38-50. Scalar knobs are materialised once per (value, H, device) and reused:
-    the tensors are read-only inputs of the kernels, and small calls are otherwise launch-bound."""
+    the tensors are read-only inputs of the kernels, and small calls are otherwise launch-bound. The first use of a
+    knob value should precede graph capture: it is a blocking copy from the host."""
     if type(hyper) == float or type(hyper) == int:
-        key = (float(hyper), H, str(device))
-        cached = _knob_cache.get(key)
-        if cached is None:
-            # built on the host and copied with a blocking transfer: the cached tensor is complete before any
-            # stream can read it (a fill kernel queued on the stream of the first caller would not be ordered
-            # with later callers on other streams). The first use of a knob value should precede graph capture.
-            cached = torch.full((H,), float(hyper), dtype=torch.float32).to(device)
-            if len(_knob_cache) < 256:
-                _knob_cache[key] = cached
-        return cached
+        dev = torch.device(device)
+        if dev.type != "cuda":
+            return torch.full((H,), float(hyper), dtype=torch.float32).to(dev)
+        return _binding.knob_tensor(float(hyper), H, torch.cuda.current_device() if dev.index is None else dev.index)
     elif isinstance(hyper, torch.Tensor):
         assert len(hyper.shape) <= 1, "Hyperparameter tensor must be 1D"
         if len(hyper.shape) == 0:

@@ -30,20 +30,23 @@ namespace {
 
 using at::Tensor;
 
-// Scalar knobs as [H] tensors, materialised once per (value, H, device): built on the host and copied with a blocking
+// Scalar knobs as [H] tensors, materialised once per (value, H, device) for every caller, Python's general path included:
+// a value that one entry has seen can be captured into a graph by another. Built on the host and copied with a blocking
 // transfer, so that a cached tensor is complete before any stream can read it.
-const float* knob_pointer(double value, int64_t H, c10::Device dev, Tensor& keep) {
+Tensor knob_tensor(double value, int64_t H, c10::Device dev) {
   static std::mutex mu;
-  static auto* cache = new std::map<std::tuple<float, int64_t, int>, Tensor>();   // never destroyed: CUDA may be gone at exit
-  const auto key = std::make_tuple((float)value, H, (int)dev.index());
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache->find(key);
-  if (it == cache->end()) {
-    keep = at::full({H}, (float)value, at::TensorOptions().dtype(at::kFloat)).to(dev);
-    if (cache->size() >= 256) return keep.data_ptr<float>();
-    it = cache->emplace(key, keep).first;
+  static auto* cache = new std::map<std::tuple<double, int64_t, int>, Tensor>();   // never destroyed: CUDA may be gone at exit
+  const auto key = std::make_tuple(value, H, (int)dev.index());
+  const bool cacheable = !std::isnan(value);                 // NaN has no place in an ordered map
+  if (cacheable) {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache->find(key);
+    if (it != cache->end()) return it->second;
   }
-  return it->second.data_ptr<float>();
+  Tensor t = at::full({H}, value, at::TensorOptions().dtype(at::kFloat)).to(dev);   // may run Python: not under the lock
+  std::lock_guard<std::mutex> lock(mu);
+  if (!cacheable || cache->size() >= 256) return t;
+  return cache->emplace(key, t).first->second;
 }
 
 // A knob argument: None -> null, number or ready tensor -> pointer; false: not one of these.
@@ -56,7 +59,8 @@ bool knob(PyObject* o, int64_t H, c10::Device dev, const float** out, Tensor& ke
       PyErr_Clear();
       return false;
     }
-    *out = knob_pointer(v, H, dev, keep);
+    keep = knob_tensor(v, H, dev);
+    *out = keep.data_ptr<float>();
     return true;
   }
   if (!THPVariable_Check(o)) return false;
@@ -79,6 +83,19 @@ bool view_strides(const Tensor& t, bool nhd, long long* st) {
 }
 
 Tensor* status_words[64];   // kept for the life of the process: kernels write to them
+
+PyObject* py_knob_tensor(PyObject*, PyObject* const* args, Py_ssize_t nargs) {   // (value, H, device index) -> [H] fp32
+  HANDLE_TH_ERRORS
+  if (nargs != 3) {
+    PyErr_SetString(PyExc_TypeError, "knob_tensor takes 3 arguments");
+    return nullptr;
+  }
+  const double value = PyFloat_AsDouble(args[0]);
+  const long H = PyLong_AsLong(args[1]), index = PyLong_AsLong(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  return THPVariable_Wrap(knob_tensor(value, H, c10::Device(c10::kCUDA, (c10::DeviceIndex)index)));
+  END_HANDLE_TH_ERRORS
+}
 
 PyObject* set_status_word(PyObject*, PyObject* o) {   // the int32 word of its device that expired waits are written to
   if (!THPVariable_Check(o) || THPVariable_Unpack(o).get_device() < 0 || THPVariable_Unpack(o).get_device() >= 64) {
@@ -190,6 +207,8 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 PyMethodDef kMethods[] = {
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(forward)), METH_FASTCALL,
      "The whole path in one call; None for arguments that are left to the caller."},
+    {"knob_tensor", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_knob_tensor)), METH_FASTCALL,
+     "A scalar knob as an [H] tensor on a CUDA device, materialised once."},
     {"set_status_word", set_status_word, METH_O, "Registers the device status word of a CUDA device."},
     {nullptr, nullptr, 0, nullptr}};
 

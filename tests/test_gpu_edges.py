@@ -147,3 +147,28 @@ def _check_mask_to_lut(nk):
 @pytest.mark.parametrize("nk", [12280, 12281, 12288, 12289, 51200])
 def test_block_mask_rows_where_dynamic_shared_memory_reaches_48_kb(nk):
     _in_new_process(f"_check_mask_to_lut({nk})")
+
+
+def _check_capture_with_a_known_knob():
+    import spargeattn_b200 as S
+    g = torch.Generator().manual_seed(5)
+    q, k, v = (torch.randn(1, 2, 512, 64, generator=g).bfloat16().cuda() for _ in range(3))
+    S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=0.5)
+    want, _ = S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=0.4375, return_sparsity=True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o = S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=0.4375)
+    graph.replay()
+    assert torch.equal(o, want)
+
+
+def test_a_knob_that_one_entry_has_seen_can_be_captured_by_another():
+    _in_new_process("_check_capture_with_a_known_knob()")
+
+
+def test_a_knob_beyond_fp32_is_refused():
+    import spargeattn_b200 as S
+    q = torch.randn(1, 2, 256, 64).bfloat16().cuda()
+    for kw in ({"topk": 1e300}, {"topk": 1e300, "return_sparsity": True}, {"pvthreshd": -1e300}):
+        with pytest.raises(RuntimeError):
+            S.spas_sage2_attn_meansim_topk_cuda(q, q, q, **kw)
