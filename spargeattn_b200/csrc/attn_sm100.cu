@@ -179,11 +179,10 @@ constexpr int kAttnThreads = 192;
 template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16 = false>
 __global__ void __launch_bounds__(kAttnThreads, (AttnShape<D, PVF16>::kCtasPerSm))
 attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-            const __grid_constant__ CUtensorMap tmap_v, OutT* __restrict__ o, const int32_t* __restrict__ lut,
-            const int32_t* __restrict__ valid, const float* __restrict__ pvthr, const float* __restrict__ q_scale,
-            const float* __restrict__ k_scale, const float* __restrict__ v_scale, int32_t* dev_status, int N, int H,
-            int nq, int nk, float sm_scale_log2, long long osb, long long osh, long long osn,
-            int32_t* __restrict__ pv_count, const int32_t* __restrict__ q_ranges) {
+            const __grid_constant__ CUtensorMap tmap_v, OutT* __restrict__ o, const int32_t* lut, const int32_t* valid,
+            const float* pvthr, const float* q_scale, const float* k_scale, const float* v_scale, int32_t* dev_status, int N,
+            int H, int nq, int nk, float sm_scale_log2, long long osb, long long osh, long long osn,
+            int32_t* __restrict__ pv_count, const int32_t* q_ranges) {
   using Shape = AttnShape<D, PVF16>;
   constexpr bool PV_SKIP = PV_MODE != 0, pv_per_warp = PV_MODE == 2, GRAN3 = GRAN == 3;
   constexpr int SK = Shape::kStagesK, NV = Shape::kSlotsV;

@@ -122,8 +122,7 @@ __global__ void __launch_bounds__(1024) prep_combine_kernel(PrepScratch s, int s
 // what the first kernel read last is still in L2.
 template <typename T, int D, bool SMOOTH_K, bool WANT_POOL>
 __global__ void __launch_bounds__(kPassThreads, 3)
-prep_second_kernel(const __grid_constant__ PrepArgs a, const __grid_constant__ VQuantArgs vq, const double* __restrict__ kp, int parts,
-                   int spans) {
+prep_second_kernel(const __grid_constant__ PrepArgs a, const __grid_constant__ VQuantArgs vq, const double* kp, int parts, int spans) {
   using Shape = PrepShape<D>;
   constexpr int KU = Shape::kKUnits;
   __shared__ PoolQuantShared<D, 64, Shape::kKBlocks, WANT_POOL> sm;

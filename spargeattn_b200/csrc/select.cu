@@ -253,8 +253,7 @@ __device__ __forceinline__ void scan_chunks_wide(const uint16_t* sorted, uint16_
 
 template <typename T, int D, int RW, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t* __restrict__ sim_q,
-              const uint8_t* __restrict__ sim_k, const float* __restrict__ topk, const float* __restrict__ cdfthr,
+select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim_k, const float* topk, const float* cdfthr,
               uint8_t* __restrict__ mask, int32_t* __restrict__ lut, int32_t* __restrict__ valid, int H, int nq, int nk,
               int is_causal, int sink, int best_first, int scan_log_nx, int cdf_len, const __grid_constant__ VQuantArgs vq, int row_ctas) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -527,9 +526,8 @@ select_kernel(const T* __restrict__ pq, const T* __restrict__ pk, const uint8_t*
 // One CTA per mask row: compaction of a user block mask into the LUT.
 // dynamic smem: int per warp, int idx[nk]
 constexpr int kMaskWarps = kSelThreads / 32;
-__global__ void __launch_bounds__(kSelThreads) mask_to_lut_kernel(const uint8_t* __restrict__ mask, int elem_size,
-                                                                  int32_t* __restrict__ lut, int32_t* __restrict__ valid,
-                                                                  int nk) {
+__global__ void __launch_bounds__(kSelThreads) mask_to_lut_kernel(const uint8_t* mask, int elem_size, int32_t* __restrict__ lut,
+                                                                  int32_t* __restrict__ valid, int nk) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int* s_warp = reinterpret_cast<int*>(smem_raw);   // not static: that would count against the 48 KB of the launch too
   int* s_idx = s_warp + kMaskWarps;
