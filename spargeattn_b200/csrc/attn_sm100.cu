@@ -31,6 +31,7 @@
 #include "attn.cuh"
 #include "launch.cuh"
 #include "sm100_ptx.cuh"
+#include "step_word.cuh"
 
 namespace sparge {
 
@@ -353,9 +354,9 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       }
       if (lane == 0) {
         if (s + 1 < nsteps) {
-          // the top bit marks a block whose keys need masks; a second block that there is not has it too
-          auto marked = [&](int j) { return ((j * 64 + 64 > N) || (CAUSAL && (j * 64 + 63 > qi * 128))) ? j | INT_MIN : j; };
-          load_k(s + 1, na, nb, make_int4(marked(na), nb < 0 ? INT_MIN : marked(nb), __float_as_int(ka), __float_as_int(kb)));
+          // a second block that there is not counts as masked
+          auto word = [&](int j) { return step_word(j, (j * 64 + 64 > N) || (CAUSAL && (j * 64 + 63 > qi * 128))); };
+          load_k(s + 1, na, nb, make_int4(word(na), nb < 0 ? step_word(0, true) : word(nb), __float_as_int(ka), __float_as_int(kb)));
         }
         if (ok && s >= 0) load_v(2 * s, ja);
         if (ok && s >= 0 && jb >= 0) load_v(2 * s + 1, jb);
@@ -500,16 +501,16 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       const bool two = cnt - 2 * s >= 2;                          // the last step of an odd count has one block
       // Key masks, or one block only: the general path for both blocks. One test, made while the scores travel, keeps the
       // ordinary step free of branches (with a test per block after the load: 2.44 instead of 2.33 ms at [1,12,32760,128]).
-      const bool plain = !GRAN3 && __all_sync(0xffffffffu, (mt.x | mt.y) >= 0);
+      const bool plain = !GRAN3 && __all_sync(0xffffffffu, !step_masked(mt.x | mt.y));
       float cc[2][4];   // scale of each block's scores (per-thread granularity: of each pair of key columns)
       int klim[2] = {64, 64};   // keys with block-local index >= klim are masked
 #pragma unroll
       for (int b = 0; b < 2; b++) {
         cc[b][0] = cc[b][1] = cc[b][2] = cc[b][3] = qs * __int_as_float(b ? mt.w : mt.z);
         if (!plain) {
-          const int j = (b ? mt.y : mt.x) & INT_MAX, key0 = j * 64;
+          const int word = b ? mt.y : mt.x, key0 = step_index(word) * 64;
           if (GRAN3) {
-            const float4 k4 = *reinterpret_cast<const float4*>(ks_row + (size_t)j * 4);
+            const float4 k4 = *reinterpret_cast<const float4*>(ks_row + (size_t)step_block(word, nk) * 4);
             cc[b][0] = qs * k4.x; cc[b][1] = qs * k4.y; cc[b][2] = qs * k4.z; cc[b][3] = qs * k4.w;
           }
           klim[b] = min(64, N - key0);

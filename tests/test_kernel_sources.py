@@ -1,6 +1,10 @@
 """CPU checks of rules that the kernels' sources have to keep and that no run can show."""
 import os
 import re
+import shutil
+import subprocess
+
+import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "spargeattn_b200", "csrc")
 
@@ -24,3 +28,35 @@ def test_kernels_that_wait_for_the_one_before_do_not_claim_constant_inputs():
     for name, parameters, _ in kernels:
         for parameter in parameters.split(","):
             assert not ("const" in parameter and "__restrict__" in parameter), (name, parameter)
+
+
+def test_any_step_word_names_a_block_of_the_row(tmp_path):
+    """The softmax warps go on after an expired wait, on whatever the word in shared memory then holds."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no g++")
+    src = tmp_path / "words.cpp"
+    src.write_text('''
+#include <initializer_list>
+#include "step_word.cuh"
+int main() {
+  using namespace sparge;
+  for (int nk : {1, 2, 63, 1861, 65535}) {
+    for (unsigned w = 0; w < 1u << 16; w++)
+      for (unsigned hi : {0u, 0x8000u, 0x7fffu, 0xffffu, 0x1234u}) {
+        const int j = step_block((int)(hi << 16 | w), nk);
+        if (j < 0 || j >= nk) return 1;
+      }
+    for (int j = 0; j < nk; j++)
+      for (bool m : {false, true})
+        if (step_block(step_word(j, m), nk) != j || step_masked(step_word(j, m)) != m) return 2;
+  }
+  return 0;
+}
+''')
+    subprocess.run([gxx, "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(tmp_path / "words")], check=True)
+    assert subprocess.run([str(tmp_path / "words")]).returncode == 0
+    # every load that takes the word is through step_block; step_index feeds the key masks
+    text = open(os.path.join(CSRC, "attn_sm100.cu")).read()
+    assert re.findall(r"(\S+) step_index\(word\) \* 64;", text) == ["="] and text.count("step_index(") == 1
+    assert text.count("(size_t)step_block(word, nk)") == text.count("step_block(") == 1
