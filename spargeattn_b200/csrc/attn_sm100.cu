@@ -214,7 +214,10 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   const int bh = blockIdx.y, h = bh % H;
   const int q_begin = q_ranges ? q_ranges[2 * bh] : 0;
   const int q_count = q_ranges ? min(q_ranges[2 * bh + 1], nq - q_begin) : (int)gridDim.x;
-  if ((int)blockIdx.x >= q_count) return;
+  if ((int)blockIdx.x >= q_count) {
+    pdl_wait();   // when every CTA leaves here, this kernel must still not end before the ones that it depends on
+    return;
+  }
   const int qi = q_begin + q_count - 1 - (int)blockIdx.x;
   const size_t row_id = (size_t)bh * nq + qi;
 

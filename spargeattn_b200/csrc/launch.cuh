@@ -4,6 +4,8 @@
 // completed and their writes are visible), pdl_trigger() lets the next one be scheduled. The trigger stands at a kernel's
 // end: given at its start, blocks of the next kernel sat in slots that the current one still needed (a [1,24,4608,128]
 // call took 207 us, 195 without dependent launches, 188 like this). Without the launch attribute both are no-ops.
+// No block leaves a kernel in front of pdl_wait() by a return: if all of them did, the kernel would end before the one it
+// depends on, and what follows on the stream (the next user of the workspace) waits for this one only.
 // A kernel with a pdl_wait() takes no `const T* __restrict__`: that promises data which nothing writes while the kernel runs,
 // so that loads may go through the non-coherent path and in front of the wait, and the kernel before it still writes.
 #pragma once

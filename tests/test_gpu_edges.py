@@ -172,3 +172,16 @@ def test_a_knob_beyond_fp32_is_refused():
     for kw in ({"topk": 1e300}, {"topk": 1e300, "return_sparsity": True}, {"pvthreshd": -1e300}):
         with pytest.raises(RuntimeError):
             S.spas_sage2_attn_meansim_topk_cuda(q, q, q, **kw)
+
+
+def test_a_share_without_query_blocks_leaves_the_output_alone():
+    """Every CTA of the attention kernel leaves at once; what follows on the stream reuses the call's workspace."""
+    from spargeattn_b200.sharding import attention_units
+    import spargeattn_b200 as S
+    g = torch.Generator().manual_seed(6)
+    q, k, v = (torch.randn(1, 2, 2304, 128, generator=g).bfloat16().cuda() for _ in range(3))
+    want = S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=0.5)
+    none = torch.zeros(1, 2, 2, dtype=torch.int32, device="cuda")
+    for _ in range(20):
+        attention_units(q, k, v, none, 1, topk=0.5)
+        assert torch.equal(S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=0.5), want)

@@ -30,6 +30,11 @@ def test_kernels_that_wait_for_the_one_before_do_not_claim_constant_inputs():
             assert not ("const" in parameter and "__restrict__" in parameter), (name, parameter)
 
 
+def test_no_block_returns_before_it_has_waited():
+    for name, _, body in _waiting_kernels():
+        assert not re.search(r"\breturn;", body[:body.index("pdl_wait")]), name
+
+
 def test_any_step_word_names_a_block_of_the_row(tmp_path):
     """The softmax warps go on after an expired wait, on whatever the word in shared memory then holds."""
     gxx = shutil.which("g++")
