@@ -1,5 +1,6 @@
 """Sizes at which the selection and the fused preparation change shape: edges of their tiles and groups, the smallest and
 largest member of each dispatch, against the oracle or the path that the other tests compare with it."""
+import ctypes
 import subprocess
 import sys
 
@@ -185,3 +186,25 @@ def test_a_share_without_query_blocks_leaves_the_output_alone():
     for _ in range(20):
         attention_units(q, k, v, none, 1, topk=0.5)
         assert torch.equal(S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=0.5), want)
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+    """Launches into a capture that has been invalidated are refused by the runtime: the call says so, and the thread's last
+    error, which the next check of anybody's launch would report, stays clear."""
+    from spargeattn_b200 import _cabi, ops
+    rt = ctypes.CDLL("libcudart.so.12")
+    mask = torch.ones(1, 1, 2, 4, dtype=torch.uint8, device="cuda")
+    lut, valid = torch.empty(1, 1, 2, 4, dtype=torch.int32, device="cuda"), torch.empty(1, 1, 2, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(ctypes.byref(stream), 1) == 0
+    assert rt.cudaStreamBeginCapture(stream, 2) == 0                     # relaxed: nothing else of the process is held up
+    assert rt.cudaStreamSynchronize(stream) != 0                         # not allowed in a capture: invalidates it
+    rt.cudaGetLastError()
+    status = _cabi.lib.sparge_mask_to_lut(mask.data_ptr(), 1, lut.data_ptr(), valid.data_ptr(), 1, 1, 2, 4, stream)
+    left = rt.cudaGetLastError()
+    rt.cudaStreamEndCapture(stream, ctypes.byref(graph))
+    rt.cudaGetLastError()
+    assert rt.cudaStreamDestroy(stream) == 0
+    assert status == _cabi.ERR_CUDA and left == 0
+    assert ops.mask_to_lut(mask)[1].tolist() == [[[4, 4]]]
