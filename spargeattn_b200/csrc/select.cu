@@ -29,6 +29,13 @@ namespace sparge {
 
 constexpr int kSelThreads = 256;
 
+// The attribute is always set to what an SM gives a block, never to what one launch needs: it is the kernel's, and a thread
+// with a shorter row would lower it between another thread's attribute and launch.
+template <typename K>
+static bool allow_dynamic_smem(K kernel, size_t smem) {
+  return smem <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
+}
+
 // Exclusive prefix count of `flag` over the CTA's threads in thread order, plus CTA total.
 // s_warp must hold kSelThreads/32 ints. Contains two __syncthreads.
 __device__ __forceinline__ int block_exclusive_count(bool flag, int* s_warp, int& total) {
@@ -569,8 +576,7 @@ static int launch_select(const SelectArgs& a, cudaStream_t st) {
   const size_t smem = kSelTileKeys * (D * sizeof(T) + 16) + (size_t)WARPS * RW * select_row(a.nk, D, cdf_len).total();
   if (smem > 200 * 1024) return SPARGE_ERR_TOO_LARGE;
   auto kern = select_kernel<T, D, RW, WARPS>;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return SPARGE_ERR_CUDA;
+  if (!allow_dynamic_smem(kern, smem)) return SPARGE_ERR_CUDA;
   const int row_ctas = (a.nq + WARPS * RW - 1) / (WARPS * RW);
   const cudaError_t e = launch(kern, dim3(row_ctas + (a.vq.v ? a.vq.spans : 0), a.BH), WARPS * 32, smem, st, a.dependent,
                                (const T*)a.pq, (const T*)a.pk, a.sim_q, a.sim_k, a.topk, a.cdf, a.mask, a.lut, a.valid, a.H, a.nq,
@@ -602,10 +608,7 @@ int mask_to_lut_launch(const void* mask, int elem_size, int32_t* lut, int32_t* v
                        cudaStream_t st) {
   if (nk > 50 * 1024 || rows > 2147483647LL) return SPARGE_ERR_TOO_LARGE;
   const size_t smem = ((size_t)kMaskWarps + nk) * sizeof(int);
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(mask_to_lut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return SPARGE_ERR_CUDA;
-  }
+  if (!allow_dynamic_smem(mask_to_lut_kernel, smem)) return SPARGE_ERR_CUDA;
   const cudaError_t e = launch(mask_to_lut_kernel, dim3((unsigned)rows), kSelThreads, smem, st, dependent, (const uint8_t*)mask,
                                elem_size, lut, valid, nk);
   return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;

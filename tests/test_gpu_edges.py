@@ -3,6 +3,7 @@ largest member of each dispatch, against the oracle or the path that the other t
 import ctypes
 import subprocess
 import sys
+import threading
 
 import pytest
 import torch
@@ -208,3 +209,28 @@ def test_a_refused_launch_leaves_no_error_behind():
     assert rt.cudaStreamDestroy(stream) == 0
     assert status == _cabi.ERR_CUDA and left == 0
     assert ops.mask_to_lut(mask)[1].tolist() == [[[4, 4]]]
+
+
+def test_rows_of_different_lengths_from_several_threads():
+    """The kernels' shared-memory attribute is common to all threads: a short row must not take a long one's away."""
+    from spargeattn_b200 import ops
+    problems = []
+
+    def run(nk):
+        try:
+            dev = [t.cuda() for t in _pooled(1, 4, nk, 128, torch.bfloat16, nk)]
+            dev[2:] = [t.to(torch.uint8) for t in dev[2:]]
+            knob, mask = torch.full((1,), 0.5).cuda(), torch.ones(1, 1, 1, nk + 12000, dtype=torch.uint8, device="cuda")
+            for _ in range(2000):
+                ops.select_blocks(*dev, knob, None, False, False)
+                ops.mask_to_lut(mask)
+        except Exception as e:
+            problems.append(e)
+
+    threads = [threading.Thread(target=run, args=(nk,)) for nk in (4000, 4600, 12000)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not problems
