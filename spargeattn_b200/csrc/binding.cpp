@@ -163,6 +163,7 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   a.sink = PyObject_IsTrue(args[11]), a.smooth_k = PyObject_IsTrue(args[12]);
   if (PyErr_Occurred()) return nullptr;
   if (args[15] != Py_None) {
+    if (!THPVariable_Check(args[15])) Py_RETURN_NONE;
     const Tensor& r = THPVariable_Unpack(args[15]);
     if (r.scalar_type() != at::kInt || r.numel() != 2 * B * H || !r.is_contiguous() || r.device() != dev) Py_RETURN_NONE;
     a.q_ranges = r.data_ptr<int32_t>();

@@ -234,3 +234,18 @@ def test_rows_of_different_lengths_from_several_threads():
         t.join()
     torch.cuda.synchronize()
     assert not problems
+
+
+@pytest.mark.parametrize("ranges", [[0, 1, 0, 1], "0101", torch.zeros(1, 2, 2), torch.zeros(1, 2, 2, dtype=torch.int32), None])
+def test_row_ranges_that_are_no_device_tensor(ranges):
+    """What the binding cannot take it leaves to the general path, which complains; without ranges it takes the call."""
+    from spargeattn_b200 import core
+    q = torch.randn(1, 2, 256, 64).bfloat16().cuda()
+    args = (False, None, True, -0.1, None, 0.5, 50, False, "HND", False, False)
+    r = core._binding.forward(q, q, q, None, -0.1, None, 0.5, 50, None, False, False, False, True, False, "HND", ranges, 1, False)
+    if ranges is None:
+        assert torch.equal(r, core._meansim_attention(q, q, q, *args))
+    else:
+        assert r is None
+        with pytest.raises((AttributeError, AssertionError, RuntimeError)):
+            core._meansim_attention(q, q, q, *args, q_block_ranges=ranges, q_blocks_max=1)
