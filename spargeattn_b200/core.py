@@ -298,9 +298,10 @@ def spas_sage2_attn_meansim_topk_cuda(q, k, v, attn_mask=None, dropout_p=0.0, is
 def _block_sparse_general(q, k, v, mask_id, scale, smooth_k, pvthreshd, tensor_layout, return_sparsity):
     q, k, v = _prologue(q, k, v, tensor_layout)
     headdim = q.size(-1)
+    if headdim not in [64, 128]:                          # before the mask is looked at, and as the quantisers say it
+        raise ValueError("headdim should be in [64, 128]. For other headdim, you can use padding and specify the softmax scale.")
     assert mask_id is not None, "mask_id is required"
     assert mask_id.dim() == 4 and mask_id.is_contiguous()
-    assert headdim in [64, 128], "headdim should be in [64, 128]. For other headdim, you can use padding and specify the softmax scale."
     if mask_id.dtype.is_floating_point:
         mask_id = mask_id != 0                            # -0.0 must count as false
     pvthreshd = _pv_threshold_tensor(pvthreshd, q.size(-3), q.device)

@@ -249,3 +249,15 @@ def test_row_ranges_that_are_no_device_tensor(ranges):
         assert r is None
         with pytest.raises((AttributeError, AssertionError, RuntimeError)):
             core._meansim_attention(q, q, q, *args, q_block_ranges=ranges, q_blocks_max=1)
+
+
+def test_block_mask_entry_refuses_other_head_sizes_with_a_value_error():
+    import spargeattn_b200 as S
+    q, ok = (torch.randn(1, 2, 256, d).bfloat16().cuda() for d in (96, 64))
+    mask = torch.ones(1, 2, 2, 4, dtype=torch.bool, device="cuda")
+    for kw in ({"mask_id": mask}, {"mask_id": mask, "smooth_k": False}, {"mask_id": None}, {"mask_id": mask, "return_sparsity": True}):
+        with pytest.raises(ValueError):
+            S.block_sparse_sage2_attn_cuda(q, q, q, **kw)
+    for mask_id in (None, mask[0], mask.transpose(2, 3)):
+        with pytest.raises(AssertionError):
+            S.block_sparse_sage2_attn_cuda(ok, ok, ok, mask_id=mask_id)
