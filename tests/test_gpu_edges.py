@@ -261,3 +261,50 @@ def test_block_mask_entry_refuses_other_head_sizes_with_a_value_error():
     for mask_id in (None, mask[0], mask.transpose(2, 3)):
         with pytest.raises(AssertionError):
             S.block_sparse_sage2_attn_cuda(ok, ok, ok, mask_id=mask_id)
+
+
+@pytest.mark.parametrize("kw", [dict(topk=0.4), dict(topk=0.4, pvthreshd=4.0, is_causal=True), dict(cdfthreshd=0.9, simthreshd1=0.3),
+                                dict(cdfthreshd=0.8, pvthreshd=4.0, attention_sink=True, smooth_k=False)])
+@pytest.mark.parametrize("N,D,dtype,v_dtype", [(1000, 64, torch.bfloat16, torch.float16), (2048, 128, torch.float16, torch.float16),
+                                               (2500, 128, torch.bfloat16, torch.bfloat16)])
+def test_c_entry_of_the_whole_path(kw, N, D, dtype, v_dtype):
+    """The C signature: its strides, the parts at the reported offsets, a workspace of exactly the reported size."""
+    import spargeattn_b200 as S
+    from spargeattn_b200 import _cabi, core, ops
+    B, H = 2, 3
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(B, N, H, D, generator=g).to(t).cuda().transpose(1, 2) for t in (dtype, dtype, v_dtype))   # token-major
+    causal, sink, smooth = kw.get("is_causal", False), kw.get("attention_sink", False), kw.get("smooth_k", True)
+    fn = S.spas_sage2_attn_meansim_topk_cuda if "topk" in kw else S.spas_sage2_attn_meansim_cuda
+    want = fn(q, k, v, **{"simthreshd1": -0.1, **kw})
+    vec = lambda name, default=None: None if kw.get(name, default) is None else torch.full((H,), kw.get(name, default), device="cuda")
+    thr, cdf, topk, pv = vec("simthreshd1", -0.1), vec("cdfthreshd"), vec("topk"), vec("pvthreshd")
+    o, ws, at = ops.meansim_forward(q, k, v, torch.empty(B, H, N, D, dtype=dtype, device="cuda"), thr, cdf, topk, pv, D ** -0.5, causal,
+                                    False, sink, smooth)
+    assert torch.equal(o, want)
+    # the parts, against the separate entries
+    km = ops.k_mean(k) if smooth else None
+    pq, sq, q8, qs = ops.pool_sim_quant(q, None, 128, thr)
+    pk, sk, k8, ks = ops.pool_sim_quant(k, km, 64, thr)
+    lut, valid, _ = ops.select_blocks(pq, pk, sq, sk, topk, cdf, causal, sink, best_first=pv is None)
+    v8, vs = ops.quant_v(v)
+    parts = dict(pq=pq, pk=pk, sim_q=sq, sim_k=sk, q_int8=q8, k_int8=k8, q_scale=qs, k_scale=ks, lut=lut, valid=valid, v8=v8, v_scale=vs)
+    if smooth:
+        parts["km"] = km
+    assert set(ops.WS_PARTS) == set(parts) | {"scratch", "km"}
+    for name, t in parts.items():
+        assert torch.equal(ws[at[name]:at[name] + t.numel() * t.element_size()], t.contiguous().view(-1).view(torch.uint8)), name
+    # one byte short is refused, exactly enough does not touch what lies behind
+    nbytes = int(_cabi.lib.sparge_forward_workspace_bytes(B, H, N, D))
+    guarded, out = torch.full((nbytes + 4096,), 0x5a, dtype=torch.uint8, device="cuda"), torch.empty_like(q)
+    st3 = lambda t: (ctypes.c_longlong * 3)(*t.stride()[:3])
+    ptr = lambda t: None if t is None else t.data_ptr()
+    call = lambda n: _cabi.lib.sparge_meansim_forward(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), ptr(thr), ptr(cdf), ptr(topk), ptr(pv), guarded.data_ptr(), n, None, B, H,
+        N, D, ops._dt(q), ops._dt(v), int(causal), 0, int(sink), int(smooth), D ** -0.5, st3(q), st3(k), st3(v), st3(out), None)
+    torch.cuda.synchronize()
+    assert call(nbytes - 1) == _cabi.ERR_INVALID_ARG
+    assert call(nbytes) == _cabi.OK
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and bool((guarded[nbytes:] == 0x5a).all())
+    ops.check_device_status()
