@@ -178,8 +178,9 @@ def test_host_front_end_matches_device_call():
 
 
 def test_concurrent_preparation_gives_the_same_bytes():
-    """Mid-sized calls run Q pooling and the V quantiser on side streams beside the K chain: same bytes as the
-    one-stream order, also when calls follow each other on different streams."""
+    """The entry-by-entry path (what a call takes whose arguments the native call leaves to it) runs Q pooling and the V
+    quantiser on side streams beside the K chain for mid-sized problems: same bytes as the one-stream order, also when
+    calls follow each other on different streams."""
     import spargeattn_b200 as S
     from spargeattn_b200 import core
     B, H, N, D = 1, 2, 3000, 128
@@ -211,8 +212,8 @@ def test_concurrent_preparation_gives_the_same_bytes():
                                 dict(topk=0.4, tensor_layout="NHD")])
 @pytest.mark.parametrize("shape,dtype", [((2, 3, 1100, 64), torch.bfloat16), ((1, 2, 2048, 128), torch.float16)])
 def test_single_call_path_equals_the_entry_by_entry_path(kw, shape, dtype):
-    """Small problems are issued by one C call (sparge_meansim_forward) instead of nine wrappers: the same kernels in
-    the same order on the same stream, so the bytes are the same, for every knob, with and without return_sparsity."""
+    """The native one-call path (fused preparation, four or five launches) against the separate entries: the same arithmetic,
+    so the bytes are the same, for every knob, with and without return_sparsity."""
     import spargeattn_b200 as S
     from spargeattn_b200 import core
     B, H, N, D = shape
