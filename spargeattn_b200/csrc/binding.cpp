@@ -168,6 +168,8 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (r.scalar_type() != at::kInt || r.numel() != 2 * B * H || !r.is_contiguous() || r.device() != dev) Py_RETURN_NONE;
     a.q_ranges = r.data_ptr<int32_t>();
     a.q_blocks_max = (int)PyLong_AsLong(args[16]);
+    if (PyErr_Occurred()) return nullptr;
+    if (a.q_blocks_max <= 0) Py_RETURN_NONE;
   }
 
   c10::cuda::set_device(dev.index());

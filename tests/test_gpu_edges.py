@@ -308,3 +308,11 @@ def test_c_entry_of_the_whole_path(kw, N, D, dtype, v_dtype):
     torch.cuda.synchronize()
     assert torch.equal(out, want) and bool((guarded[nbytes:] == 0x5a).all())
     ops.check_device_status()
+
+
+def test_ranges_without_a_largest_count_are_an_assertion():
+    from spargeattn_b200.sharding import attention_units
+    q = torch.randn(1, 2, 256, 64).bfloat16().cuda()
+    for largest in (None, 0, -1):                          # None: read back from the ranges, which are empty
+        with pytest.raises(AssertionError):
+            attention_units(q, q, q, torch.zeros(1, 2, 2, dtype=torch.int32), largest, topk=0.5)
