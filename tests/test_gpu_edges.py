@@ -316,3 +316,27 @@ def test_ranges_without_a_largest_count_are_an_assertion():
     for largest in (None, 0, -1):                          # None: read back from the ranges, which are empty
         with pytest.raises(AssertionError):
             attention_units(q, q, q, torch.zeros(1, 2, 2, dtype=torch.int32), largest, topk=0.5)
+
+
+def test_native_calls_on_several_streams_and_threads():
+    """Each call takes its workspace and output on the stream it runs on; scalar knobs are shared."""
+    import spargeattn_b200 as S
+    g = torch.Generator().manual_seed(8)
+    x = [[torch.randn(1, 2, n, 128, generator=g).bfloat16().cuda() for _ in range(3)] for n in (700, 1500, 2600, 4000)]
+    call = lambda i, j: S.spas_sage2_attn_meansim_topk_cuda(*x[i], topk=0.3 + 0.01 * j, is_causal=j % 2 == 1)
+    want = [[call(i, j) for j in range(4)] for i in range(4)]
+    torch.cuda.synchronize()
+    got = [[] for _ in range(4)]
+
+    def run(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got[i] = [call((i + r) % 4, r % 4) for r in range(40)]
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(4):
+        assert len(got[i]) == 40 and all(torch.equal(o, want[(i + r) % 4][r % 4]) for r, o in enumerate(got[i]))
