@@ -22,7 +22,7 @@ from ._cabi import _binding
 SAGE2_TOKEN_LEVEL_CAUSAL = False
 
 # The Sage1-signature entry points of the reference (core.py:235-319) keep V in fp16 and run an fp16 P.V kernel.
-# True: they run the fp16-PV variant of the attention kernel here as well (about 1.2x the FP8 kernel's time);
+# True: they run the fp16-PV variant of the attention kernel here as well (1.2x the FP8 kernel's time at D = 128);
 # False: they share the FP8-PV kernel of the Sage2 entry points (faster; output within cosine 0.9996 but only
 # 1.4-2.4 % relative L1 of the reference's, because V and P are rounded to e4m3).
 SAGE1_FP16_PV = True
@@ -93,19 +93,18 @@ def _empty_like_layout(q):
 
 
 _SIDE_STREAMS = {}
-# The three preparation chains of a call (K mean -> K pooling / quantisation; Q pooling / quantisation; V quantiser)
-# are independent until the selection and the attention kernel. For a share of a few heads (what a rank owns under
-# row sharding on many GPUs) no single one of these kernels fills the GPU, and running the chains on three streams
-# shortens the call; for a whole multi-head problem every kernel fills all CTA slots by itself and the extra
-# streams only add event traffic (measured: 3.006 against 3.03 ms for 12 heads of 32 760 tokens, 56.4 against 55.6 ms
-# for 24 heads of 119 056), and a handful of short launches is bound by the host's launch rate, which events
-# worsen. Hence the window, in (batch * heads * tokens) rows.
+# Calls of fewer (batch * heads * tokens) rows than this are issued by one native call (forward.cu: four or five launches
+# on one workspace). That is all of them: it is faster at every size (0.067 -> 0.03 ms at [1, 4, 2048, 64]). The sequence of
+# separate entries gives the same bytes and takes what the native call leaves to it (a `scale` that is neither None nor a
+# Python number); 0 sends every call there.
+SINGLE_CALL_MAX_ROWS = 1 << 62
+# In that sequence the three preparation chains (K mean -> K pooling / quantisation; Q pooling / quantisation; V quantiser)
+# run on three streams for problems of this many (batch * heads * tokens) rows: they are independent until the selection,
+# and for a few heads none of their kernels fills the GPU (two heads of 32 760 tokens: 0.568 -> 0.543 ms). A larger problem
+# fills it with each kernel (12 heads: 3.006 against 3.03 ms; 24 of 119 056: 56.4 against 55.6 ms), a smaller one is bound
+# by the host, which events slow down.
 CONCURRENT_PREP_MIN_ROWS = 16384
 CONCURRENT_PREP_MAX_ROWS = 163840
-# Calls of fewer (batch * heads * tokens) rows than this are issued by one native call (forward.cu: four or five launches
-# on one workspace) -- all of them: it is faster at every size (0.067 -> 0.03 ms at [1, 4, 2048, 64]). The sequence of
-# separate entries below it gives the same bytes; it is what a caller composes who wants the intermediate tensors.
-SINGLE_CALL_MAX_ROWS = 1 << 62
 
 
 def _side_streams(device):

@@ -131,7 +131,7 @@ __device__ __forceinline__ void pack_p(uint32_t* w, float a, float b, float c, f
 // row's 16-byte chunks chunk0 ... of the 128B-swizzled tile. `prow` = shared address of the row, rsw = row & 7.
 // The scores are converted with the integer-to-float instruction: it is exact and runs at half rate beside the FMA
 // pipe's packed f32x2 work (adding a float bias as an integer multiply-add instead cost 3 % of the kernel).
-// EXACT: one factor per pair of key columns (c4, see block_rowmax_g; all equal for the coarser granularities) and a key
+// EXACT: one factor per pair of key columns (c4, see block_rowmax_masked; all equal for the coarser granularities) and a key
 // limit: keys >= klim get probability zero.
 template <bool EXACT, bool PVF16>
 __device__ __forceinline__ float block_exp(const uint32_t* sr, const float* c4, float m, int klim, uint32_t prow, int chunk0,
@@ -207,8 +207,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   // the shuffles let the compiler see that these are the same for the whole warp: branches on them need no convergence
   // bookkeeping and the operands of the MMA instructions can be kept in uniform registers
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  // Query blocks are issued last-first: under a causal mask the late rows hold the most live blocks,
-  // and starting the longest rows first keeps the final wave short.
+  // Query blocks are issued last-first: under a causal mask the late rows hold the most live blocks, and a head's longest
+  // rows start first. (Heads follow one another, so the last head's longest rows still start late.)
   // With q_ranges, (batch, head) bh computes only its query blocks [begin, begin + count): the unit of the
   // multi-GPU row sharding. The grid is sized for the largest count; the other CTAs leave at once.
   const int bh = blockIdx.y, h = bh % H;

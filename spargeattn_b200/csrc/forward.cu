@@ -66,8 +66,12 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
   p.v_mode = copy_v ? kVHalf : a.pv_fp16 ? kVNone : kVFp8;
   // While the selection has at most eight rows per SM it is a chain of latencies that leaves the memory system idle: V is
   // quantised beside it. From there on it fills the chip, and V is cheaper beside K, where its rows are still in L2.
-  // Whole call, us, beside K / beside the selection: 39.4 / 36.9 (2 x 8 heads of 1000), 181.0 / 179.6 (24 of 4608),
-  // 416.5 / 415.5 (16 of 8191), but 2 541 / 2 543 (12 of 32760) and 3 586 / 3 606 (60 of 17776, D = 64).
+  // Whole call, topk 0.2, us, beside K / beside the selection, by rows of the selection:
+  //   below   128 rows ([16 heads, 1000 tokens]) 39.6 / 37.1, 256 ([8,4096]) 49.8 / 48.1, 256 ([1,32760]) 386 / 380,
+  //           576 ([16,4608]) 89.1 / 86.6, 864 ([24,4608]) 122.0 / 120.5, 931 ([1,119056]) 1 292 / 1 287,
+  //           1 024 ([16,8191]) 250.8 / 251.5; two long heads lose: 1 024 ([2,65536]) 761 / 770
+  //   above   1 440 ([40,4608]) 185.3 / 185.0, 1 668 ([12,17776]) 574 / 578, 2 304 ([12,24576]) 728 / 746 (cdf 750 / 771),
+  //           3 072 ([12,32760]) 1 411 / 1 420; D = 64 still gains: 1 920 ([30,8192]) 244.2 / 240.8
   VQuantArgs v_later = {};
   const bool v_beside_selection = select && (long long)p.BH * nq <= 8 * 148;
   int rc = prep_launch(p, v_beside_selection ? &v_later : nullptr, st);

@@ -6,8 +6,8 @@
 // The arithmetic is that of the standalone entries (kmean.cu, pool_quant.cu, quant_v.cu), so the bytes are the same.
 //
 // Why one launch for three tensors: pooling is bound by instruction issue and the column passes by memory, so their
-// CTAs, interleaved in the grid, fill each other's gaps, and a short sequence pays for three launches instead of nine
-// and a memset. The unit of the grid is a span of 256 tokens of one head: with 256 threads that is one or two 128-row
+// CTAs, interleaved in the grid, fill each other's gaps, and a call pays for two launches (three from
+// 2 049 tokens on) instead of nine and a memset. The unit of the grid is a span of 256 tokens of one head: with 256 threads that is one or two 128-row
 // blocks of Q, two or four 64-row blocks of K, or one column pass that is long enough to keep its loads in flight.
 #include "column_passes.cuh"
 #include "launch.cuh"

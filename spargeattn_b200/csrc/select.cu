@@ -585,9 +585,12 @@ static int launch_select(const SelectArgs& a, cudaStream_t st) {
 }
 
 // Two rows per warp share every K value and its conversion, but then a row's steps run behind the other's: worth it where
-// the scores are most of the work and rows are plenty. One against two rows per warp, top-k mode, us: 59 / 71 at 21 rows
-// per SM (12 heads of 256 x 512 blocks), 124 / 114 at 55 (32 heads), 69 / 63 at 56 (60 heads of 139 x 278, D = 64); cdf
-// mode, whose sort and scan are per row: 84 / 108, 178 / 208, 117 / 120.
+// the scores are most of the work and rows are plenty. One against two rows per warp, top-k mode, us, by rows per SM:
+//   256 x 512 blocks:  59 / 71 at 21, 70 / 71 at 28, 78 / 71 at 31, 94 / 90 at 35, 101 / 90 at 42, 125 / 116 at 55
+//   64 x 128:          23 / 26 at 26, 31 / 31 at 35, 34 / 31 at 42;   139 x 278, D = 64: 39 / 42 at 28, 51 / 51 at 34, 57 / 51 at 45
+// Causal rows, whose pairs differ in length, gain nothing or lose: 256 x 512 68 / 80 at 35, 97 / 99 at 55. Long rows fill the
+// SM's shared memory with fewer warps: 931 x 1861 blocks 324 / 397 at 38, 1 123 / 1 181 at 151. cdf mode, whose sort and scan
+// are per row, is always one row per warp (84 / 108 at 21, 178 / 208 at 55).
 constexpr long long kSelPairRows = 148 * 32;
 template <typename T, int D>
 static int dispatch_select(const SelectArgs& a, cudaStream_t st) {
