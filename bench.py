@@ -33,7 +33,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 
 METRIC = "dense_equivalent_attention_throughput_topk0.5"
 # DRAM bytes (read + write) of one attention launch per workload index, as captured by ncu (see profiles/)
-ATTN_DRAM_TRAFFIC_FROM_PROFILE = {2: 155120896 + 69793536}
+ATTN_DRAM_TRAFFIC_FROM_PROFILE = {2: 155773440 + 66030336}
 UNIT = "TOPS"
 NOMINAL_8BIT_TOPS = 4500.0
 
@@ -198,11 +198,31 @@ def measured_8bit_peaks(ops):
     return i8["tops"], f8["tops"], combined
 
 
-def attention_parts(S, core, ops, q, k, v, topk, causal, pvthreshd, reps):
-    """Per-kernel times of one call and the attention kernel's active-block rate."""
+def t_graph(fn, reps, replays=5):
+    """Device time per call of `fn`, captured `reps` times into a CUDA graph: a short chain of launches costs the host more
+    to issue than the device to run."""
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(reps):
+            fn()
+    return t_gpu(graph.replay, replays, warm=1) / reps
+
+
+def attention_parts(S, core, ops, sharding, q, k, v, topk, causal, pvthreshd, reps):
+    """The two parts of one call: everything before the attention kernel (the call itself, with no query block to compute),
+    and the attention kernel on the same operands and LUT with its active-block rate."""
     B, H, N, D = q.shape
     dev = q.device
     qc, kc, vc = core._prologue(q, k, v, "HND")
+    nd = B * H * N * D
+    nq, nk = (N + 127) // 128, (N + 63) // 64
+    none = torch.zeros(B, H, 2, dtype=torch.int32, device=dev)
+    # q read and written as INT8, k twice and INT8, v twice and FP8, the LUT
+    pre_bytes = 3 * nd + 5 * nd + 5 * nd + B * H * nq * nk * 4
+    t = t_graph(lambda: sharding.attention_units(qc, kc, vc, none, 1, topk=topk, is_causal=causal, pvthreshd=pvthreshd), reps)
+    kern = {"preparation_and_selection": {"ms": t, "GBps": pre_bytes / t / 1e6, "alg_bytes": pre_bytes}}
     thr = core.hyperparameter_check(-0.1, H, dev)
     tk = core.hyperparameter_check(topk, H, dev)
     pv = core._pv_threshold_tensor(pvthreshd, H, dev)       # None for the API default (test compiled out)
@@ -211,22 +231,8 @@ def attention_parts(S, core, ops, q, k, v, topk, causal, pvthreshd, reps):
     pk, sk, k8, ks = ops.pool_sim_quant(kc, km, 64, thr)
     lut, valid, _ = ops.select_blocks(pq, pk, sq, sk, tk, None, causal, False, best_first=pv is None)
     v8, vs = ops.quant_v(vc)
-    nd = B * H * N * D
-    nq, nk = (N + 127) // 128, (N + 63) // 64
-    kern = {}
-    t = t_gpu(lambda: ops.k_mean(kc), reps)
-    kern["k_mean"] = {"ms": t, "GBps": 2 * nd / t / 1e6, "alg_bytes": 2 * nd}
-    t = t_gpu(lambda: ops.pool_sim_quant(qc, None, 128, thr), reps)
-    kern["pool_quant_q"] = {"ms": t, "GBps": 3 * nd / t / 1e6, "alg_bytes": 3 * nd}
-    t = t_gpu(lambda: ops.pool_sim_quant(kc, km, 64, thr), reps)
-    kern["pool_quant_k"] = {"ms": t, "GBps": 3 * nd / t / 1e6, "alg_bytes": 3 * nd}
-    sel_bytes = B * H * (2 * (nq + nk) * D + nq * nk * 4)
-    t = t_gpu(lambda: ops.select_blocks(pq, pk, sq, sk, tk, None, causal, False, best_first=pv is None), reps)
-    kern["select"] = {"ms": t, "GBps": sel_bytes / t / 1e6, "alg_bytes": sel_bytes}
-    t = t_gpu(lambda: ops.quant_v(vc), reps)
-    kern["quant_v"] = {"ms": t, "GBps": 3 * nd / t / 1e6, "alg_bytes": 3 * nd}
     out = torch.empty_like(qc)
-    t_attn = t_gpu(lambda: ops.attn_fwd(q8, k8, v8, lut, valid, pv, qs, ks, vs, D ** -0.5, False, qc.dtype, out), reps)
+    t_attn = t_graph(lambda: ops.attn_fwd(q8, k8, v8, lut, valid, pv, qs, ks, vs, D ** -0.5, False, qc.dtype, out), reps)
     live = int(valid.sum().item())
     active_flop = 4.0 * 128 * 64 * D * live
     kern["attn"] = {"ms": t_attn, "active_TOPS": active_flop / (t_attn * 1e-3) / 1e12, "live_blocks": live,
@@ -243,7 +249,7 @@ def launches_per_call(idx, syn):
     return 5 if syn.workload_shape(idx)[2] > 2048 else 4
 
 
-def config_row(S, core, ops, syn, idx, topk, pvthreshd, dev, peak8, reps=5):
+def config_row(S, core, ops, sharding, syn, idx, topk, pvthreshd, dev, peak8, reps=5):
     """One workload through the public API on this GPU: call latency, dense-equivalent and active-block rates."""
     w = syn.WORKLOADS[idx]
     B, H, N, D = syn.workload_shape(idx)
@@ -251,13 +257,13 @@ def config_row(S, core, ops, syn, idx, topk, pvthreshd, dev, peak8, reps=5):
     q, k, v = (t.view(B, H, N, D) for t in syn.workload_heads_qkv(idx, heads, dev))
     api = lambda: S.spas_sage2_attn_meansim_topk_cuda(q, k, v, topk=topk, is_causal=w["causal"], pvthreshd=pvthreshd)
     ms = t_gpu(api, reps, warm=3)
-    kern, _ = attention_parts(S, core, ops, q, k, v, topk, w["causal"], pvthreshd, reps)
+    kern, _ = attention_parts(S, core, ops, sharding, q, k, v, topk, w["causal"], pvthreshd, reps)
     a = kern["attn"]
     row = {"workload": workload_text(syn, idx, topk, pvthreshd), "api_ms": ms,
            "dense_equiv_TOPS": dense_equiv_ops(B, H, N, D, w["causal"]) / ms / 1e9, "attn_ms": a["ms"],
            "active_TOPS": a["active_TOPS"], "frac_of_measured_8bit_peak": a["active_TOPS"] / peak8,
            "density": a["density"],
-           "preprocess_ms": sum(kern[n]["ms"] for n in ("k_mean", "pool_quant_q", "pool_quant_k", "select", "quant_v"))}
+           "preprocess_ms": kern["preparation_and_selection"]["ms"]}
     if idx == 1:    # the same shape through block_sparse_sage2_attn_cuda with a Bernoulli(0.4) block mask, diagonal forced
         mask = syn.bernoulli_block_mask(B, H, N, 0.4, 1, dev)
         t = t_gpu(lambda: S.block_sparse_sage2_attn_cuda(q, k, v, mask_id=mask), reps, warm=3)
@@ -469,12 +475,11 @@ def main():
         bf16_peak = float(peaks.get("bf16_tflops", 1590.0))
         peak_src = "measured" if peaks else "fallback"
         reps = max(5, min(args.steps, 20))
-        kernels, parts = attention_parts(S, core, ops, q, k, v, topk, causal, args.pvthreshd, reps)
+        kernels, parts = attention_parts(S, core, ops, sharding, q, k, v, topk, causal, args.pvthreshd, reps)
         # the peak probe loads the tensor pipe for ~0.1 s and can pull the clocks down for a moment: it runs after
         # the kernels have been timed, and the other workloads below start with their own warm-up calls
         i8_peak, f8_peak, peak8 = measured_8bit_peaks(ops)
-        for kname in ("k_mean", "pool_quant_q", "pool_quant_k", "select", "quant_v"):
-            kernels[kname]["frac_of_hbm_peak"] = kernels[kname]["GBps"] / hbm_peak
+        kernels["preparation_and_selection"]["frac_of_hbm_peak"] = kernels["preparation_and_selection"]["GBps"] / hbm_peak
         a = kernels["attn"]
         roofline = {"kernel": "attn_kernel (tcgen05 INT8 QK^T + FP8 PV)", "bound": "tensor", "achieved": a["active_TOPS"],
                     "peak": peak8, "unit": "TFLOP/s", "frac": a["active_TOPS"] / peak8,
@@ -485,8 +490,8 @@ def main():
                                   f"vendor nominal {NOMINAL_8BIT_TOPS:.0f} (frac_of_nominal {a['active_TOPS'] / NOMINAL_8BIT_TOPS:.3f})"),
                     "algorithmic_flop_per_launch": a["active_flop"], "launch_ms": a["ms"],
                     "traffic": ATTN_DRAM_TRAFFIC_FROM_PROFILE.get(idx) if world == 1 else None,
-                    "traffic_note": ("dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload, from the ncu "
-                                     "capture summarised in profiles/attn_kernel_cfg2_wan480p.md (a recorded figure, not measured "
+                    "traffic_note": ("dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload, from an ncu "
+                                     "capture (a recorded figure, not measured "
                                      f"by this run); algorithmic operand bytes of this launch: {a['alg_bytes']}"),
                     "hbm_peak_GBps": hbm_peak}
         if world == 1 and not args.no_extras:
@@ -509,12 +514,12 @@ def main():
             rows = {}
             if idx == 2:
                 for tk_, pv_ in ((0.3, 50.0), (0.7, 50.0), (0.5, 5.0)):
-                    rows[f"cfg2_topk{tk_:g}_pv{pv_:g}"] = config_row(S, core, ops, syn, 2, tk_, pv_, dev, peak8)
+                    rows[f"cfg2_topk{tk_:g}_pv{pv_:g}"] = config_row(S, core, ops, sharding, syn, 2, tk_, pv_, dev, peak8)
             del q, k, v
             torch.cuda.empty_cache()
             for j in (0, 1, 3, 4):
                 if j != idx:
-                    rows[f"cfg{j}"] = config_row(S, core, ops, syn, j, syn.WORKLOADS[j]["topk"], 50.0, dev, peak8)
+                    rows[f"cfg{j}"] = config_row(S, core, ops, sharding, syn, j, syn.WORKLOADS[j]["topk"], 50.0, dev, peak8)
             extras["configs"] = rows
             extras["reference_on_this_gpu"] = reference_on_gpu([0, 1, 2, 3, 4])
         ops.check_device_status(dev)
