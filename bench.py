@@ -489,7 +489,7 @@ def main():
                                   f"harmonic mean. For context: 2 x {peak_src} dense bf16 burst = {2 * bf16_peak:.0f}, "
                                   f"vendor nominal {NOMINAL_8BIT_TOPS:.0f} (frac_of_nominal {a['active_TOPS'] / NOMINAL_8BIT_TOPS:.3f})"),
                     "algorithmic_flop_per_launch": a["active_flop"], "launch_ms": a["ms"],
-                    "traffic": ATTN_DRAM_TRAFFIC_FROM_PROFILE.get(idx) if world == 1 else None,
+                    "traffic": ATTN_DRAM_TRAFFIC_FROM_PROFILE.get(idx) if part_world == 1 else None,
                     "traffic_note": ("dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload, from an ncu "
                                      "capture (a recorded figure, not measured "
                                      f"by this run); algorithmic operand bytes of this launch: {a['alg_bytes']}"),
