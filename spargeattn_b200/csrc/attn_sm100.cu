@@ -176,14 +176,15 @@ constexpr int kAttnThreads = 192;
 
 // GRAN = qk_quant_gran: 1 one Q scale per 128-row block, 2 one per 32-row group (the K scale is per 64-key block in
 // both), 3 per-thread Q/K scales. PV_MODE = PVThresholdMode: 0 no skip test, 1 the test decides per block, 2 per
-// 32-row group.
-template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16 = false>
+// 32-row group. ORDERED: rows in the order of row_order or order_heads (AttnArgs); a variant of its own because the two
+// registers that it takes cost the others 1 %.
+template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16 = false, bool ORDERED = false>
 __global__ void __launch_bounds__(kAttnThreads, (AttnShape<D, PVF16>::kCtasPerSm))
 attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
             const __grid_constant__ CUtensorMap tmap_v, OutT* __restrict__ o, const int32_t* lut, const int32_t* valid,
             const float* pvthr, const float* q_scale, const float* k_scale, const float* v_scale, int32_t* dev_status, int N,
             int H, int nq, int nk, float sm_scale_log2, long long osb, long long osh, long long osn,
-            int32_t* __restrict__ pv_count, const int32_t* q_ranges) {
+            int32_t* __restrict__ pv_count, const int32_t* q_ranges, const int32_t* row_order, int order_heads) {
   using Shape = AttnShape<D, PVF16>;
   constexpr bool PV_SKIP = PV_MODE != 0, pv_per_warp = PV_MODE == 2, GRAN3 = GRAN == 3;
   constexpr int SK = Shape::kStagesK, NV = Shape::kSlotsV;
@@ -198,6 +199,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   __shared__ uint64_t bar_q, bar_k_full[SK], bar_k_empty[SK], bar_v_full[NV], bar_v_empty[NV], bar_s_full, bar_s_free,
       bar_p_ready[2], bar_o_done[2], bar_vote[2];   // the pairs alternate by step
   __shared__ uint32_t s_tmem_base;
+  __shared__ int s_row;                // ORDERED: the CTA's row
   __shared__ int s_skip[2][2], s_fail;   // [step parity][block of the pair]
   // PV-skip votes, one byte per softmax warp: [step parity][block of the pair]
   __shared__ uint32_t s_vote[2][2];
@@ -207,18 +209,29 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   // the shuffles let the compiler see that these are the same for the whole warp: branches on them need no convergence
   // bookkeeping and the operands of the MMA instructions can be kept in uniform registers
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  // Query blocks are issued last-first: under a causal mask the late rows hold the most live blocks, and a head's longest
-  // rows start first. (Heads follow one another, so the last head's longest rows still start late.)
+  // Query blocks are issued last-first: under a causal mask the late rows hold the most live blocks, and the longest rows of
+  // a head, or of a group of heads, start first. row_order names the rows of a map that is not known beforehand.
   // With q_ranges, (batch, head) bh computes only its query blocks [begin, begin + count): the unit of the
   // multi-GPU row sharding. The grid is sized for the largest count; the other CTAs leave at once.
-  const int bh = blockIdx.y, h = bh % H;
+  int at = 0;   // ORDERED: the CTA's row
+  if (ORDERED) {
+    const int i = blockIdx.y * gridDim.x + blockIdx.x;
+    if (row_order) {
+      pdl_wait();
+      at = __shfl_sync(0xffffffffu, row_order[i], 0);
+    } else {
+      const int first = i / (order_heads * nq) * order_heads, j = i - first * nq, heads = min(order_heads, (int)gridDim.y - first);
+      at = (first + j % heads) * nq + nq - 1 - j / heads;
+    }
+  }
+  const int bh = ORDERED ? at / nq : blockIdx.y, h = bh % H;
   const int q_begin = q_ranges ? q_ranges[2 * bh] : 0;
   const int q_count = q_ranges ? min(q_ranges[2 * bh + 1], nq - q_begin) : (int)gridDim.x;
   if ((int)blockIdx.x >= q_count) {
     pdl_wait();   // when every CTA leaves here, this kernel must still not end before the ones that it depends on
     return;
   }
-  const int qi = q_begin + q_count - 1 - (int)blockIdx.x;
+  const int qi = ORDERED ? at - bh * nq : q_begin + q_count - 1 - (int)blockIdx.x;
   const size_t row_id = (size_t)bh * nq + qi;
 
   if (warp == kMmaWarp) {
@@ -250,6 +263,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     }
     mbar_fence_init();
     s_fail = 0;
+    if (ORDERED) s_row = at;   // for the epilogue: a register that lives through the loop costs
   }
   pdl_wait();   // everything below reads what the kernels before this one wrote
   // V's scales wait in shared memory for the epilogue, where 128 loads per thread from global memory were a fifth of a
@@ -641,12 +655,14 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       // One count per 32-row group, the layout of the reference's PV_Count (qk_int_sv_f8_cuda_sm89.cuh:650-656).
       // With the per-block decision the four entries of a block are equal; with the per-warp decision each group
       // has its own.
-      if (pv_count && lane == 0) pv_count[row_id * 4 + warp] = npv;
+      const int row_end = ORDERED ? *(volatile int*)&s_row : 0, bh_end = ORDERED ? row_end / nq : bh;
+      const int qrow_end = ORDERED ? (row_end - bh_end * nq) * 128 + row : qrow;
+      if (pv_count && lane == 0) pv_count[(ORDERED ? (size_t)row_end : row_id) * 4 + warp] = npv;
       // A row that saw no key at all (token-level causal mask over every live block of its row of blocks) has an
       // empty sum: it is written as zeros. (The reference gives such a row the plain average of V over the masked
       // keys, because its mask value is a large finite number and exp2(mask - mask) = 1.)
       const float inv = d > 0.f ? rcp_approx(d) : 0.f;
-      OutT* orow = o + (size_t)(bh / H) * osb + (size_t)(bh % H) * osh + (size_t)qrow * osn;
+      OutT* orow = o + (size_t)(bh_end / H) * osb + (size_t)(bh_end % H) * osh + (size_t)qrow_end * osn;
 #pragma unroll
       for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t ov[32];
@@ -660,7 +676,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
           w[i] = pack2<OutT>(__uint_as_float(ov[2 * i]) * inv * vs.x, __uint_as_float(ov[2 * i + 1]) * inv * vs.y);
           w[i + 1] = pack2<OutT>(__uint_as_float(ov[2 * i + 2]) * inv * vs.z, __uint_as_float(ov[2 * i + 3]) * inv * vs.w);
         }
-        if (qrow < N) {
+        if (qrow_end < N) {
           uint4* dst = reinterpret_cast<uint4*>(orow + c0);
 #pragma unroll
           for (int i = 0; i < 4; i++) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
@@ -732,9 +748,11 @@ static bool attn_attributes(const void* kern, int smem, std::atomic<uint64_t>& d
   return true;
 }
 
-template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16>
+template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16, bool ORDERED = false>
 static int launch_attn(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, cudaStream_t st) {
-  auto kern = attn_kernel<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16>;
+  if (GRAN == 1 && PV_MODE != 2 && !ORDERED && !a.q_ranges && (a.row_order || a.order_heads > 1))
+    return launch_attn<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16, GRAN == 1 && PV_MODE != 2>(a, tq, tk, tv, st);
+  auto kern = attn_kernel<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16, ORDERED>;
   constexpr int smem = AttnShape<D, PVF16>::kSmemBytes;
   static std::atomic<uint64_t> done{0};
   if (!attn_attributes((const void*)kern, smem, done)) return SPARGE_ERR_CUDA;
@@ -742,7 +760,7 @@ static int launch_attn(const AttnArgs& a, const CUtensorMap& tq, const CUtensorM
   const int gx = a.q_ranges ? min(a.q_blocks_max, nq) : nq;
   const cudaError_t e = launch(kern, dim3(gx, a.B * a.H), kAttnThreads, smem, st, a.dependent, tq, tk, tv, (OutT*)a.o, a.lut,
                                a.valid, a.pvthr, a.q_scale, a.k_scale, a.v_scale, a.dev_status, a.N, a.H, nq, nk,
-                               a.sm_scale * kLog2e, a.o_st[0], a.o_st[1], a.o_st[2], a.pv_count, a.q_ranges);
+                               a.sm_scale * kLog2e, a.o_st[0], a.o_st[1], a.o_st[2], a.pv_count, a.q_ranges, a.row_order, a.order_heads);
   return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
 }
 

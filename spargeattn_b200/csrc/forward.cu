@@ -2,7 +2,10 @@
 // (spas_sage_attn/core.py:39-169), of their fp16-PV counterparts (:235-319) and of block_sparse_sage2_attn_cuda
 // (:171-233): K mean, pooling + self-similarity + INT8 quantisation of Q and K, V quantiser, block selection + LUT,
 // block-sparse attention, on one stream with every intermediate tensor carved out of one workspace. Four launches (five
-// from 2 049 tokens on), each a programmatic dependent of the one before it; issued entry by entry the path takes ten.
+// from 2 049 tokens on, six where the rows of a cdf selection are sorted by length), each a programmatic dependent of the
+// one before it; issued entry by entry the path takes ten.
+#include <algorithm>
+
 #include "attn.cuh"
 #include "forward.cuh"
 #include "prep.cuh"
@@ -87,6 +90,21 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
   }
   if (rc != SPARGE_OK) return rc;
 
+  // With cdf selection or a causal map the rows differ in length, and a long one that starts late keeps the chip waiting: they
+  // are computed longest first, over as many heads as have their K and V in kOrderBytes (all twelve heads of [1,12,32760,128],
+  // 100 MB, cost more in L2 misses than the order gave). A causal row is the longer the later it is. cdf counts are sorted,
+  // where there are more rows than the chip holds at a time and a row is long enough to be worth the launch.
+  constexpr long long kOrderBytes = 48LL << 20;
+  constexpr int kSortBlocks = 80;
+  const long long head_bytes = (a.pv_fp16 ? 3LL : 2LL) * a.N * a.D;
+  const int order_heads = (int)std::max(1LL, std::min((long long)p.BH, kOrderBytes / head_bytes));
+  int32_t* rows = nullptr;
+  if (select && a.cdf && !a.q_ranges && nk > kSortBlocks && (long long)p.BH * nq > 2 * 148) {
+    rows = static_cast<int32_t*>(p.scratch);   // free again: the preparation's partial sums
+    rc = row_order_launch(valid, rows, p.BH * nq, order_heads * nq, nk, st);
+    if (rc != SPARGE_OK) return rc;
+  }
+
   AttnArgs t = {};
   t.q8 = p.q8, t.k8 = p.k8, t.o = a.o, t.lut = lut, t.valid = valid, t.pvthr = a.pvthr;
   t.q_scale = p.qs, t.k_scale = p.ks, t.v_scale = p.v_scale, t.dev_status = a.dev_status;
@@ -97,6 +115,7 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
     t.o_st[i] = a.o_st[i];
     t.v_st[i] = copy_v ? packed[i] : a.v_st[i];
   }
+  t.row_order = rows, t.order_heads = select && a.is_causal ? order_heads : 0;
   t.q_ranges = a.q_ranges, t.q_blocks_max = a.q_blocks_max, t.B = a.B, t.H = a.H, t.N = a.N, t.D = a.D;
   t.out_dtype = a.dtype, t.causal = a.kernel_causal, t.gran = 1, t.pv_mode = a.pvthr != nullptr, t.dependent = true;
   t.sm_scale = a.sm_scale;

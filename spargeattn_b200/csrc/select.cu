@@ -566,6 +566,45 @@ __global__ void __launch_bounds__(kSelThreads) mask_to_lut_kernel(const uint8_t*
   pdl_trigger();
 }
 
+// Counting sort of a group of rows by their number of live blocks, longest first, by one CTA per group. Rows of one bucket
+// come in any order: it decides when a row is computed, not what comes out.
+constexpr int kOrderThreads = 1024, kOrderBuckets = 256;
+__global__ void __launch_bounds__(kOrderThreads) row_order_kernel(const int32_t* valid, int32_t* __restrict__ rows, int n, int group,
+                                                                  int nk) {
+  __shared__ int s_place[kOrderBuckets], s_sum[kOrderBuckets / 32];
+  const int tid = threadIdx.x, first = blockIdx.x * group, last = min(n, first + group);
+  if (tid < kOrderBuckets) s_place[tid] = 0;
+  pdl_wait();
+  __syncthreads();
+  auto bucket = [&](int i) { return kOrderBuckets - 1 - (int)((long long)min(max(valid[i], 0), nk) * (kOrderBuckets - 1) / nk); };
+  for (int i = first + tid; i < last; i += kOrderThreads) atomicAdd(&s_place[bucket(i)], 1);
+  __syncthreads();
+  int mine = 0, incl = 0;
+  if (tid < kOrderBuckets) {
+    incl = mine = s_place[tid];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((tid & 31) >= o) incl += t;
+    }
+    if ((tid & 31) == 31) s_sum[tid >> 5] = incl;
+  }
+  __syncthreads();
+  if (tid < kOrderBuckets) {
+    for (int w = 0; w < tid >> 5; w++) incl += s_sum[w];
+    s_place[tid] = first + incl - mine;
+  }
+  __syncthreads();
+  for (int i = first + tid; i < last; i += kOrderThreads) rows[atomicAdd(&s_place[bucket(i)], 1)] = i;
+  pdl_trigger();
+}
+
+int row_order_launch(const int32_t* valid, int32_t* rows, int n, int group, int nk, cudaStream_t st) {
+  return launch(row_order_kernel, dim3((n + group - 1) / group), kOrderThreads, 0, st, true, valid, rows, n, group, nk) == cudaSuccess
+             ? SPARGE_OK
+             : SPARGE_ERR_CUDA;
+}
+
 template <typename T, int D, int RW, int WARPS>
 static int launch_select(const SelectArgs& a, cudaStream_t st) {
   // cdf mode reproduces torch.cumsum over the [B*H*nq, nk] matrix of sorted probabilities: the scan's chunking

@@ -310,6 +310,28 @@ def test_c_entry_of_the_whole_path(kw, N, D, dtype, v_dtype):
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("kw", [dict(cdfthreshd=0.8, simthreshd1=0.3), dict(topk=0.3, is_causal=True), dict(cdfthreshd=0.7, is_causal=True, pvthreshd=4.0)])
+@pytest.mark.parametrize("H,N,D", [(148, 256, 64), (297, 128, 64), (5, 7700, 128), (41, 4996, 128)])
+def test_longest_rows_first(kw, H, N, D):
+    """Rows that differ in length are computed in another order: from 297 of them on, here one group of heads, the last case
+    two. Every row has to come out, with the bytes of the separate entries, which compute them in their own order."""
+    import spargeattn_b200 as S
+    from spargeattn_b200 import core, ops
+    g = torch.Generator("cuda").manual_seed(N)
+    q, k, v = (torch.randn(1, H, N, D, generator=g, device="cuda").bfloat16() for _ in range(3))
+    k[:, :, :64] *= 3
+    fn = S.spas_sage2_attn_meansim_topk_cuda if "topk" in kw else S.spas_sage2_attn_meansim_cuda
+    one = fn(q, k, v, **kw)
+    single = core.SINGLE_CALL_MAX_ROWS
+    try:
+        core.SINGLE_CALL_MAX_ROWS = 0
+        separate = fn(q, k, v, **kw)
+    finally:
+        core.SINGLE_CALL_MAX_ROWS = single
+    ops.check_device_status()
+    assert torch.equal(one, separate)
+
+
 def test_ranges_without_a_largest_count_are_an_assertion():
     from spargeattn_b200.sharding import attention_units
     q = torch.randn(1, 2, 256, 64).bfloat16().cuda()
