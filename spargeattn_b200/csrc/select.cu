@@ -92,7 +92,9 @@ __device__ __forceinline__ float key_value<__nv_bfloat16>(uint32_t k) {
 //   2  per row, by its warp alone (shuffles and ballots): fp64 softmax, selection threshold by bisection over the 16 key
 //      bits with eight keys per lane and load, final map and LUT.
 // What bounds it: instruction issue of the score chains (1.3 per score and channel), then the fp64 pipe; a short row is a
-// chain of dependent reductions.
+// chain of dependent reductions. With one row per warp the chain is kept short: the first tile is asked for together with the
+// query, exponentials go four at a time and are kept, the three counts of a bisection round share one reduction. Whole
+// calls: [2,8,1000,128] 36.9 -> 35.8 us, [1,24,4608,128] 177.2 -> 176.9, cdf [1,16,8191,128] 382 -> 381.
 constexpr int kSelTileKeys = 64;
 // Marks of a block that is not self-similar: in place of its score, and in place of its probability (zero, with the sign
 // bit telling that the block is live whatever the selection says).
@@ -289,18 +291,43 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
 #pragma unroll
   for (int r = 0; r < RW; r++) q_similar[r] = sim_q[(size_t)bh * nq + min(q0 + r, nq - 1)];
 
+  // The query, each value twice (a packed FMA takes it as it is), and the first tile: asked for together, one latency less.
+  const T* pkb = pk + (size_t)bh * nk * D;
+  constexpr int kTileLoads = kSelTileKeys * kChunksPerRow / (WARPS * 32);   // 128-bit loads of a tile by a thread
+  constexpr bool kFirstTile = RW == 1 && kTileLoads <= 8;
+  auto tile_load = [&](int j0, int i) {
+    const int row = i / kChunksPerRow, c = i % kChunksPerRow;
+    return j0 + row < nk ? *reinterpret_cast<const uint4*>(pkb + (size_t)(j0 + row) * D + c * 8) : make_uint4(0, 0, 0, 0);
+  };
+  auto tile_store = [&](int i, const uint4& val) {
+    *reinterpret_cast<uint4*>(smem_raw + i / kChunksPerRow * kTileRowBytes + i % kChunksPerRow * 16) = val;
+  };
+  {
+    T qv[RW][D / 32];
 #pragma unroll
-  for (int r = 0; r < RW; r++) {   // the query, each value twice: a packed FMA takes it as it is
-    float2* s_q = reinterpret_cast<float2*>(work_of(r));
-    for (int d = lane; d < D; d += 32) {
-      const float v = q0 + r < nq ? Elem<T>::to_float(pq[((size_t)bh * nq + q0 + r) * D + d]) : 0.f;
-      s_q[d] = make_float2(v, v);
+    for (int r = 0; r < RW; r++)
+#pragma unroll
+      for (int d = 0; d < D / 32; d++) qv[r][d] = pq[((size_t)bh * nq + min(q0 + r, nq - 1)) * D + d * 32 + lane];
+    uint4 first[kFirstTile ? kTileLoads : 1];
+    if (kFirstTile) {
+#pragma unroll
+      for (int i = 0; i < kTileLoads; i++) first[i] = tile_load(0, threadIdx.x + i * WARPS * 32);
+    }
+#pragma unroll
+    for (int r = 0; r < RW; r++)
+#pragma unroll
+      for (int d = 0; d < D / 32; d++) {
+        const float v = Elem<T>::to_float(qv[r][d]);
+        reinterpret_cast<float2*>(work_of(r))[d * 32 + lane] = make_float2(v, v);
+      }
+    if (kFirstTile) {
+#pragma unroll
+      for (int i = 0; i < kTileLoads; i++) tile_store(threadIdx.x + i * WARPS * 32, first[i]);
     }
   }
 
   // ---- 1: scores
   const float scale = (D == 64) ? 0.125f : 0.08838834764831845f;   // float(D ** -0.5)
-  const T* pkb = pk + (size_t)bh * nk * D;
   const uint8_t* simk = sim_k + (size_t)bh * nk;
   const int cta_limit = limit_of(min(nq, ((int)blockIdx.x + 1) * WARPS * RW) - 1);   // keys any row of the CTA sees
   const T minus_inf = Elem<T>::from_float(-INFINITY);
@@ -313,12 +340,9 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
 #pragma unroll
     for (int hf = 0; hf < 2; hf++) similar[hf] = j0 + 32 * hf + lane < nk ? simk[j0 + 32 * hf + lane] : 0;
     if (seen) {
-      __syncthreads();                                       // previous tile fully consumed
-      for (int i = threadIdx.x; i < kSelTileKeys * kChunksPerRow; i += WARPS * 32) {
-        const int row = i / kChunksPerRow, c = i % kChunksPerRow;
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (j0 + row < nk) val = *reinterpret_cast<const uint4*>(pkb + (size_t)(j0 + row) * D + c * 8);
-        *reinterpret_cast<uint4*>(smem_raw + row * kTileRowBytes + c * 16) = val;
+      if (!kFirstTile || j0 > 0) {
+        __syncthreads();                                     // previous tile fully consumed
+        for (int i = threadIdx.x; i < kSelTileKeys * kChunksPerRow; i += WARPS * 32) tile_store(i, tile_load(j0, i));
       }
       __syncthreads();
     }
@@ -379,13 +403,31 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
       q_similar[i] = q_similar[i + 1];
     }
 
-    // fp64 softmax -> 16-bit keys (p >= 0, so the bit pattern orders like the value). The exponentials are evaluated
-    // twice, once for the sum and once for the probabilities, instead of being stored.
-    double Z = 0.0;
-    for (int j = lane; j < nk; j += 32) {
+    // fp64 softmax -> 16-bit keys (p >= 0, so the bit pattern orders like the value). One row per warp is a chain of
+    // latencies: the exponentials of its first 256 keys are evaluated four at a time and kept. The others are evaluated twice,
+    // once for the sum and once for the probabilities, instead of being stored; so are all of them with two rows per warp,
+    // where the registers cost more than the instructions ([2,30,17776,64]: call 3 552 -> 3 576 us).
+    constexpr int kKeep = RW == 1 ? 8 : 0;
+    const double dmx = (double)mx;
+    double e[kKeep > 0 ? kKeep : 1], Z = 0.0;
+#pragma unroll
+    for (int g = 0; g < kKeep; g += 4) {
+      if (g * 32 < nk) {
+#pragma unroll
+        for (int i = g; i < g + 4; i++) {
+          const int j = i * 32 + lane;
+          const uint16_t raw = j < nk ? s_key[j] : kNotSimilarScore;
+          const float sc = key_value<T>(raw);
+          e[i] = exp_nonpositive(raw != kNotSimilarScore && sc != -INFINITY ? (double)sc - dmx : -1000.0);
+        }
+#pragma unroll
+        for (int i = g; i < g + 4; i++) Z += e[i];
+      }
+    }
+    for (int j = kKeep * 32 + lane; j < nk; j += 32) {
       const uint16_t raw = s_key[j];
       const float sc = key_value<T>(raw);
-      if (raw != kNotSimilarScore && sc != -INFINITY) Z += exp_nonpositive((double)sc - (double)mx);
+      if (raw != kNotSimilarScore && sc != -INFINITY) Z += exp_nonpositive((double)sc - dmx);
     }
     Z = warp_sum(Z);
     const double rz = 1.0 / Z;
@@ -393,13 +435,22 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
     // n_sel blocks. Zeros are equal too, and the comparisons below can count them.
     const bool undefined = Z != Z;
     const int padded = (nk + 255) / 256 * 256;
-    for (int j = lane; j < padded; j += 32) {
+    auto key_of = [&](uint16_t raw, double ej) -> uint16_t {
+      if (raw == kNotSimilarScore) return kNotSimilarKey;
+      if (key_value<T>(raw) == -INFINITY || undefined) return 0;
+      return (uint16_t)key_bits<T>(Elem<T>::from_float((float)(ej * rz)));
+    };
+#pragma unroll
+    for (int i = 0; i < kKeep; i++) {                        // (a row has 256 keys or padding)
+      const int j = i * 32 + lane;
+      s_key[j] = j < nk ? key_of(s_key[j], e[i]) : (uint16_t)0;
+    }
+    for (int j = kKeep * 32 + lane; j < padded; j += 32) {
       uint16_t key = 0;
       if (j < nk) {
         const uint16_t raw = s_key[j];
         const float sc = key_value<T>(raw);
-        if (raw == kNotSimilarScore) key = kNotSimilarKey;
-        else if (sc != -INFINITY && !undefined) key = (uint16_t)key_bits<T>(Elem<T>::from_float((float)(exp_nonpositive((double)sc - (double)mx) * rz)));
+        key = key_of(raw, raw != kNotSimilarScore && sc != -INFINITY ? exp_nonpositive((double)sc - dmx) : 0.0);
       }
       s_key[j] = key;
     }
@@ -435,16 +486,24 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
     // reductions); padding and not-similar keys count as zero
     const uint4* groups = reinterpret_cast<const uint4*>(s_key);
     const uint4 own = groups[lane];                          // all there is of a row of up to 256 blocks
-    auto count = [&](uint32_t cand) {
+    auto count_lane = [&](uint32_t cand) {
       const uint32_t cand2 = cand | (cand << 16);
       int c = count_ge<T>(own, cand2);
       for (int i = lane + 32; i < padded / 8; i += 32) c += count_ge<T>(groups[i], cand2);
-      return (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
+      return (unsigned)c;
     };
+    auto count = [&](uint32_t cand) { return (int)__reduce_add_sync(0xffffffffu, count_lane(cand)); };
     uint32_t thr_key = count(1u << 14) >= n_sel ? 1u << 14 : 0u;
 #pragma unroll 1
     for (int bit = 12; bit >= 0; bit -= 2) {
-      const int c1 = count(thr_key | (1u << bit)), c2 = count(thr_key | (2u << bit)), c3 = count(thr_key | (3u << bit));
+      int c1, c2, c3;
+      const unsigned l1 = count_lane(thr_key | (1u << bit)), l2 = count_lane(thr_key | (2u << bit)), l3 = count_lane(thr_key | (3u << bit));
+      if (RW == 1 && padded < 1024) {                        // ten bits hold a count: one reduction for all three
+        const unsigned c = __reduce_add_sync(0xffffffffu, l1 | (l2 << 10) | (l3 << 20));
+        c1 = c & 1023, c2 = (c >> 10) & 1023, c3 = c >> 20;
+      } else {
+        c1 = (int)__reduce_add_sync(0xffffffffu, l1), c2 = (int)__reduce_add_sync(0xffffffffu, l2), c3 = (int)__reduce_add_sync(0xffffffffu, l3);
+      }
       thr_key |= (uint32_t)((c1 >= n_sel) + (c2 >= n_sel) + (c3 >= n_sel)) << bit;
     }
     const int remaining = n_sel - count(thr_key + 1);
