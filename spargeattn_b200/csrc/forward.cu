@@ -91,10 +91,13 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
   if (rc != SPARGE_OK) return rc;
 
   // With cdf selection or a causal map the rows differ in length, and a long one that starts late keeps the chip waiting: they
-  // are computed longest first, over as many heads as have their K and V in kOrderBytes (all twelve heads of [1,12,32760,128],
-  // 100 MB, cost more in L2 misses than the order gave). A causal row is the longer the later it is. cdf counts are sorted,
-  // where there are more rows than the chip holds at a time and a row is long enough to be worth the launch.
-  constexpr long long kOrderBytes = 48LL << 20;
+  // are computed longest first, over as many heads as have their K and V in kOrderBytes. A causal row is the longer the later
+  // it is. cdf counts are sorted, where there are more rows than the chip holds at a time and a row is long enough to be worth
+  // the launch: 239 -> 243 us with 64 blocks a row (cdf, [1,24,4096,128]), 374.7 -> 369.9 with 94 ([1,24,6000,128]).
+  // Calls in us, head by head and with 16 / 32 / 48 / 96 MB: causal top-k [1,32,32768,128] 5 052 and 5 013 / 4 980 / 4 989 / 5 064,
+  // [1,40,15000,64] 1 250 and 1 166 / 1 173 / 1 162 / 1 159; cdf [1,12,32760,128] 3 266 and 3 269 / 3 243 / 3 269 / 3 273,
+  // [2,20,10800,64] 1 333 and 1 306 / 1 293 / 1 312 / 1 287, [1,24,16200,128] 1 904 and 1 855 / 1 847 / 1 863 / 1 876.
+  constexpr long long kOrderBytes = 32LL << 20;
   constexpr int kSortBlocks = 80;
   const long long head_bytes = (a.pv_fp16 ? 3LL : 2LL) * a.N * a.D;
   const int order_heads = (int)std::max(1LL, std::min((long long)p.BH, kOrderBytes / head_bytes));
