@@ -14,10 +14,10 @@ struct AttnArgs {
   const float *pvthr, *q_scale, *k_scale, *v_scale;
   int32_t *dev_status, *pv_count;
   const int32_t* q_ranges;
-  // Which row a CTA computes, without q_ranges: row_order [B*H*ceil(N/128)], or else late rows first over groups of
-  // order_heads heads (0 or 1: head by head)
+  // Which row a CTA computes, without q_ranges: row_order [B*H*ceil(N/128)], or else late rows first in each of
+  // order_groups groups of heads (0, or as many as there are heads: head by head)
   const int32_t* row_order;
-  int order_heads;
+  int order_groups;
   int q_blocks_max, B, H, N, D, out_dtype, causal, gran, pv_mode;
   bool v_f16, dependent;            // dependent: programmatic launch behind the kernel before it on the stream
   float sm_scale;

@@ -30,6 +30,7 @@
 
 #include "attn.cuh"
 #include "launch.cuh"
+#include "row_groups.cuh"
 #include "sm100_ptx.cuh"
 #include "step_word.cuh"
 
@@ -176,7 +177,7 @@ constexpr int kAttnThreads = 192;
 
 // GRAN = qk_quant_gran: 1 one Q scale per 128-row block, 2 one per 32-row group (the K scale is per 64-key block in
 // both), 3 per-thread Q/K scales. PV_MODE = PVThresholdMode: 0 no skip test, 1 the test decides per block, 2 per
-// 32-row group. ORDERED: rows in the order of row_order or order_heads (AttnArgs); a variant of its own because the two
+// 32-row group. ORDERED: rows in the order of row_order or order_groups (AttnArgs); a variant of its own because the two
 // registers that it takes cost the others 1 %.
 template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16 = false, bool ORDERED = false>
 __global__ void __launch_bounds__(kAttnThreads, (AttnShape<D, PVF16>::kCtasPerSm))
@@ -184,7 +185,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
             const __grid_constant__ CUtensorMap tmap_v, OutT* __restrict__ o, const int32_t* lut, const int32_t* valid,
             const float* pvthr, const float* q_scale, const float* k_scale, const float* v_scale, int32_t* dev_status, int N,
             int H, int nq, int nk, float sm_scale_log2, long long osb, long long osh, long long osn,
-            int32_t* __restrict__ pv_count, const int32_t* q_ranges, const int32_t* row_order, int order_heads) {
+            int32_t* __restrict__ pv_count, const int32_t* q_ranges, const int32_t* row_order, int order_groups) {
   using Shape = AttnShape<D, PVF16>;
   constexpr bool PV_SKIP = PV_MODE != 0, pv_per_warp = PV_MODE == 2, GRAN3 = GRAN == 3;
   constexpr int SK = Shape::kStagesK, NV = Shape::kSlotsV;
@@ -215,13 +216,13 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   // multi-GPU row sharding. The grid is sized for the largest count; the other CTAs leave at once.
   int at = 0;   // ORDERED: the CTA's row
   if (ORDERED) {
-    const int i = blockIdx.y * gridDim.x + blockIdx.x;
     if (row_order) {
       pdl_wait();
-      at = __shfl_sync(0xffffffffu, row_order[i], 0);
+      at = __shfl_sync(0xffffffffu, row_order[blockIdx.y * nq + blockIdx.x], 0);
     } else {
-      const int first = i / (order_heads * nq) * order_heads, j = i - first * nq, heads = min(order_heads, (int)gridDim.y - first);
-      at = (first + j % heads) * nq + nq - 1 - j / heads;
+      const HeadGroup group = head_group(group_of_head(blockIdx.y, gridDim.y, order_groups), gridDim.y, order_groups);
+      const int j = (blockIdx.y - group.first) * nq + blockIdx.x;
+      at = (group.first + j % group.heads) * nq + nq - 1 - j / group.heads;
     }
   }
   const int bh = ORDERED ? at / nq : blockIdx.y, h = bh % H;
@@ -750,7 +751,7 @@ static bool attn_attributes(const void* kern, int smem, std::atomic<uint64_t>& d
 
 template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16, bool ORDERED = false>
 static int launch_attn(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, cudaStream_t st) {
-  if (GRAN == 1 && PV_MODE != 2 && !ORDERED && !a.q_ranges && (a.row_order || a.order_heads > 1))
+  if (GRAN == 1 && PV_MODE != 2 && !ORDERED && !a.q_ranges && (a.row_order || (a.order_groups > 0 && a.order_groups < a.B * a.H)))
     return launch_attn<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16, GRAN == 1 && PV_MODE != 2>(a, tq, tk, tv, st);
   auto kern = attn_kernel<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16, ORDERED>;
   constexpr int smem = AttnShape<D, PVF16>::kSmemBytes;
@@ -760,7 +761,7 @@ static int launch_attn(const AttnArgs& a, const CUtensorMap& tq, const CUtensorM
   const int gx = a.q_ranges ? min(a.q_blocks_max, nq) : nq;
   const cudaError_t e = launch(kern, dim3(gx, a.B * a.H), kAttnThreads, smem, st, a.dependent, tq, tk, tv, (OutT*)a.o, a.lut,
                                a.valid, a.pvthr, a.q_scale, a.k_scale, a.v_scale, a.dev_status, a.N, a.H, nq, nk,
-                               a.sm_scale * kLog2e, a.o_st[0], a.o_st[1], a.o_st[2], a.pv_count, a.q_ranges, a.row_order, a.order_heads);
+                               a.sm_scale * kLog2e, a.o_st[0], a.o_st[1], a.o_st[2], a.pv_count, a.q_ranges, a.row_order, a.order_groups);
   return e == cudaSuccess ? SPARGE_OK : SPARGE_ERR_CUDA;
 }
 

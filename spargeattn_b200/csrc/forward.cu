@@ -91,8 +91,10 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
   if (rc != SPARGE_OK) return rc;
 
   // With cdf selection or a causal map the rows differ in length, and a long one that starts late keeps the chip waiting: they
-  // are computed longest first, over as many heads as have their K and V in kOrderBytes. A causal row is the longer the later
-  // it is. cdf counts are sorted, where there are more rows than the chip holds at a time and a row is long enough to be worth
+  // are computed longest first, over even groups of as many heads as have their K and V in kOrderBytes. (Full groups and a rest
+  // of one or two heads start the rest's longest rows last, which is slower than head by head: cdf [1,24,5632,128] 303 us head
+  // by head, 312 as 22 + 2 heads, 295 as 12 + 12; causal top-k [1,17,8192,128] 267 / 271 / 244, [1,16,50000,64] 4 564 / 4 601 /
+  // 4 411, fp16 P.V [1,16,16384,128] 944 / 991 / 876.) A causal row is the longer the later it is. cdf counts are sorted, where there are more rows than the chip holds at a time and a row is long enough to be worth
   // the launch: 239 -> 243 us with 64 blocks a row (cdf, [1,24,4096,128]), 374.7 -> 369.9 with 94 ([1,24,6000,128]).
   // Calls in us, head by head and with 16 / 32 / 48 / 96 MB: causal top-k [1,32,32768,128] 5 052 and 5 013 / 4 980 / 4 989 / 5 064,
   // [1,40,15000,64] 1 250 and 1 166 / 1 173 / 1 162 / 1 159; cdf [1,12,32760,128] 3 266 and 3 269 / 3 243 / 3 269 / 3 273,
@@ -100,11 +102,12 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
   constexpr long long kOrderBytes = 32LL << 20;
   constexpr int kSortBlocks = 80;
   const long long head_bytes = (a.pv_fp16 ? 3LL : 2LL) * a.N * a.D;
-  const int order_heads = (int)std::max(1LL, std::min((long long)p.BH, kOrderBytes / head_bytes));
+  const int most_heads = (int)std::max(1LL, std::min((long long)p.BH, kOrderBytes / head_bytes));
+  const int order_groups = (p.BH + most_heads - 1) / most_heads;
   int32_t* rows = nullptr;
   if (select && a.cdf && !a.q_ranges && nk > kSortBlocks && (long long)p.BH * nq > 2 * 148) {
     rows = static_cast<int32_t*>(p.scratch);   // free again: the preparation's partial sums
-    rc = row_order_launch(valid, rows, p.BH * nq, order_heads * nq, nk, st);
+    rc = row_order_launch(valid, rows, p.BH, nq, order_groups, nk, st);
     if (rc != SPARGE_OK) return rc;
   }
 
@@ -118,7 +121,7 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
     t.o_st[i] = a.o_st[i];
     t.v_st[i] = copy_v ? packed[i] : a.v_st[i];
   }
-  t.row_order = rows, t.order_heads = select && a.is_causal ? order_heads : 0;
+  t.row_order = rows, t.order_groups = select && a.is_causal ? order_groups : 0;
   t.q_ranges = a.q_ranges, t.q_blocks_max = a.q_blocks_max, t.B = a.B, t.H = a.H, t.N = a.N, t.D = a.D;
   t.out_dtype = a.dtype, t.causal = a.kernel_causal, t.gran = 1, t.pv_mode = a.pvthr != nullptr, t.dependent = true;
   t.sm_scale = a.sm_scale;

@@ -23,6 +23,7 @@
 #include <cfloat>
 
 #include "launch.cuh"
+#include "row_groups.cuh"
 #include "select.cuh"
 
 namespace sparge {
@@ -628,10 +629,11 @@ __global__ void __launch_bounds__(kSelThreads) mask_to_lut_kernel(const uint8_t*
 // Counting sort of a group of rows by their number of live blocks, longest first, by one CTA per group. Rows of one bucket
 // come in any order: it decides when a row is computed, not what comes out.
 constexpr int kOrderThreads = 1024, kOrderBuckets = 256;
-__global__ void __launch_bounds__(kOrderThreads) row_order_kernel(const int32_t* valid, int32_t* __restrict__ rows, int n, int group,
-                                                                  int nk) {
+__global__ void __launch_bounds__(kOrderThreads) row_order_kernel(const int32_t* valid, int32_t* __restrict__ rows, int heads,
+                                                                  int nq, int nk) {
   __shared__ int s_place[kOrderBuckets], s_sum[kOrderBuckets / 32];
-  const int tid = threadIdx.x, first = blockIdx.x * group, last = min(n, first + group);
+  const HeadGroup group = head_group(blockIdx.x, heads, gridDim.x);
+  const int tid = threadIdx.x, first = group.first * nq, last = first + group.heads * nq;
   if (tid < kOrderBuckets) s_place[tid] = 0;
   pdl_wait();
   __syncthreads();
@@ -658,10 +660,9 @@ __global__ void __launch_bounds__(kOrderThreads) row_order_kernel(const int32_t*
   pdl_trigger();
 }
 
-int row_order_launch(const int32_t* valid, int32_t* rows, int n, int group, int nk, cudaStream_t st) {
-  return launch(row_order_kernel, dim3((n + group - 1) / group), kOrderThreads, 0, st, true, valid, rows, n, group, nk) == cudaSuccess
-             ? SPARGE_OK
-             : SPARGE_ERR_CUDA;
+int row_order_launch(const int32_t* valid, int32_t* rows, int heads, int nq, int groups, int nk, cudaStream_t st) {
+  return launch(row_order_kernel, dim3(groups), kOrderThreads, 0, st, true, valid, rows, heads, nq, nk) == cudaSuccess ? SPARGE_OK
+                                                                                                                      : SPARGE_ERR_CUDA;
 }
 
 template <typename T, int D, int RW, int WARPS>

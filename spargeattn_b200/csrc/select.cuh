@@ -16,8 +16,8 @@ struct SelectArgs {
 };
 int select_launch(const SelectArgs& a, cudaStream_t st);
 
-// rows [n]: the row numbers 0 .. n - 1, in groups of `group` consecutive ones, in a group the largest counts (of nk) first
-int row_order_launch(const int32_t* valid, int32_t* rows, int n, int group, int nk, cudaStream_t st);
+// rows [heads * nq]: the row numbers, in `groups` even groups of heads, in a group the largest counts (of nk) first
+int row_order_launch(const int32_t* valid, int32_t* rows, int heads, int nq, int groups, int nk, cudaStream_t st);
 
 int mask_to_lut_launch(const void* mask, int elem_size, int32_t* lut, int32_t* valid, long long rows, int nk, bool dependent,
                        cudaStream_t st);

@@ -332,6 +332,39 @@ def test_longest_rows_first(kw, H, N, D):
     assert torch.equal(one, separate)
 
 
+def _rows_of_many_lengths(B, H, N, D, dtype):
+    """q, k, v whose query blocks are alike in themselves and look at anything from a few key blocks to nearly all."""
+    g = torch.Generator("cuda").manual_seed(N)
+    per_block = lambda size: torch.randn(B, H, (N + size - 1) // size, D, generator=g, device="cuda").repeat_interleave(size, 2)[:, :, :N]
+    noise = lambda: 0.3 * torch.randn(B, H, N, D, generator=g, device="cuda")
+    sharp = (4 * torch.rand(B, H, (N + 127) // 128, 1, generator=g, device="cuda")).repeat_interleave(128, 2)[:, :, :N]
+    return (sharp * per_block(128) + noise()).to(dtype), (per_block(64) + noise()).to(dtype), noise().to(dtype)
+
+
+@pytest.mark.parametrize("B,H,N,D", [(1, 6, 6400, 128), (2, 25, 5300, 128), (1, 21, 33000, 64), (3, 9, 33000, 128)])
+def test_order_of_the_rows(B, H, N, D):
+    """The sorted order that a cdf call leaves in its workspace: every row once, in even groups of heads (as many heads as have
+    their K and V in some tens of MB; a short last group starts its longest rows late), longest first in each group. A
+    bucket is 1/255 of a row."""
+    from spargeattn_b200 import ops
+    q, k, v = _rows_of_many_lengths(B, H, N, D, torch.bfloat16)
+    vec = lambda x: torch.full((H,), x, device="cuda")
+    _, ws, at = ops.meansim_forward(q, k, v, torch.empty_like(q), vec(-0.1), vec(0.8), None, None, D ** -0.5, False, False, False, True)
+    ops.check_device_status()
+    nq, nk = (N + 127) // 128, (N + 63) // 64
+    part = lambda name: ws[at[name]:at[name] + B * H * nq * 4].view(torch.int32).cpu().long()
+    rows, valid = part("scratch"), part("valid")
+    assert torch.equal(rows.sort().values, torch.arange(B * H * nq))
+    assert valid.max() - valid.min() > nk // 4                                     # the order is put to a test
+    ends = (rows.cummax(0).values == torch.arange(B * H * nq)).nonzero().flatten() + 1   # the first n rows are 0 .. n - 1
+    ends = [0] + [int(e) for e in ends if e % nq == 0]
+    heads = [(b - a) // nq for a, b in zip(ends, ends[1:])]
+    assert sum(heads) == B * H and max(heads) - min(heads) <= 1 and max(heads) > 1, heads
+    bucket = 255 - valid[rows] * 255 // nk
+    for a, b in zip(ends, ends[1:]):
+        assert bool((bucket[a:b].diff() >= 0).all())
+
+
 def test_ranges_without_a_largest_count_are_an_assertion():
     from spargeattn_b200.sharding import attention_units
     q = torch.randn(1, 2, 256, 64).bfloat16().cuda()

@@ -35,6 +35,35 @@ def test_no_block_returns_before_it_has_waited():
         assert not re.search(r"\breturn;", body[:body.index("pdl_wait")]), name
 
 
+def test_heads_are_grouped_evenly(tmp_path):
+    """Groups of heads follow one another, cover all heads, differ by one head at most, and a head finds its own."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no g++")
+    src = tmp_path / "groups.cpp"
+    src.write_text('''
+#include <initializer_list>
+#include "row_groups.cuh"
+int main() {
+  using namespace sparge;
+  for (int heads : {1, 2, 3, 13, 16, 24, 25, 26, 60, 997, 65535})
+    for (int groups = 1; groups <= heads; groups += heads < 1000 || groups < 40 || groups > heads - 40 ? 1 : 611) {
+      int next = 0;
+      for (int g = 0; g < groups; g++) {
+        const HeadGroup h = head_group(g, heads, groups);
+        if (h.first != next || h.heads < heads / groups || h.heads > (heads + groups - 1) / groups) return 1;
+        if (group_of_head(h.first, heads, groups) != g || group_of_head(h.first + h.heads - 1, heads, groups) != g) return 2;
+        next = h.first + h.heads;
+      }
+      if (next != heads) return 3;
+    }
+  return 0;
+}
+''')
+    subprocess.run([gxx, "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(tmp_path / "groups")], check=True)
+    assert subprocess.run([str(tmp_path / "groups")]).returncode == 0
+
+
 def test_any_step_word_names_a_block_of_the_row(tmp_path):
     """The softmax warps go on after an expired wait, on whatever the word in shared memory then holds."""
     gxx = shutil.which("g++")
