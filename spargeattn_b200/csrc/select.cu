@@ -94,8 +94,8 @@ __device__ __forceinline__ float key_value<__nv_bfloat16>(uint32_t k) {
 //      bits with eight keys per lane and load, final map and LUT.
 // What bounds it: instruction issue of the score chains (1.3 per score and channel), then the fp64 pipe; a short row is a
 // chain of dependent reductions. With one row per warp the chain is kept short: the first tile is asked for together with the
-// query, exponentials go four at a time and are kept, the three counts of a bisection round share one reduction. Whole
-// calls: [2,8,1000,128] 36.9 -> 35.8 us, [1,24,4608,128] 177.2 -> 176.9, cdf [1,16,8191,128] 382 -> 381.
+// query, exponentials go four at a time and are kept. (One reduction for the three counts of a bisection round, ten bits each,
+// is slower: 6.02 -> 6.16 us for 64 rows of 32 blocks, 9.75 -> 9.92 for 864 of 72, 18.1 -> 18.3 for 1 536 of 254.)
 constexpr int kSelTileKeys = 64;
 // Marks of a block that is not self-similar: in place of its score, and in place of its probability (zero, with the sign
 // bit telling that the block is live whatever the selection says).
@@ -487,24 +487,16 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
     // reductions); padding and not-similar keys count as zero
     const uint4* groups = reinterpret_cast<const uint4*>(s_key);
     const uint4 own = groups[lane];                          // all there is of a row of up to 256 blocks
-    auto count_lane = [&](uint32_t cand) {
+    auto count = [&](uint32_t cand) {
       const uint32_t cand2 = cand | (cand << 16);
       int c = count_ge<T>(own, cand2);
       for (int i = lane + 32; i < padded / 8; i += 32) c += count_ge<T>(groups[i], cand2);
-      return (unsigned)c;
+      return (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
     };
-    auto count = [&](uint32_t cand) { return (int)__reduce_add_sync(0xffffffffu, count_lane(cand)); };
     uint32_t thr_key = count(1u << 14) >= n_sel ? 1u << 14 : 0u;
 #pragma unroll 1
     for (int bit = 12; bit >= 0; bit -= 2) {
-      int c1, c2, c3;
-      const unsigned l1 = count_lane(thr_key | (1u << bit)), l2 = count_lane(thr_key | (2u << bit)), l3 = count_lane(thr_key | (3u << bit));
-      if (RW == 1 && padded < 1024) {                        // ten bits hold a count: one reduction for all three
-        const unsigned c = __reduce_add_sync(0xffffffffu, l1 | (l2 << 10) | (l3 << 20));
-        c1 = c & 1023, c2 = (c >> 10) & 1023, c3 = c >> 20;
-      } else {
-        c1 = (int)__reduce_add_sync(0xffffffffu, l1), c2 = (int)__reduce_add_sync(0xffffffffu, l2), c3 = (int)__reduce_add_sync(0xffffffffu, l3);
-      }
+      const int c1 = count(thr_key | (1u << bit)), c2 = count(thr_key | (2u << bit)), c3 = count(thr_key | (3u << bit));
       thr_key |= (uint32_t)((c1 >= n_sel) + (c2 >= n_sel) + (c3 >= n_sel)) << bit;
     }
     const int remaining = n_sel - count(thr_key + 1);
