@@ -93,9 +93,10 @@ __device__ __forceinline__ float key_value<__nv_bfloat16>(uint32_t k) {
 //   2  per row, by its warp alone (shuffles and ballots): fp64 softmax, selection threshold by bisection over the 16 key
 //      bits with eight keys per lane and load, final map and LUT.
 // What bounds it: instruction issue of the score chains (1.3 per score and channel), then the fp64 pipe; a short row is a
-// chain of dependent reductions. With one row per warp the chain is kept short: the first tile is asked for together with the
-// query, exponentials go four at a time and are kept. (One reduction for the three counts of a bisection round, ten bits each,
-// is slower: 6.02 -> 6.16 us for 64 rows of 32 blocks, 9.75 -> 9.92 for 864 of 72, 18.1 -> 18.3 for 1 536 of 254.)
+// chain of dependent reductions. With one row per warp the first tile is asked for together with the query: kernel alone
+// 6.64 -> 6.08 us for 64 rows of 32 blocks, 10.78 -> 10.14 for 864 of 72, cdf 16.05 -> 15.20 for 1 024 of 128. (One reduction
+// for the three counts of a bisection round, ten bits each, is slower: 6.02 -> 6.16 us for 64 rows of 32 blocks, 9.75 -> 9.92
+// for 864 of 72, 18.1 -> 18.3 for 1 536 of 254.)
 constexpr int kSelTileKeys = 64;
 // Marks of a block that is not self-similar: in place of its score, and in place of its probability (zero, with the sign
 // bit telling that the block is live whatever the selection says).
@@ -404,31 +405,15 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
       q_similar[i] = q_similar[i + 1];
     }
 
-    // fp64 softmax -> 16-bit keys (p >= 0, so the bit pattern orders like the value). One row per warp is a chain of
-    // latencies: the exponentials of its first 256 keys are evaluated four at a time and kept. The others are evaluated twice,
-    // once for the sum and once for the probabilities, instead of being stored; so are all of them with two rows per warp,
-    // where the registers cost more than the instructions ([2,30,17776,64]: call 3 552 -> 3 576 us).
-    constexpr int kKeep = RW == 1 ? 8 : 0;
-    const double dmx = (double)mx;
-    double e[kKeep > 0 ? kKeep : 1], Z = 0.0;
-#pragma unroll
-    for (int g = 0; g < kKeep; g += 4) {
-      if (g * 32 < nk) {
-#pragma unroll
-        for (int i = g; i < g + 4; i++) {
-          const int j = i * 32 + lane;
-          const uint16_t raw = j < nk ? s_key[j] : kNotSimilarScore;
-          const float sc = key_value<T>(raw);
-          e[i] = exp_nonpositive(raw != kNotSimilarScore && sc != -INFINITY ? (double)sc - dmx : -1000.0);
-        }
-#pragma unroll
-        for (int i = g; i < g + 4; i++) Z += e[i];
-      }
-    }
-    for (int j = kKeep * 32 + lane; j < nk; j += 32) {
+    // fp64 softmax -> 16-bit keys (p >= 0, so the bit pattern orders like the value). The exponentials are evaluated
+    // twice, once for the sum and once for the probabilities, instead of being stored. (The first 256 kept in registers, evaluated four at a time, made the
+    // kernel alone 0.1-2 us shorter and calls of short rows longer: a row of 40 blocks has two per lane, and a call fetches the
+    // code anew. [1,30,2500,128] top-k 120.1 -> 121.2 us, cdf 162.3 -> 163.2, against cdf [1,16,8191,128] 381.9 -> 380.6.)
+    double Z = 0.0;
+    for (int j = lane; j < nk; j += 32) {
       const uint16_t raw = s_key[j];
       const float sc = key_value<T>(raw);
-      if (raw != kNotSimilarScore && sc != -INFINITY) Z += exp_nonpositive((double)sc - dmx);
+      if (raw != kNotSimilarScore && sc != -INFINITY) Z += exp_nonpositive((double)sc - (double)mx);
     }
     Z = warp_sum(Z);
     const double rz = 1.0 / Z;
@@ -436,22 +421,13 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
     // n_sel blocks. Zeros are equal too, and the comparisons below can count them.
     const bool undefined = Z != Z;
     const int padded = (nk + 255) / 256 * 256;
-    auto key_of = [&](uint16_t raw, double ej) -> uint16_t {
-      if (raw == kNotSimilarScore) return kNotSimilarKey;
-      if (key_value<T>(raw) == -INFINITY || undefined) return 0;
-      return (uint16_t)key_bits<T>(Elem<T>::from_float((float)(ej * rz)));
-    };
-#pragma unroll
-    for (int i = 0; i < kKeep; i++) {                        // (a row has 256 keys or padding)
-      const int j = i * 32 + lane;
-      s_key[j] = j < nk ? key_of(s_key[j], e[i]) : (uint16_t)0;
-    }
-    for (int j = kKeep * 32 + lane; j < padded; j += 32) {
+    for (int j = lane; j < padded; j += 32) {
       uint16_t key = 0;
       if (j < nk) {
         const uint16_t raw = s_key[j];
         const float sc = key_value<T>(raw);
-        key = key_of(raw, raw != kNotSimilarScore && sc != -INFINITY ? exp_nonpositive((double)sc - dmx) : 0.0);
+        if (raw == kNotSimilarScore) key = kNotSimilarKey;
+        else if (sc != -INFINITY && !undefined) key = (uint16_t)key_bits<T>(Elem<T>::from_float((float)(exp_nonpositive((double)sc - (double)mx) * rz)));
       }
       s_key[j] = key;
     }
