@@ -177,8 +177,10 @@ constexpr int kAttnThreads = 192;
 
 // GRAN = qk_quant_gran: 1 one Q scale per 128-row block, 2 one per 32-row group (the K scale is per 64-key block in
 // both), 3 per-thread Q/K scales. PV_MODE = PVThresholdMode: 0 no skip test, 1 the test decides per block, 2 per
-// 32-row group. ORDERED: rows in the order of row_order or order_groups (AttnArgs); a variant of its own because the two
-// registers that it takes cost the others 1 %.
+// 32-row group. ORDERED: rows in the order of row_order or order_groups (AttnArgs), without row ranges and without counts of
+// products. A variant of its own: with the same rows in the same order it is slower without the skip test (calls of
+// [1,12,32760,128] 2 510 -> 2 530 us, [2,30,17776,64] 3 548 -> 3 584, [1,24,4608,128] 171.4 -> 173.0) and no slower with it
+// (2 742 -> 2 737, 3 907 -> 3 837). Registers are not the reason: it takes 164-168, the other 163-168.
 template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16 = false, bool ORDERED = false>
 __global__ void __launch_bounds__(kAttnThreads, (AttnShape<D, PVF16>::kCtasPerSm))
 attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -226,9 +228,9 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     }
   }
   const int bh = ORDERED ? at / nq : blockIdx.y, h = bh % H;
-  const int q_begin = q_ranges ? q_ranges[2 * bh] : 0;
-  const int q_count = q_ranges ? min(q_ranges[2 * bh + 1], nq - q_begin) : (int)gridDim.x;
-  if ((int)blockIdx.x >= q_count) {
+  const int q_begin = !ORDERED && q_ranges ? q_ranges[2 * bh] : 0;
+  const int q_count = !ORDERED && q_ranges ? min(q_ranges[2 * bh + 1], nq - q_begin) : (int)gridDim.x;
+  if (!ORDERED && (int)blockIdx.x >= q_count) {
     pdl_wait();   // when every CTA leaves here, this kernel must still not end before the ones that it depends on
     return;
   }
@@ -285,7 +287,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     OutT* obase = o + (size_t)(bh / H) * osb + (size_t)(bh % H) * osh + (size_t)qi * 128 * osn;
     for (int i = tid; i < rows * kChunks; i += kAttnThreads)
       reinterpret_cast<uint4*>(obase + (size_t)(i / kChunks) * osn)[i % kChunks] = make_uint4(0, 0, 0, 0);
-    if (pv_count && tid < 4) pv_count[row_id * 4 + tid] = 0;
+    if (!ORDERED && pv_count && tid < 4) pv_count[row_id * 4 + tid] = 0;
   } else if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -658,7 +660,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       // has its own.
       const int row_end = ORDERED ? *(volatile int*)&s_row : 0, bh_end = ORDERED ? row_end / nq : bh;
       const int qrow_end = ORDERED ? (row_end - bh_end * nq) * 128 + row : qrow;
-      if (pv_count && lane == 0) pv_count[(ORDERED ? (size_t)row_end : row_id) * 4 + warp] = npv;
+      if (!ORDERED && pv_count && lane == 0) pv_count[row_id * 4 + warp] = npv;
       // A row that saw no key at all (token-level causal mask over every live block of its row of blocks) has an
       // empty sum: it is written as zeros. (The reference gives such a row the plain average of V over the masked
       // keys, because its mask value is a large finite number and exp2(mask - mask) = 1.)
@@ -751,7 +753,7 @@ static bool attn_attributes(const void* kern, int smem, std::atomic<uint64_t>& d
 
 template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16, bool ORDERED = false>
 static int launch_attn(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, cudaStream_t st) {
-  if (GRAN == 1 && PV_MODE != 2 && !ORDERED && !a.q_ranges && (a.row_order || (a.order_groups > 0 && a.order_groups < a.B * a.H)))
+  if (GRAN == 1 && PV_MODE != 2 && !ORDERED && !a.q_ranges && !a.pv_count && (a.row_order || (a.order_groups > 0 && a.order_groups < a.B * a.H)))
     return launch_attn<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16, GRAN == 1 && PV_MODE != 2>(a, tq, tk, tv, st);
   auto kern = attn_kernel<D, CAUSAL, PV_MODE, OutT, GRAN, PVF16, ORDERED>;
   constexpr int smem = AttnShape<D, PVF16>::kSmemBytes;
