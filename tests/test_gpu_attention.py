@@ -212,7 +212,7 @@ def test_concurrent_preparation_gives_the_same_bytes():
                                 dict(topk=0.4, tensor_layout="NHD")])
 @pytest.mark.parametrize("shape,dtype", [((2, 3, 1100, 64), torch.bfloat16), ((1, 2, 2048, 128), torch.float16)])
 def test_single_call_path_equals_the_entry_by_entry_path(kw, shape, dtype):
-    """The native one-call path (fused preparation, four or five launches) against the separate entries: the same arithmetic,
+    """The native one-call path (fused preparation, four to six launches) against the separate entries: the same arithmetic,
     so the bytes are the same, for every knob, with and without return_sparsity."""
     import spargeattn_b200 as S
     from spargeattn_b200 import core

@@ -310,17 +310,34 @@ def test_c_entry_of_the_whole_path(kw, N, D, dtype, v_dtype):
     ops.check_device_status()
 
 
-@pytest.mark.parametrize("kw", [dict(cdfthreshd=0.8, simthreshd1=0.3), dict(topk=0.3, is_causal=True), dict(cdfthreshd=0.7, is_causal=True, pvthreshd=4.0)])
-@pytest.mark.parametrize("H,N,D", [(148, 256, 64), (297, 128, 64), (5, 7700, 128), (41, 4996, 128)])
-def test_longest_rows_first(kw, H, N, D):
-    """Rows that differ in length are computed in another order: from 297 of them on, here one group of heads, the last case
-    two. Every row has to come out, with the bytes of the separate entries, which compute them in their own order."""
+def _rows_of_many_lengths(B, H, N, D, dtype):
+    """q, k, v whose query blocks are alike in themselves and look at anything from a few key blocks to nearly all."""
+    g = torch.Generator("cuda").manual_seed(N)
+    per_block = lambda size: torch.randn(B, H, (N + size - 1) // size, D, generator=g, device="cuda").repeat_interleave(size, 2)[:, :, :N]
+    noise = lambda: 0.3 * torch.randn(B, H, N, D, generator=g, device="cuda")
+    sharp = (4 * torch.rand(B, H, (N + 127) // 128, 1, generator=g, device="cuda")).repeat_interleave(128, 2)[:, :, :N]
+    return (sharp * per_block(128) + noise()).to(dtype), (per_block(64) + noise()).to(dtype), noise().to(dtype)
+
+
+@pytest.mark.parametrize("kw", [dict(cdfthreshd=0.8, simthreshd1=-0.1), dict(topk=0.3, is_causal=True), dict(cdfthreshd=0.7, is_causal=True, pvthreshd=4.0),
+                                dict(cdfthreshd=0.8, simthreshd1=-0.1, fp16_pv=True), dict(topk=0.3, is_causal=True, fp16_pv=True)])
+@pytest.mark.parametrize("B,H,N,D,layout", [(1, 148, 256, 64, "HND"), (1, 297, 128, 64, "HND"), (1, 5, 7700, 128, "HND"), (1, 41, 4996, 128, "HND"),
+                                            (1, 41, 5200, 128, "HND"), (2, 4, 5190, 64, "NHD"), (2, 25, 10300, 64, "HND"), (3, 2, 6700, 128, "NHD")])
+def test_longest_rows_first(kw, B, H, N, D, layout):
+    """Rows that differ in length are computed in another order, sorted by their counts in cdf calls of more than 296 rows of
+    more than 80 blocks, by position in the other causal ones: one group of heads and several, one batch and several, both
+    kinds of V. Every row has to come out, with the bytes of the separate entries, which compute them in their own order."""
     import spargeattn_b200 as S
     from spargeattn_b200 import core, ops
-    g = torch.Generator("cuda").manual_seed(N)
-    q, k, v = (torch.randn(1, H, N, D, generator=g, device="cuda").bfloat16() for _ in range(3))
-    k[:, :, :64] *= 3
-    fn = S.spas_sage2_attn_meansim_topk_cuda if "topk" in kw else S.spas_sage2_attn_meansim_cuda
+    kw = dict(kw, tensor_layout=layout)
+    fp16_pv = kw.pop("fp16_pv", False)
+    q, k, v = _rows_of_many_lengths(B, H, N, D, torch.float16 if fp16_pv else torch.bfloat16)
+    if layout == "NHD":
+        q, k, v = (x.transpose(1, 2).contiguous() for x in (q, k, v))
+    sage = "sage" if fp16_pv else "sage2"
+    fn = getattr(S, f"spas_{sage}_attn_meansim_topk_cuda" if "topk" in kw else f"spas_{sage}_attn_meansim_cuda")
+    del_me = torch.full_like(q, float("nan"))              # what the output's memory holds: a row left out shows
+    del del_me
     one = fn(q, k, v, **kw)
     single = core.SINGLE_CALL_MAX_ROWS
     try:
@@ -332,20 +349,13 @@ def test_longest_rows_first(kw, H, N, D):
     assert torch.equal(one, separate)
 
 
-def _rows_of_many_lengths(B, H, N, D, dtype):
-    """q, k, v whose query blocks are alike in themselves and look at anything from a few key blocks to nearly all."""
-    g = torch.Generator("cuda").manual_seed(N)
-    per_block = lambda size: torch.randn(B, H, (N + size - 1) // size, D, generator=g, device="cuda").repeat_interleave(size, 2)[:, :, :N]
-    noise = lambda: 0.3 * torch.randn(B, H, N, D, generator=g, device="cuda")
-    sharp = (4 * torch.rand(B, H, (N + 127) // 128, 1, generator=g, device="cuda")).repeat_interleave(128, 2)[:, :, :N]
-    return (sharp * per_block(128) + noise()).to(dtype), (per_block(64) + noise()).to(dtype), noise().to(dtype)
-
-
-@pytest.mark.parametrize("B,H,N,D", [(1, 6, 6400, 128), (2, 25, 5300, 128), (1, 21, 33000, 64), (3, 9, 33000, 128)])
-def test_order_of_the_rows(B, H, N, D):
-    """The sorted order that a cdf call leaves in its workspace: every row once, in even groups of heads (as many heads as have
-    their K and V in some tens of MB; a short last group starts its longest rows late), longest first in each group. A
-    bucket is 1/255 of a row."""
+@pytest.mark.parametrize("B,H,N,D,ordered", [(1, 6, 6400, 128, True), (2, 25, 5300, 128, True), (1, 21, 33000, 64, True), (3, 9, 33000, 128, True),
+                                             (1, 8, 5120, 64, False), (1, 8, 5121, 64, True),       # 80, 81 blocks
+                                             (1, 4, 9472, 64, False), (1, 3, 12672, 64, True)])     # 296, 297 rows
+def test_order_of_the_rows(B, H, N, D, ordered):
+    """The sorted order that a cdf call of more than 296 rows of more than 80 blocks leaves in its workspace: every row once, in
+    even groups of heads (as many heads as have their K and V in some tens of MB; a short last group starts its longest rows
+    late), longest first in each group. A bucket is 1/255 of a row."""
     from spargeattn_b200 import ops
     q, k, v = _rows_of_many_lengths(B, H, N, D, torch.bfloat16)
     vec = lambda x: torch.full((H,), x, device="cuda")
@@ -354,7 +364,9 @@ def test_order_of_the_rows(B, H, N, D):
     nq, nk = (N + 127) // 128, (N + 63) // 64
     part = lambda name: ws[at[name]:at[name] + B * H * nq * 4].view(torch.int32).cpu().long()
     rows, valid = part("scratch"), part("valid")
-    assert torch.equal(rows.sort().values, torch.arange(B * H * nq))
+    assert torch.equal(rows.sort().values, torch.arange(B * H * nq)) == ordered
+    if not ordered:
+        return
     assert valid.max() - valid.min() > nk // 4                                     # the order is put to a test
     ends = (rows.cummax(0).values == torch.arange(B * H * nq)).nonzero().flatten() + 1   # the first n rows are 0 .. n - 1
     ends = [0] + [int(e) for e in ends if e % nq == 0]
