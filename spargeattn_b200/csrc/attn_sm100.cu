@@ -178,9 +178,10 @@ constexpr int kAttnThreads = 192;
 // GRAN = qk_quant_gran: 1 one Q scale per 128-row block, 2 one per 32-row group (the K scale is per 64-key block in
 // both), 3 per-thread Q/K scales. PV_MODE = PVThresholdMode: 0 no skip test, 1 the test decides per block, 2 per
 // 32-row group. ORDERED: rows in the order of row_order or order_groups (AttnArgs), without row ranges and without counts of
-// products. A variant of its own: with the same rows in the same order it is slower without the skip test (calls of
-// [1,12,32760,128] 2 510 -> 2 530 us, [2,30,17776,64] 3 548 -> 3 584, [1,24,4608,128] 171.4 -> 173.0) and no slower with it
-// (2 742 -> 2 737, 3 907 -> 3 837). Registers are not the reason: it takes 164-168, the other 163-168.
+// products. A variant of its own: it takes the row's place from shared memory in the epilogue, and the plain kernel, which has
+// it from its block index, is slower like that (calls of [1,12,32760,128] 2 519 -> 2 549 us, [2,30,17776,64] 3 539 -> 3 595,
+// with the skip test 2 737 -> 2 860 and 3 900 -> 4 117). With the same rows in the same order a call of the variant takes
+// 2 502, 3 540, 2 709 and 3 853 us; in short CTAs the order's arithmetic shows ([1,24,4608,128] 170.7 -> 171.4).
 template <int D, bool CAUSAL, int PV_MODE, typename OutT, int GRAN, bool PVF16 = false, bool ORDERED = false>
 __global__ void __launch_bounds__(kAttnThreads, (AttnShape<D, PVF16>::kCtasPerSm))
 attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -202,7 +203,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   __shared__ uint64_t bar_q, bar_k_full[SK], bar_k_empty[SK], bar_v_full[NV], bar_v_empty[NV], bar_s_full, bar_s_free,
       bar_p_ready[2], bar_o_done[2], bar_vote[2];   // the pairs alternate by step
   __shared__ uint32_t s_tmem_base;
-  __shared__ int s_row;                // ORDERED: the CTA's row
+  __shared__ int s_bh, s_qi;           // ORDERED: the CTA's head and query block
   __shared__ int s_skip[2][2], s_fail;   // [step parity][block of the pair]
   // PV-skip votes, one byte per softmax warp: [step parity][block of the pair]
   __shared__ uint32_t s_vote[2][2];
@@ -266,7 +267,12 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     }
     mbar_fence_init();
     s_fail = 0;
-    if (ORDERED) s_row = at;   // for the epilogue: a register that lives through the loop costs
+    // For the epilogue. A register that lives through the loop in their place costs 1-3 % of a call, and a division of the
+    // row's number there 1 % without the skip test ([1,12,32760,128] 2 572 and 2 538 us against 2 500).
+    if (ORDERED) {
+      s_bh = bh;
+      s_qi = qi;
+    }
   }
   pdl_wait();   // everything below reads what the kernels before this one wrote
   // V's scales wait in shared memory for the epilogue, where 128 loads per thread from global memory were a fifth of a
@@ -658,8 +664,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
       // One count per 32-row group, the layout of the reference's PV_Count (qk_int_sv_f8_cuda_sm89.cuh:650-656).
       // With the per-block decision the four entries of a block are equal; with the per-warp decision each group
       // has its own.
-      const int row_end = ORDERED ? *(volatile int*)&s_row : 0, bh_end = ORDERED ? row_end / nq : bh;
-      const int qrow_end = ORDERED ? (row_end - bh_end * nq) * 128 + row : qrow;
+      const int bh_end = ORDERED ? *(volatile int*)&s_bh : bh;
+      const int qrow_end = ORDERED ? *(volatile int*)&s_qi * 128 + row : qrow;
       if (!ORDERED && pv_count && lane == 0) pv_count[row_id * 4 + warp] = npv;
       // A row that saw no key at all (token-level causal mask over every live block of its row of blocks) has an
       // empty sum: it is written as zeros. (The reference gives such a row the plain average of V over the masked
