@@ -93,10 +93,11 @@ __device__ __forceinline__ float key_value<__nv_bfloat16>(uint32_t k) {
 //   2  per row, by its warp alone (shuffles and ballots): fp64 softmax, selection threshold by bisection over the 16 key
 //      bits with eight keys per lane and load, final map and LUT.
 // What bounds it: instruction issue of the score chains (1.3 per score and channel), then the fp64 pipe; a short row is a
-// chain of dependent reductions. With one row per warp the first tile is asked for together with the query: kernel alone
-// 6.64 -> 6.08 us for 64 rows of 32 blocks, 10.78 -> 10.14 for 864 of 72, cdf 16.05 -> 15.20 for 1 024 of 128. (One reduction
-// for the three counts of a bisection round, ten bits each, is slower: 6.02 -> 6.16 us for 64 rows of 32 blocks, 9.75 -> 9.92
-// for 864 of 72, 18.1 -> 18.3 for 1 536 of 254.)
+// chain of dependent reductions. With one row per warp the first tile is asked for together with the query (kernel alone
+// 6.64 -> 6.08 us for 64 rows of 32 blocks, 10.78 -> 10.14 for 864 of 72, cdf 16.05 -> 15.20 for 1 024 of 128; causal rows of
+// 512 lose, 47.2 -> 48.0 for 3 072), and the three counts of a bisection round share one reduction: calls of [2,8,1000,128]
+// 36.2 -> 35.6 us, [1,4,2048,64] 32.5 -> 32.2, [1,30,2500,128] 90.5 -> 90.0 (causal but the second), cdf [1,16,8191,128] 379.6 -> 378.9, although the
+// kernel alone, run again and again, takes 0.1-0.3 us longer.
 constexpr int kSelTileKeys = 64;
 // Marks of a block that is not self-similar: in place of its score, and in place of its probability (zero, with the sign
 // bit telling that the block is live whatever the selection says).
@@ -406,9 +407,10 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
     }
 
     // fp64 softmax -> 16-bit keys (p >= 0, so the bit pattern orders like the value). The exponentials are evaluated
-    // twice, once for the sum and once for the probabilities, instead of being stored. (The first 256 kept in registers, evaluated four at a time, made the
-    // kernel alone 0.1-2 us shorter and calls of short rows longer: a row of 40 blocks has two per lane, and a call fetches the
-    // code anew. [1,30,2500,128] top-k 120.1 -> 121.2 us, cdf 162.3 -> 163.2, against cdf [1,16,8191,128] 381.9 -> 380.6.)
+    // twice, once for the sum and once for the probabilities, instead of being stored. (The first 256 kept in registers,
+    // evaluated four at a time, made the kernel alone 0.1-2 us shorter and calls of short rows longer: a row of 40 blocks has
+    // two per lane, and a call fetches the code anew. [1,30,2500,128] top-k 120.1 -> 121.2 us, cdf 162.3 -> 163.2, against cdf
+    // [1,16,8191,128] 381.9 -> 380.6.)
     double Z = 0.0;
     for (int j = lane; j < nk; j += 32) {
       const uint16_t raw = s_key[j];
@@ -463,16 +465,24 @@ select_kernel(const T* pq, const T* pk, const uint8_t* sim_q, const uint8_t* sim
     // reductions); padding and not-similar keys count as zero
     const uint4* groups = reinterpret_cast<const uint4*>(s_key);
     const uint4 own = groups[lane];                          // all there is of a row of up to 256 blocks
-    auto count = [&](uint32_t cand) {
+    auto count_lane = [&](uint32_t cand) {
       const uint32_t cand2 = cand | (cand << 16);
       int c = count_ge<T>(own, cand2);
       for (int i = lane + 32; i < padded / 8; i += 32) c += count_ge<T>(groups[i], cand2);
-      return (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
+      return (unsigned)c;
     };
+    auto count = [&](uint32_t cand) { return (int)__reduce_add_sync(0xffffffffu, count_lane(cand)); };
     uint32_t thr_key = count(1u << 14) >= n_sel ? 1u << 14 : 0u;
 #pragma unroll 1
     for (int bit = 12; bit >= 0; bit -= 2) {
-      const int c1 = count(thr_key | (1u << bit)), c2 = count(thr_key | (2u << bit)), c3 = count(thr_key | (3u << bit));
+      int c1, c2, c3;
+      const unsigned l1 = count_lane(thr_key | (1u << bit)), l2 = count_lane(thr_key | (2u << bit)), l3 = count_lane(thr_key | (3u << bit));
+      if (RW == 1 && padded < 1024) {                        // ten bits hold a count: one reduction for all three
+        const unsigned c = __reduce_add_sync(0xffffffffu, l1 | (l2 << 10) | (l3 << 20));
+        c1 = c & 1023, c2 = (c >> 10) & 1023, c3 = c >> 20;
+      } else {
+        c1 = (int)__reduce_add_sync(0xffffffffu, l1), c2 = (int)__reduce_add_sync(0xffffffffu, l2), c3 = (int)__reduce_add_sync(0xffffffffu, l3);
+      }
       thr_key |= (uint32_t)((c1 >= n_sel) + (c2 >= n_sel) + (c3 >= n_sel)) << bit;
     }
     const int remaining = n_sel - count(thr_key + 1);
