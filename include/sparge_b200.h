@@ -210,7 +210,7 @@ int sparge_attn_fwd_f16pv(const int8_t* q_int8, const int8_t* k_int8, const void
 
 /* The whole path of spas_sage2_attn_meansim_topk_cuda / spas_sage2_attn_meansim_cuda (spas_sage_attn/core.py:39-169) in
  * one call: what sparge_k_mean (if smooth_k), sparge_pool_quant for Q and K, sparge_quant_v, sparge_select and
- * sparge_attn_fwd do, in four or five launches on `stream`, with every intermediate tensor carved out of `workspace`
+ * sparge_attn_fwd do, in four to six launches on `stream`, with every intermediate tensor carved out of `workspace`
  * (device memory, 256-byte aligned, at least sparge_forward_workspace_bytes(B,H,N,D) bytes; reusable by the next call
  * on the same stream). Results are those of the separate entries; it is the faster way at every size.
  *   q, k (dtype) and v (v_dtype): [B,H,N,D] views, strides in elements as {batch, head, token}, last dimension

@@ -94,11 +94,22 @@ int forward(const ForwardArgs& a, cudaStream_t st) {
   // are computed longest first, over even groups of as many heads as have their K and V in kOrderBytes. (Full groups and a rest
   // of one or two heads start the rest's longest rows last, which is slower than head by head: cdf [1,24,5632,128] 303 us head
   // by head, 312 as 22 + 2 heads, 295 as 12 + 12; causal top-k [1,17,8192,128] 267 / 271 / 244, [1,16,50000,64] 4 564 / 4 601 /
-  // 4 411, fp16 P.V [1,16,16384,128] 944 / 991 / 876.) A causal row is the longer the later it is. cdf counts are sorted, where there are more rows than the chip holds at a time and a row is long enough to be worth
-  // the launch: 239 -> 243 us with 64 blocks a row (cdf, [1,24,4096,128]), 374.7 -> 369.9 with 94 ([1,24,6000,128]).
-  // Calls in us, head by head and with 16 / 32 / 48 / 96 MB: causal top-k [1,32,32768,128] 5 052 and 5 013 / 4 980 / 4 989 / 5 064,
-  // [1,40,15000,64] 1 250 and 1 166 / 1 173 / 1 162 / 1 159; cdf [1,12,32760,128] 3 266 and 3 269 / 3 243 / 3 269 / 3 273,
-  // [2,20,10800,64] 1 333 and 1 306 / 1 293 / 1 312 / 1 287, [1,24,16200,128] 1 904 and 1 855 / 1 847 / 1 863 / 1 876.
+  // 4 411, fp16 P.V [1,16,16384,128] 944 / 991 / 876.) A causal row is the longer the later it is; other rows are sorted by
+  // their counts.
+  // kOrderBytes: with 16 MB the groups are short, above L2's 126 MB their K and V do not stay there; between, no size is the best.
+  // Calls in us, head by head and with 16 / 32 / 64 / 96 MB, runs of one setting differ by 0.1-0.5 %, by up to 4 % where marked *:
+  //   causal top-k  [1,40,15000,64] 1 400 and 1 306 / 1 301 / 1 298 / 1 298; * [1,32,32768,128] 5 408 and 5 270 / 5 160 / 5 137 /
+  //                 5 147, [1,8,65536,128] 4 371 and 4 378 / 4 229 / 4 188 / 4 183; * fp16 P.V [1,9,32768,128] 1 900 and 1 900 /
+  //                 1 830 / 1 766 / 1 780
+  //   cdf           [1,24,5632,128] 303.0 and 295.4 / 292.8 / 295.3 / 295.4, [2,30,17776,64] 5 328 and 5 237 / 5 248 / 5 234 / 5 261;
+  //                 * [1,12,32760,128] 3 457 and 3 305 / 3 245 / 3 297 / 3 233; fp16 P.V [1,24,16200,64] 1 919 and 1 838 / 1 820 /
+  //                 1 836 / 1 827
+  // Counts are sorted where there are more rows than the chip holds at a time; just above that the order gives 20 % or nothing,
+  // by what the second wave happens to be (cdf [1,3,14400,64], 339 rows, three draws: 303 -> 252, 258, 251; 400 rows 299 -> 288,
+  // 279 -> 285, 296 -> 264). Rows of one length, as when no query block is alike in itself, pay for the sort and gain nothing:
+  // 239.5 -> 241.8 with 64 blocks ([1,24,4096,128]), 435.6 -> 437.1 with 94 ([1,24,6000,128]); kSortBlocks keeps that price
+  // below 1 %. Rows that differ gain on both sides of it: 64 blocks 201.7 -> 197.1, [1,12,4096,64] 116.2 -> 105.2; 88 blocks
+  // 303.0 -> 292.8; 48 blocks 201.5 -> 201.2 ([1,40,3072,128]).
   constexpr long long kOrderBytes = 32LL << 20;
   constexpr int kSortBlocks = 80;
   const long long head_bytes = (a.pv_fp16 ? 3LL : 2LL) * a.N * a.D;

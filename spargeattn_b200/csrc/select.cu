@@ -95,9 +95,9 @@ __device__ __forceinline__ float key_value<__nv_bfloat16>(uint32_t k) {
 // What bounds it: instruction issue of the score chains (1.3 per score and channel), then the fp64 pipe; a short row is a
 // chain of dependent reductions. With one row per warp the first tile is asked for together with the query (kernel alone
 // 6.64 -> 6.08 us for 64 rows of 32 blocks, 10.78 -> 10.14 for 864 of 72, cdf 16.05 -> 15.20 for 1 024 of 128; causal rows of
-// 512 lose, 47.2 -> 48.0 for 3 072), and the three counts of a bisection round share one reduction: calls of [2,8,1000,128]
-// 36.2 -> 35.6 us, [1,4,2048,64] 32.5 -> 32.2, [1,30,2500,128] 90.5 -> 90.0 (causal but the second), cdf [1,16,8191,128] 379.6 -> 378.9, although the
-// kernel alone, run again and again, takes 0.1-0.3 us longer.
+// 512 lose, 47.2 -> 48.0 for 3 072), and the three counts of a bisection round share one reduction: causal calls of
+// [2,8,1000,128] 36.2 -> 35.6 us and [1,30,2500,128] 90.5 -> 90.0, [1,4,2048,64] 32.5 -> 32.2, cdf [1,16,8191,128] 379.6 ->
+// 378.9, although the kernel alone, run again and again, takes 0.1-0.3 us longer.
 constexpr int kSelTileKeys = 64;
 // Marks of a block that is not self-similar: in place of its score, and in place of its probability (zero, with the sign
 // bit telling that the block is live whatever the selection says).
