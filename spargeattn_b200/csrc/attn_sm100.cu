@@ -480,7 +480,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
           if (leader) {
             // fp16: 16 keys by all channels at a time. The instruction is bound by its operands' way out of shared memory, and one
             // per 64 channels fetched every row of P twice at D = 128: 12 KB a step of 16 keys instead of 8 ([1,12,32760,128],
-            // top-k 0.5: kernel 2 997 -> 2 919 us, whole call 3 230 -> 3 165).
+            // top-k 0.5: kernel 3 055 -> 2 963 us in turn under the power cap, 2 741 -> 2 658 before it sets in; whole call 3 167 ->
+            // 3 099).
             if (PVF16) {
 #pragma unroll
               for (int ks = 0; ks < 4; ks++)
